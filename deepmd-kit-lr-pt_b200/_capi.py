@@ -107,6 +107,9 @@ _FUNCS = {
     "dpb_se_a_descriptor_bwd_f32": "ppppp" "pp" "pi" "iiip",
     "dpb_se_a_descriptor_fwd_cubic_f32": "pppp" "pp" "pi" "iiip",
     "dpb_se_a_descriptor_bwd_cubic_f32": "ppppp" "pp" "pi" "iiip",
+    "dpb_se_a_descriptor_fwd_cheb_f32": "pppp" "pppp" "pi" "iiip",
+    "dpb_se_a_descriptor_bwd_cheb_f32": "ppppp" "pppp" "pi" "iiip",
+    "dpb_bt_step_set_nets": "ppp",
     "dpb_force_virial_a_f32": "pppppp" "pp" "iiiip",
     "dpb_force_virial_a_f64": "pppppp" "pp" "iiiip",
     "dpb_build_nlist_noalloc_f64": "ppppp" "iiif" "i" "pp",
@@ -199,6 +202,12 @@ def check(code: int, what: str = "") -> None:
     cls = _ERRORS.get(code, DPBError)
     msg = last_error()
     raise cls(f"DeePMD-kit Error: {what + ': ' if what else ''}{msg}")
+
+
+class ChebNet(ctypes.Structure):
+    """dpb_cheb_net of include/dpb200.h."""
+    _fields_ = [("fw", P), ("bw", P), ("iv", P), ("lut", P), ("lo", F), ("hi", F),
+                ("inv_cell", F), ("coef_scale", F), ("ncell", I), ("nintervals", I)]
 
 
 def call(name: str, *args) -> int:

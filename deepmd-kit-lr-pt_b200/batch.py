@@ -153,7 +153,7 @@ class BatchEvaluator:
                             for t in range(cfg.ntypes)])
         per_frame = np.array([np.bincount(t, minlength=cfg.ntypes) @ const_t for t in ft.types])
         self.e_const = torch.tensor(per_frame, dtype=f64, device=dev)
-        self.ptab = PipelineTables(params, dev, table_degree)
+        self.ptab = PipelineTables(params, dev, table_degree, N)
         self.graph = None
         self.plan = None
         if fused is None:
@@ -190,7 +190,7 @@ class BatchEvaluator:
         pt = self.ptab
         d.tables = ctypes.cast(pt.ptrs, _P)
         d.table_info = pt.info.ctypes.data
-        d.table_degree, d.M, d.naxis = pt.degree, M, ax
+        d.table_degree, d.M, d.naxis = pt.layout, M, ax
         d.type_rows, d.ntypes = fit.type_rows.ctypes.data, fit.ntypes
         E = fit
 
@@ -218,6 +218,8 @@ class BatchEvaluator:
         self._desc = d
         handle = ctypes.c_void_p()
         call("dpb_bt_step_create", ctypes.byref(handle), ctypes.byref(d))
+        if pt.nets is not None:
+            call("dpb_bt_step_set_nets", handle, pt.nets, ptr(pt.touched))
         self._split = _capi.lib().dpb_tune_get(b"batch_fused_split") != 0
         self.plan = handle
 
@@ -264,12 +266,9 @@ class BatchEvaluator:
              ctypes.c_float(cfg.rcut), ctypes.c_float(cfg.rcut_smth), cfg.sec.ctypes.data,
              cfg.sec.size, ptr(self.status), s)
         pt = self.ptab
-        call(pt.fwd, ptr(self.xyz), ptr(self.D), ptr(self.drow), ptr(self.em), pt.ptrs,
-             pt.info.ctypes.data, cfg.sec.ctypes.data, cfg.sec.size, N, M, ax, s)
+        pt.forward(self.xyz, self.D, self.drow, self.em, cfg.sec, N, M, ax, s)
         self.fit.layers(self.D, self.dD)
-        call(pt.bwd, ptr(self.net_deriv), ptr(self.dD), ptr(self.drow), ptr(self.xyz),
-             ptr(self.em), pt.ptrs, pt.info.ctypes.data, cfg.sec.ctypes.data, cfg.sec.size, N,
-             M, ax, s)
+        pt.backward(self.net_deriv, self.dD, self.drow, self.xyz, self.em, cfg.sec, N, M, ax, s)
         call("dpb_batch_force_virial_a", ptr(self.force), ptr(self.virial),
              ptr(self.net_deriv), ptr(self.cw), ptr(self.type), ptr(self.std),
              ptr(self.nlist), ptr(self.atom_off), ptr(self.cell_off), ptr(self.box),

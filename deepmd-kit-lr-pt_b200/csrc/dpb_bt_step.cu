@@ -36,6 +36,7 @@
 #include <algorithm>
 
 #include "dpb_batch_dev.cuh"
+#include "dpb_cheb_dev.cuh"
 #include "dpb_desc_dev.cuh"
 #include "dpb_gemm_dev.cuh"
 
@@ -69,6 +70,8 @@ struct BtStepArgs {
   BtFrames fr;
   BtSec sec;
   TypeTables tt;
+  ChebTables ct;      // piecewise Chebyshev nets (rows then go in groups of four)
+  unsigned* touched;
   double* cw;
   int* cell_of;
   int* cell_start;
@@ -181,6 +184,35 @@ __device__ __forceinline__ void bs_row_bwd(const BtStepArgs& a, int row, int lan
                            a.naxis, a.inv_nnei);
 }
 
+// The same passes for CHEB_A rows by a group of as many warps, on the
+// piecewise Chebyshev nets (two groups per CTA; each has its own half of the
+// row shared memory and its own named barrier).
+constexpr int BS_BAR0 = 8;
+
+template <bool COH>
+__device__ __forceinline__ void bs_rows_fwd(const BtStepArgs& a, int row, int warp, int lane,
+                                            float* gsm) {
+  cheb_fwd_group<BS_CH, 6, COH>(row, a.nrows, warp % CHEB_A, lane, BS_BAR0 + warp / CHEB_A, gsm,
+                                a.xyz, a.D, a.drow, a.em, a.ct, a.tt, a.M, a.naxis, a.inv_nnei,
+                                a.touched);
+}
+
+__device__ __forceinline__ void bs_rows_bwd(const BtStepArgs& a, int row, int warp, int lane,
+                                            float* gsm) {
+  cheb_bwd_group<BS_CH, 6>(row, a.nrows, warp % CHEB_A, lane, BS_BAR0 + warp / CHEB_A, gsm,
+                           a.net_deriv, a.dD, a.drow, a.xyz, a.em, a.ct, a.tt, a.M, a.naxis,
+                           a.inv_nnei, a.touched);
+}
+
+// next group of rows for the group of warps
+__device__ __forceinline__ int bs_next_group(unsigned* counter, int warp, int lane, int* s_row) {
+  const int bar = BS_BAR0 + warp / CHEB_A;
+  cheb_sync(bar);
+  if (warp % CHEB_A == 0 && lane == 0) *s_row = (int)atomicAdd(counter, 1u) * CHEB_A;
+  cheb_sync(bar);
+  return *s_row;
+}
+
 template <bool COH>
 __device__ __forceinline__ void bs_row_force(const BtStepArgs& a, int row, int lane) {
   bt_force_row<float, COH>(row, lane, a.force, a.virial, a.net_deriv, a.cw, a.type, a.std_,
@@ -193,13 +225,15 @@ __device__ __forceinline__ void bs_gemm(const BtStepArgs& a, int l, unsigned cha
   gemm_run<CfgBS, MODE, true>(a.maps[l], a.shp[l], a.epi[l], a.status, smem, bars, tmem);
 }
 
-template <int NC>
+// CHEB: the descriptor passes on the piecewise Chebyshev nets; a work item is
+// then CHEB_A rows for a group of as many warps
+template <int NC, bool CHEB>
 __global__ void __launch_bounds__(BS_THREADS, 1) k_bt_step(const __grid_constant__ BtStepArgs a) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ GemmBars bars[BS_PASSES];
   __shared__ uint32_t tmem_slot;
-  __shared__ int s_ok, s_item;
+  __shared__ int s_ok, s_item, s_rows[BS_WARPS / CHEB_A];
   __shared__ double s_part[BS_WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 1) tmem_alloc_all(&tmem_slot);
@@ -210,6 +244,8 @@ __global__ void __launch_bounds__(BS_THREADS, 1) k_bt_step(const __grid_constant
   const int nrows = a.nrows, F = a.fr.nframes;
   const int gthreads = gridDim.x * BS_THREADS, gtid = blockIdx.x * BS_THREADS + threadIdx.x;
   float* wsm = reinterpret_cast<float*>(smem) + (size_t)warp * a.wsm_floats;
+  float* gsm = wsm - (size_t)(warp % CHEB_A) * a.wsm_floats;  // the group's share
+  int* s_row = &s_rows[warp / CHEB_A];
   unsigned k = 0;
   bs_stamp(a, 0);
 
@@ -225,24 +261,42 @@ __global__ void __launch_bounds__(BS_THREADS, 1) k_bt_step(const __grid_constant
 
   // ---- P1: env rows + descriptor forward
   if (ok) {
-    for (int row = bs_next_row(a.sync + 1, lane); row < nrows;
-         row = bs_next_row(a.sync + 1, lane)) {
-      bs_row_env(a, row, lane, wsm);
-      __syncwarp();
-      if (!a.split_rows) {
-        bs_row_fwd<NC, true>(a, row, lane, wsm);
+    if constexpr (CHEB) {
+      for (int r0 = bs_next_group(a.sync + 1, warp, lane, s_row); r0 < nrows;
+           r0 = bs_next_group(a.sync + 1, warp, lane, s_row)) {
+        if (r0 + warp % CHEB_A < nrows) bs_row_env(a, r0 + warp % CHEB_A, lane, wsm);
+        if (!a.split_rows) {
+          cheb_sync(BS_BAR0 + warp / CHEB_A);  // the env pass's buffers
+          bs_rows_fwd<true>(a, r0, warp, lane, gsm);
+        }
+      }
+    } else {
+      for (int row = bs_next_row(a.sync + 1, lane); row < nrows;
+           row = bs_next_row(a.sync + 1, lane)) {
+        bs_row_env(a, row, lane, wsm);
         __syncwarp();
+        if (!a.split_rows) {
+          bs_row_fwd<NC, true>(a, row, lane, wsm);
+          __syncwarp();
+        }
       }
     }
     if (a.split_rows) {
       ok = bs_sync(a, ++k, &s_ok);
       bs_stamp(a, k);
-      if (ok)
-        for (int row = bs_next_row(a.sync + 2, lane); row < nrows;
-             row = bs_next_row(a.sync + 2, lane)) {
-          bs_row_fwd<NC, false>(a, row, lane, wsm);
-          __syncwarp();
+      if (ok) {
+        if constexpr (CHEB) {
+          for (int r0 = bs_next_group(a.sync + 2, warp, lane, s_row); r0 < nrows;
+               r0 = bs_next_group(a.sync + 2, warp, lane, s_row))
+            bs_rows_fwd<false>(a, r0, warp, lane, gsm);
+        } else {
+          for (int row = bs_next_row(a.sync + 2, lane); row < nrows;
+               row = bs_next_row(a.sync + 2, lane)) {
+            bs_row_fwd<NC, false>(a, row, lane, wsm);
+            __syncwarp();
+          }
         }
+      }
     }
     bs_smem_switch();
     ok = bs_sync(a, ++k, &s_ok);
@@ -288,13 +342,24 @@ __global__ void __launch_bounds__(BS_THREADS, 1) k_bt_step(const __grid_constant
       bt_energy_frame<float>(f, a.energy, a.e_rows, a.drow, a.e_const, a.fr, s_part);
       __syncthreads();
     }
-    for (int row = bs_next_row(a.sync + 3, lane); row < nrows;
-         row = bs_next_row(a.sync + 3, lane)) {
-      bs_row_bwd<NC>(a, row, lane, wsm);
-      __syncwarp();
-      if (!a.split_rows) {
-        bs_row_force<true>(a, row, lane);
+    if constexpr (CHEB) {
+      for (int r0 = bs_next_group(a.sync + 3, warp, lane, s_row); r0 < nrows;
+           r0 = bs_next_group(a.sync + 3, warp, lane, s_row)) {
+        bs_rows_bwd(a, r0, warp, lane, gsm);
+        if (!a.split_rows && r0 + warp % CHEB_A < nrows) {
+          __syncwarp();
+          bs_row_force<true>(a, r0 + warp % CHEB_A, lane);
+        }
+      }
+    } else {
+      for (int row = bs_next_row(a.sync + 3, lane); row < nrows;
+           row = bs_next_row(a.sync + 3, lane)) {
+        bs_row_bwd<NC>(a, row, lane, wsm);
         __syncwarp();
+        if (!a.split_rows) {
+          bs_row_force<true>(a, row, lane);
+          __syncwarp();
+        }
       }
     }
     if (a.split_rows) {
@@ -325,9 +390,43 @@ __global__ void __launch_bounds__(BS_THREADS, 1) k_bt_step(const __grid_constant
 struct BtStepPlan {
   BtStepArgs a;
   int nc;
+  bool cheb;
   int grid;
   size_t smem;
 };
+
+static const void* bs_kernel(int nc, bool cheb) {
+  return cheb      ? (const void*)k_bt_step<6, true>
+         : nc == 4 ? (const void*)k_bt_step<4, false>
+                   : (const void*)k_bt_step<6, false>;
+}
+
+// shared memory of the launch when a warp's row passes take wf floats, set on
+// the kernel with the smallest carve-out that holds it (the rest is L1)
+static int bs_set_smem(BtStepArgs& a, int nc, bool cheb, size_t wf, size_t& smem) {
+  wf = (std::max(wf, (sizeof(BtEnvSmem) + 3) / 4) + 3) / 4 * 4;
+  smem = std::max({(size_t)CfgBS::SMEM, wf * 4 * BS_WARPS + 1024,
+                   (size_t)4 * (BT_MAXCELLS + 1) + 1024});
+  if (smem + 4096 > 232448) {
+    set_error("bt_step: the per-warp descriptor staging (%zu B) does not fit", wf * 4);
+    return DPB_ERR_INVALID;
+  }
+  const void* fn = bs_kernel(nc, cheb);
+  DPB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+           "bt_step");
+  const int pct = (int)std::min<size_t>(100, ((smem + 4096) * 100 + 233471) / 233472);
+  DPB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct),
+           "bt_step");
+  int per_sm = 0;
+  DPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, BS_THREADS, smem),
+           "bt_step");
+  if (per_sm < 1) {
+    set_error("bt_step: the step kernel does not fit on an SM");
+    return DPB_ERR_INVALID;
+  }
+  a.wsm_floats = (int)wf;
+  return DPB_OK;
+}
 
 
 }  // namespace dpb
@@ -367,15 +466,6 @@ int dpb_bt_step_create(void** plan, const dpb_bt_step_desc* d) {
     return DPB_ERR_INVALID;
   }
   const int nnei = a.sec.nnei;
-  size_t wf = std::max(fwd_smem_floats(d->M, nnei), bwd_smem_floats(d->M, nnei, d->naxis));
-  wf = std::max(wf, (sizeof(BtEnvSmem) + 3) / 4);
-  wf = (wf + 3) / 4 * 4;
-  const size_t smem = std::max({(size_t)CfgBS::SMEM, wf * 4 * BS_WARPS + 1024,
-                                (size_t)4 * (BT_MAXCELLS + 1) + 1024});
-  if (smem + 4096 > 232448) {
-    set_error("bt_step: the per-warp descriptor staging (%zu B) does not fit", wf * 4);
-    return DPB_ERR_INVALID;
-  }
   // the six fitting GEMMs, in the order and with the epilogues of the step
   static const int modes[BS_PASSES] = {EPI_TANH, EPI_RES_DT, EPI_LAST,
                                        EPI_BWD_DT, EPI_BWD_RES, EPI_STORE};
@@ -427,7 +517,6 @@ int dpb_bt_step_create(void** plan, const dpb_bt_step_desc* d) {
   a.nrows = d->nrows;
   a.M = d->M;
   a.naxis = d->naxis;
-  a.wsm_floats = (int)wf;
   a.inv_nnei = 1.f / (float)nnei;
   a.rcut = d->rcut;
   a.rcut_smth = d->rcut_smth;
@@ -438,26 +527,42 @@ int dpb_bt_step_create(void** plan, const dpb_bt_step_desc* d) {
     return DPB_ERR_INVALID;
   }
   const int nc = d->table_degree + 1;
-  const void* fn = nc == 4 ? (const void*)k_bt_step<4> : (const void*)k_bt_step<6>;
-  DPB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-           "bt_step");
-  // the smallest shared-memory carve-out that holds it: the rest is L1
-  const int pct = (int)std::min<size_t>(100, ((smem + 4096) * 100 + 233471) / 233472);
-  DPB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct),
-           "bt_step");
-  int per_sm = 0;
-  DPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, BS_THREADS, smem),
-           "bt_step");
-  if (per_sm < 1) {
-    set_error("bt_step: the step kernel does not fit on an SM");
-    return DPB_ERR_INVALID;
-  }
+  size_t smem = 0;
+  if ((rc = bs_set_smem(a, nc, false,
+                        std::max(fwd_smem_floats(d->M, nnei),
+                                 bwd_smem_floats(d->M, nnei, d->naxis)),
+                        smem)))
+    return rc;
   BtStepPlan* p = new BtStepPlan;
   p->a = a;
   p->nc = nc;
+  p->cheb = false;
   p->grid = sm_count();
   p->smem = smem;
   *plan = p;
+  return DPB_OK;
+}
+
+int dpb_bt_step_set_nets(void* plan, const dpb_cheb_net* nets, unsigned* touched) {
+  BtStepPlan* p = static_cast<BtStepPlan*>(plan);
+  if (p == nullptr || p->nc != 6) {
+    set_error("bt_step_set_nets: needs a plan with quintic tables");
+    return DPB_ERR_INVALID;
+  }
+  ChebTables ct;
+  int rc = make_cheb(ct, nets, p->a.tt.ntypes, p->a.tt.sec);
+  if (rc) return rc;
+  size_t smem = 0;
+  if ((rc = bs_set_smem(p->a, p->nc, true,
+                        (std::max(cheb_fwd_floats(p->a.M, ct.wstride),
+                                  cheb_bwd_floats(p->a.M, p->a.naxis, ct.rmax)) +
+                         CHEB_A - 1) / CHEB_A,
+                        smem)))
+    return rc;
+  p->a.ct = ct;
+  p->a.touched = touched;
+  p->cheb = true;
+  p->smem = smem;
   return DPB_OK;
 }
 
@@ -470,8 +575,7 @@ int dpb_bt_step_launch(const void* plan, dpb_stream_t stream) {
   cudaStream_t st = as_stream(stream);
   DPB_CUDA(cudaMemsetAsync(p->a.sync, 0, 8 * sizeof(unsigned), st), "bt_step");
   void* args[] = {(void*)&p->a};
-  const void* fn = p->nc == 4 ? (const void*)k_bt_step<4> : (const void*)k_bt_step<6>;
-  DPB_CUDA(cudaLaunchCooperativeKernel(fn, dim3(p->grid), dim3(BS_THREADS), args, p->smem, st),
+  DPB_CUDA(cudaLaunchCooperativeKernel(bs_kernel(p->nc, p->cheb), dim3(p->grid), dim3(BS_THREADS), args, p->smem, st),
            "bt_step");
   return DPB_OK;
 }

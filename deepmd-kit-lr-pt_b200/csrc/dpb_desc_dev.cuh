@@ -267,17 +267,23 @@ __device__ __forceinline__ void write_descriptor(float* __restrict__ Dr, const f
     // run of 16-byte stores, and reads x[k, m] once per row and lane
     const int lpr = naxis >> 2, rpi = 32 / lpr;
     const int a = (lane % lpr) * 4, mr = lane / lpr;
-    float4 xa[4];
+    float2 xa[4], xb[4];  // columns a, a + 1 and a + 2, a + 3
 #pragma unroll
-    for (int k = 0; k < 4; ++k) xa[k] = *reinterpret_cast<const float4*>(sx + k * M + a);
+    for (int k = 0; k < 4; ++k) {
+      const float4 v = *reinterpret_cast<const float4*>(sx + k * M + a);
+      xa[k] = make_float2(v.x, v.y);
+      xb[k] = make_float2(v.z, v.w);
+    }
     for (int m = mr; m < M; m += rpi) {
-      const float x0 = sx[m], x1 = sx[M + m], x2 = sx[2 * M + m], x3 = sx[3 * M + m];
-      float4 o;
-      o.x = x0 * xa[0].x + x1 * xa[1].x + x2 * xa[2].x + x3 * xa[3].x;
-      o.y = x0 * xa[0].y + x1 * xa[1].y + x2 * xa[2].y + x3 * xa[3].y;
-      o.z = x0 * xa[0].z + x1 * xa[1].z + x2 * xa[2].z + x3 * xa[3].z;
-      o.w = x0 * xa[0].w + x1 * xa[1].w + x2 * xa[2].w + x3 * xa[3].w;
-      *reinterpret_cast<float4*>(Dr + m * naxis + a) = o;
+      float2 xm = f2(sx[m]);
+      float2 o01 = __fmul2_rn(xm, xa[0]), o23 = __fmul2_rn(xm, xb[0]);
+#pragma unroll
+      for (int k = 1; k < 4; ++k) {
+        xm = f2(sx[k * M + m]);
+        o01 = __ffma2_rn(xm, xa[k], o01);
+        o23 = __ffma2_rn(xm, xb[k], o23);
+      }
+      *reinterpret_cast<float4*>(Dr + m * naxis + a) = make_float4(o01.x, o01.y, o23.x, o23.y);
     }
   } else if (32 % naxis == 0) {  // fixed column a per lane, 32 / naxis rows per pass
     const int per = 32 / naxis, a = lane % naxis;
@@ -396,18 +402,16 @@ __device__ __forceinline__ void bwd_slot(float (&P)[4], const Coef4<NC>& c, cons
   }
 }
 
-template <int CH, int NC>
-__device__ __forceinline__ void desc_bwd_atom(int i, int lane, float* wsm, float* __restrict__ net_deriv, const float* __restrict__ dD,
-           const int* __restrict__ drow, const float* __restrict__ xyz,
-           const float* __restrict__ em, TypeTables tt, int M, int naxis,
-           float inv_nnei) {
-  const int nnei = tt.nnei;
-  float* s_x = wsm;                // [4][M]
-  float* s_t = s_x + 4 * M;        // [4][naxis]
-  // the atom's dD tile transposed, [naxis][M]: a lane's four channels of one
-  // column a are one 16-byte read (M % 4 == 0), conflict-free across lanes;
-  // later the slot staging
-  float* s_d = s_t + 4 * MAXAX;
+// dxyz of one center atom, this lane's four channels: dyr[channel][env column]
+// = inv_nnei (sum_a dD[m, a] x[k, a] + [m < naxis] sum_m' dD[m', a = m] x[k, m']).
+// s_x [4][M], s_t [4][naxis]; s_d: the atom's dD tile transposed, [naxis][M]: a
+// lane's four channels of one column a are one 16-byte read (M % 4 == 0),
+// conflict-free across lanes.
+__device__ __forceinline__ void bwd_dyr(float (&dyr)[4][4], int i, int lane, float* s_x,
+                                        float* s_t, float* s_d, const float* __restrict__ dD,
+                                        const int* __restrict__ drow,
+                                        const float* __restrict__ xyz, int M, int naxis,
+                                        float inv_nnei) {
   const float* xi = xyz + (size_t)i * 4 * M;
   const unsigned long long pol = l2_policy_first();
   const float* dr = dD + (size_t)drow[i] * M * naxis;
@@ -448,21 +452,18 @@ __device__ __forceinline__ void desc_bwd_atom(int i, int lane, float* wsm, float
     const float* xa = s_x + k * M;
     const float* xb = s_x + (k + 2) * M;
     const float* da = s_d + a * M;
-    float acc0 = 0.f, acc1 = 0.f;
+    float2 p0 = f2(0.f), p1 = f2(0.f);  // even and odd channels
     for (int mp = 0; mp < M; mp += 4) {
       const float4 u = *reinterpret_cast<const float4*>(xa + mp);
       const float4 v = *reinterpret_cast<const float4*>(xb + mp);
       const float4 dv = *reinterpret_cast<const float4*>(da + mp);
-      const float d0 = dv.x, d1 = dv.y, d2 = dv.z, d3 = dv.w;
-      acc0 += d0 * u.x;
-      acc1 += d0 * v.x;
-      acc0 += d1 * u.y;
-      acc1 += d1 * v.y;
-      acc0 += d2 * u.z;
-      acc1 += d2 * v.z;
-      acc0 += d3 * u.w;
-      acc1 += d3 * v.w;
+      const float2 d01 = make_float2(dv.x, dv.y), d23 = make_float2(dv.z, dv.w);
+      p0 = __ffma2_rn(d01, make_float2(u.x, u.y), p0);
+      p1 = __ffma2_rn(d01, make_float2(v.x, v.y), p1);
+      p0 = __ffma2_rn(d23, make_float2(u.z, u.w), p0);
+      p1 = __ffma2_rn(d23, make_float2(v.z, v.w), p1);
     }
+    const float acc0 = p0.x + p0.y, acc1 = p1.x + p1.y;
     s_t[lane] = acc0;
     s_t[lane + 32] = acc1;
   } else {
@@ -477,25 +478,29 @@ __device__ __forceinline__ void desc_bwd_atom(int i, int lane, float* wsm, float
   // dxyz[k, m] = sum_a dD[m, a] x[k, a] + [m < naxis] T[k, m]
   const int m0 = 4 * lane;
   const bool act = m0 < M;
-  float dyr[4][4];
+  float2 c01[4], c23[4];  // channel pairs
 #pragma unroll
-  for (int ch = 0; ch < 4; ++ch)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) dyr[ch][k] = 0.f;
+  for (int k = 0; k < 4; ++k) c01[k] = c23[k] = f2(0.f);
   if (act) {
     for (int a = 0; a < naxis; ++a) {
-      const float x0 = s_x[a], x1 = s_x[M + a], x2 = s_x[2 * M + a], x3 = s_x[3 * M + a];
       const float4 g4 = *reinterpret_cast<const float4*>(s_d + a * M + m0);
-      const float gch[4] = {g4.x, g4.y, g4.z, g4.w};
+      const float2 g01 = make_float2(g4.x, g4.y), g23 = make_float2(g4.z, g4.w);
 #pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        const float g = gch[ch];
-        dyr[ch][0] += g * x0;
-        dyr[ch][1] += g * x1;
-        dyr[ch][2] += g * x2;
-        dyr[ch][3] += g * x3;
+      for (int k = 0; k < 4; ++k) {
+        const float2 xk = f2(s_x[k * M + a]);
+        c01[k] = __ffma2_rn(g01, xk, c01[k]);
+        c23[k] = __ffma2_rn(g23, xk, c23[k]);
       }
     }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    dyr[0][k] = c01[k].x;
+    dyr[1][k] = c01[k].y;
+    dyr[2][k] = c23[k].x;
+    dyr[3][k] = c23[k].y;
+  }
+  if (act) {
 #pragma unroll
     for (int ch = 0; ch < 4; ++ch) {
       const int m = m0 + ch;
@@ -506,6 +511,21 @@ __device__ __forceinline__ void desc_bwd_atom(int i, int lane, float* wsm, float
       }
     }
   }
+}
+
+template <int CH, int NC>
+__device__ __forceinline__ void desc_bwd_atom(int i, int lane, float* wsm, float* __restrict__ net_deriv, const float* __restrict__ dD,
+           const int* __restrict__ drow, const float* __restrict__ xyz,
+           const float* __restrict__ em, TypeTables tt, int M, int naxis,
+           float inv_nnei) {
+  const int nnei = tt.nnei;
+  float* s_x = wsm;                // [4][M]
+  float* s_t = s_x + 4 * M;        // [4][naxis]
+  float* s_d = s_t + 4 * MAXAX;    // the dD tile, later the slot staging
+  float dyr[4][4];
+  bwd_dyr(dyr, i, lane, s_x, s_t, s_d, dD, drow, xyz, M, naxis, inv_nnei);
+  const int m0 = 4 * lane;
+  const bool act = m0 < M;
   float2 dyr01[4], dyr23[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {

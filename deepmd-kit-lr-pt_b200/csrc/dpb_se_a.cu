@@ -24,6 +24,7 @@
 #include "dpb_common.cuh"
 #include "dpb_envmath.cuh"
 #include "dpb_internal.cuh"
+#include "dpb_cheb_dev.cuh"
 #include "dpb_desc_dev.cuh"
 
 namespace dpb {
@@ -199,6 +200,37 @@ k_desc_bwd(float* __restrict__ net_deriv, const float* __restrict__ dD,
   if (i >= nloc) return;
   float* wsm = reinterpret_cast<float*>(dsm4) + (size_t)w * warp_floats;
   desc_bwd_atom<CH, NC>(i, lane, wsm, net_deriv, dD, drow, xyz, em, tt, M, naxis, inv_nnei);
+}
+
+// The two passes on piecewise Chebyshev embeddings: a CTA of eight warps per
+// group of eight atoms (dpb_cheb_dev.cuh).
+template <int CH, int NC>
+__global__ void __launch_bounds__(CHEB_A * 32, 4)
+k_desc_fwd_cheb(float* __restrict__ xyz_out, float* __restrict__ D,
+                const int* __restrict__ drow, const float* __restrict__ em,
+                const __grid_constant__ ChebTables ct, const __grid_constant__ TypeTables tt,
+                int nloc, int M, int naxis, float inv_nnei, unsigned* touched) {
+  extern __shared__ float4 dsm4[];
+  pdl_wait();
+  pdl_trigger();
+  cheb_fwd_group<CH, NC>(blockIdx.x * CHEB_A, nloc, threadIdx.x >> 5, threadIdx.x & 31, 0,
+                         reinterpret_cast<float*>(dsm4), xyz_out, D, drow, em, ct, tt, M, naxis,
+                         inv_nnei, touched);
+}
+
+template <int CH, int NC>
+__global__ void __launch_bounds__(CHEB_A * 32, 2)
+k_desc_bwd_cheb(float* __restrict__ net_deriv, const float* __restrict__ dD,
+                const int* __restrict__ drow, const float* __restrict__ xyz,
+                const float* __restrict__ em, const __grid_constant__ ChebTables ct,
+                const __grid_constant__ TypeTables tt, int nloc, int M, int naxis,
+                float inv_nnei, const unsigned* touched) {
+  extern __shared__ float4 dsm4[];
+  pdl_wait();
+  pdl_trigger();
+  cheb_bwd_group<CH, NC>(blockIdx.x * CHEB_A, nloc, threadIdx.x >> 5, threadIdx.x & 31, 0,
+                         reinterpret_cast<float*>(dsm4), net_deriv, dD, drow, xyz, em, ct, tt, M,
+                         naxis, inv_nnei, touched);
 }
 
 template <typename T>
@@ -510,9 +542,82 @@ static int desc_bwd(float* net_deriv, const float* d_descrpt, const int* descrpt
   }
 }
 
+// checks shared by the descriptor entry points on piecewise Chebyshev embeddings
+static int cheb_args(TypeTables& tt, ChebTables& ct, const float* const* tables,
+                     const float* table_info, const dpb_cheb_net* nets, const int* sec, int nsec,
+                     int M, int naxis) {
+  int rc = make_tables(tt, tables, table_info, sec, nsec, M);
+  if (rc) return rc;
+  if (naxis <= 0 || naxis > MAXAX || naxis > M) {
+    set_error("se_a descriptor: axis_neuron must be in [1, min(%d, M)]", MAXAX);
+    return DPB_ERR_INVALID;
+  }
+  return make_cheb(ct, nets, nsec - 1, sec);
+}
+
+static int desc_fwd_cheb(float* xyz, float* descrpt, const int* descrpt_row, const float* em,
+                         const float* const* tables, const float* table_info,
+                         const dpb_cheb_net* nets, unsigned* touched, const int* sec, int nsec,
+                         int nloc, int M, int naxis, cudaStream_t st) {
+  TypeTables tt;
+  ChebTables ct;
+  int rc = cheb_args(tt, ct, tables, table_info, nets, sec, nsec, M, naxis);
+  if (rc || nloc <= 0) return rc;
+  const float inv = tt.nnei > 0 ? 1.f / (float)tt.nnei : 0.f;
+  const size_t smem = sizeof(float) * cheb_fwd_floats(M, ct.wstride);
+  auto kern = k_desc_fwd_cheb<3, 6>;
+  DPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+           "se_a_descriptor_fwd_cheb");
+  DPB_CUDA(launch_pdl(kern, dim3(ceil_div(nloc, CHEB_A)), dim3(CHEB_A * 32), smem, st, xyz,
+                      descrpt, descrpt_row, em, ct, tt, nloc, M, naxis, inv, touched),
+           "se_a_descriptor_fwd_cheb");
+  return DPB_OK;
+}
+
+static int desc_bwd_cheb(float* net_deriv, const float* d_descrpt, const int* descrpt_row,
+                         const float* xyz, const float* em, const float* const* tables,
+                         const float* table_info, const dpb_cheb_net* nets,
+                         const unsigned* touched, const int* sec, int nsec, int nloc, int M,
+                         int naxis, cudaStream_t st) {
+  TypeTables tt;
+  ChebTables ct;
+  int rc = cheb_args(tt, ct, tables, table_info, nets, sec, nsec, M, naxis);
+  if (rc || nloc <= 0) return rc;
+  const float inv = tt.nnei > 0 ? 1.f / (float)tt.nnei : 0.f;
+  const size_t smem = sizeof(float) * cheb_bwd_floats(M, naxis, ct.rmax);
+  auto kern = k_desc_bwd_cheb<3, 6>;
+  DPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+           "se_a_descriptor_bwd_cheb");
+  DPB_CUDA(launch_pdl(kern, dim3(ceil_div(nloc, CHEB_A)), dim3(CHEB_A * 32), smem, st, net_deriv,
+                      d_descrpt, descrpt_row, xyz, em, ct, tt, nloc, M, naxis, inv, touched),
+           "se_a_descriptor_bwd_cheb");
+  return DPB_OK;
+}
+
 }  // namespace dpb
 
 extern "C" {
+
+int dpb_se_a_descriptor_fwd_cheb_f32(float* xyz, float* descrpt, const int* descrpt_row,
+                                     const float* em, const float* const* tables,
+                                     const float* table_info, const dpb_cheb_net* nets,
+                                     unsigned* touched, const int* sec, int nsec, int nloc,
+                                     int last_layer_size, int axis_neuron,
+                                     dpb_stream_t stream) {
+  return desc_fwd_cheb(xyz, descrpt, descrpt_row, em, tables, table_info, nets, touched, sec,
+                       nsec, nloc, last_layer_size, axis_neuron, as_stream(stream));
+}
+
+int dpb_se_a_descriptor_bwd_cheb_f32(float* net_deriv, const float* d_descrpt,
+                                     const int* descrpt_row, const float* xyz, const float* em,
+                                     const float* const* tables, const float* table_info,
+                                     const dpb_cheb_net* nets, const unsigned* touched,
+                                     const int* sec, int nsec, int nloc, int last_layer_size,
+                                     int axis_neuron, dpb_stream_t stream) {
+  return desc_bwd_cheb(net_deriv, d_descrpt, descrpt_row, xyz, em, tables, table_info, nets,
+                       touched, sec, nsec, nloc, last_layer_size, axis_neuron,
+                       as_stream(stream));
+}
 
 int dpb_se_a_descriptor_fwd_f32(float* xyz, float* descrpt, const int* descrpt_row,
                                 const float* em, const float* const* tables,

@@ -62,7 +62,7 @@ class ForwardLower:
         self.status = z(1, torch.int32)
         self.avg = torch.tensor(params.davg, dtype=f32, device=dev)
         self.std = torch.tensor(params.dstd, dtype=f32, device=dev)
-        self.ptab = PipelineTables(params, dev, table_degree)
+        self.ptab = PipelineTables(params, dev, table_degree, n)
         self.fit = None
         self.nloc = -1
 
@@ -112,12 +112,9 @@ class ForwardLower:
              ctypes.c_float(cfg.rcut), ctypes.c_float(cfg.rcut_smth), sec.ctypes.data, sec.size,
              ptr(self.status), s)
         pt = self.ptab
-        call(pt.fwd, ptr(self.xyz), ptr(self.D), ptr(self.drow), ptr(self.em), pt.ptrs,
-             pt.info.ctypes.data, sec.ctypes.data, sec.size, nloc, M, ax, s)
+        pt.forward(self.xyz, self.D, self.drow, self.em, sec, nloc, M, ax, s)
         self.fit.forward_backward(self.D[:nloc], self.dD[:nloc], energy)
-        call(pt.bwd, ptr(self.net_deriv), ptr(self.dD), ptr(self.drow), ptr(self.xyz),
-             ptr(self.em), pt.ptrs, pt.info.ctypes.data, sec.ctypes.data, sec.size, nloc, M,
-             ax, s)
+        pt.backward(self.net_deriv, self.dD, self.drow, self.xyz, self.em, sec, nloc, M, ax, s)
         call("dpb_force_virial_a_env_mixed_acc", ptr(force), ptr(virial), ptr(self.net_deriv),
              ptr(c), ptr(t), ptr(self.std), ptr(self.nlist), ptr(self.identity), nloc, nall,
              cfg.nnei, cfg.ntypes, ctypes.c_float(cfg.rcut), ctypes.c_float(cfg.rcut_smth), s)

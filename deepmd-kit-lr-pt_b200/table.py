@@ -239,3 +239,123 @@ def cubic_table(table: np.ndarray, info: np.ndarray, stride_mult: int = 1):
     C[K, 0] = y[K]
     C[K, 1] = d[K]
     return C, np.array([lower, mx, mx, h, h, float(K)])
+
+
+CHEB_K = 16          # polynomials per interval (degree 15)
+CHEB_MAX_INTERVALS = 16
+CHEB_CELLS = 32      # lookup cells per unit of x, the finest interval width
+
+
+def chebyshev_net(table: np.ndarray, info: np.ndarray, tol: float = 1.5e-8,
+                  tol_slope: float = 5e-7):
+    """The compressed embedding of one table as a piecewise Chebyshev
+    expansion of degree 15 over the table's fine region [lower, upper), for
+    the tensor-core descriptor kernels (dpb_se_a_descriptor_*_cheb_f32).
+
+    Intervals start at width 8 and are halved until the expansion agrees with
+    the table at every knot and midpoint: the value to tol of the largest
+    |G|, the slope to tol_slope of the largest |G'| (the cubic
+    re-interpolation's own remainder is of that size, and FP32 resolves
+    6e-8). A smooth net needs 6-10 intervals; one that needs more than
+    CHEB_MAX_INTERVALS, or whose bounds are no multiples of the cell width,
+    returns None and stays on the table.
+
+    Returns (C [R, 16, M] float64, centers [R], halfwidths [R], lut
+    [cells] uint8)."""
+    lower, upper, _, s0, _ = (float(v) for v in info[:5])
+    M = table.shape[1] // 6
+    first = int(round((upper - lower) / s0))
+    ncell = (upper - lower) * CHEB_CELLS
+    if (first < 1 or first > table.shape[0] or abs(first * s0 - (upper - lower)) > 1e-9 or
+            ncell != round(ncell) or not 1 <= ncell <= 1 << 16):
+        return None
+    T = np.asarray(table[:first], np.float64).reshape(first, M, 6)
+
+    def poly(rows, t):
+        c = T[rows]
+        t = t[:, None]
+        v, g = c[..., 5], 5.0 * c[..., 5]
+        for p in range(4, -1, -1):
+            v = v * t + c[..., p]
+        for p in range(4, 0, -1):
+            g = g * t + p * c[..., p]
+        return v, g
+
+    knots = np.arange(first)
+    zero, half = np.zeros(first), np.full(first, 0.5 * s0)
+    ref = [poly(knots, zero), poly(knots, half)]
+    big = max(np.abs(v).max() for v, _ in ref)
+    steep = max(np.abs(g).max() for _, g in ref)
+    if not (np.isfinite(big) and np.isfinite(steep)) or big == 0.0:
+        return None
+    k = np.arange(CHEB_K)
+    theta = np.pi * (k + 0.5) / CHEB_K
+    node = np.cos(theta)
+    dct = (2.0 / CHEB_K) * np.cos(k[:, None] * theta[None, :])
+    dct[0] *= 0.5
+
+    def fit(a, b):
+        c, h = 0.5 * (a + b), 0.5 * (b - a)
+        x = c + h * node
+        r = np.clip(((x - lower) / s0).astype(np.int64), 0, first - 1)
+        C = dct @ poly(r, x - (lower + r * s0))[0]
+        for off, (v, g) in zip((0.0, 0.5 * s0), ref):
+            i0 = int(np.ceil((a - lower - off) / s0 - 1e-9))
+            i1 = int(np.ceil((b - lower - off) / s0 - 1e-9))
+            t = (lower + off + np.arange(i0, i1) * s0 - c) / h
+            P = [np.ones_like(t), t]
+            U = [np.ones_like(t), 2 * t]
+            for _ in range(2, CHEB_K):
+                P.append(2 * t * P[-1] - P[-2])
+                U.append(2 * t * U[-1] - U[-2])
+            dP = np.stack([np.zeros_like(t)] + [q * U[q - 1] for q in range(1, CHEB_K)], 1)
+            if i1 > i0 and (np.abs(np.stack(P, 1) @ C - v[i0:i1]).max() > tol * big or
+                            np.abs(dP @ C / h - g[i0:i1]).max() > tol_slope * steep):
+                return None
+        return C
+
+    todo = [(lower + 8.0 * j, min(lower + 8.0 * (j + 1), upper))
+            for j in range(int(np.ceil((upper - lower) / 8.0)))][::-1]
+    out = []
+    while todo:
+        a, b = todo.pop()
+        C = fit(a, b)
+        if C is not None:
+            out.append((a, b, C))
+            if len(out) + len(todo) > CHEB_MAX_INTERVALS:
+                return None
+            continue
+        m = 0.5 * (a + b)
+        if (m - lower) * CHEB_CELLS != round((m - lower) * CHEB_CELLS):
+            return None
+        todo += [(m, b), (a, m)]
+    lut = np.empty(int(ncell), np.uint8)
+    for r, (a, b, _) in enumerate(out):
+        lut[int((a - lower) * CHEB_CELLS):int((b - lower) * CHEB_CELLS)] = r
+    return (np.stack([C for _, _, C in out]), np.array([0.5 * (a + b) for a, b, _ in out]),
+            np.array([0.5 * (b - a) for a, b, _ in out]), lut)
+
+
+def chebyshev_fragments(C: np.ndarray):
+    """(fw, bw, scale): the operand arrays of dpb_cheb_net (uint32, in the
+    order of the tensor cores' B fragments) for coefficients C [R, 16, M]:
+    C * scale as two FP16 terms, scale a power of two."""
+    R, K, M = C.shape
+    scale = 2.0 ** (14 - int(np.ceil(np.log2(np.abs(C).max()))))
+    nt, ks = -(-M // 8), -(-M // 16)
+    X = np.zeros((R, K, ks * 16))
+    X[:, :, :M] = C * scale
+    hi = X.astype(np.float16)
+    lo = (X - hi.astype(np.float64)).astype(np.float16)
+    lane = np.arange(32)
+    g, q = lane >> 2, lane & 3
+    quad = np.stack([2 * q, 2 * q + 1, 2 * q + 8, 2 * q + 9], 1)  # [32, 4]
+
+    def pack(sel):
+        # [..., 32, 4] halves of hi and lo -> 16 bytes per lane
+        return np.ascontiguousarray(np.concatenate([sel(hi), sel(lo)], -1)).view(np.uint32)
+
+    fw = pack(lambda h: np.stack([h[:, quad, (8 * j + g)[:, None]] for j in range(nt)], 1))
+    bw = pack(lambda h: np.stack([np.stack([h[:, (8 * n + g)[:, None], 16 * s + quad]
+                                            for s in range(ks)], 1) for n in range(2)], 1))
+    return fw, bw, scale

@@ -417,6 +417,31 @@ typedef struct {
   const float* const* w;
 } dpb_gemm_layer;
 
+/* One neighbor type's embedding as a piecewise Chebyshev expansion over
+ * [lo, hi) (no counterpart in the reference): on interval r, with
+ * t = (x - iv[2 r]) * iv[2 r + 1] in [-1, 1),
+ *   G(x)[m] = sum_{k < 16} T_k(t) C[r][k][m].
+ * lut[c] is the interval of cell c = int((x - lo) * inv_cell), c < ncell.
+ * C * coef_scale (a power of two; largest entry below 2^15) is stored as two
+ * FP16 terms hi + lo in the operand order of mma.m16n8k16's B fragment, 16
+ * bytes (two hi pairs, two lo pairs) per lane = 4 g + q:
+ *   fw [nintervals][ceil(M/8)][32]: channel 8 j + g of k = 2q, 2q+1 | 2q+8, 2q+9;
+ *   bw [nintervals][2][ceil(M/16)][32]: k = 8 h + g of channels
+ *      16 s + 2q, 2q+1 | 2q+8, 2q+9 (zero beyond M).
+ * fw, bw, iv and lut are device pointers; at most 16 intervals. */
+typedef struct {
+  const void* fw;
+  const void* bw;
+  const float* iv;
+  const unsigned char* lut;
+  float lo;
+  float hi;
+  float inv_cell;
+  float coef_scale;
+  int ncell;
+  int nintervals;
+} dpb_cheb_net;
+
 /* Everything one batched-frames step touches (device buffers unless noted):
  * the frame table and geometry scratch of dpb_batch_env_mat_a_f32, the
  * descriptor tables and buffers of dpb_se_a_descriptor_{fwd,bwd}[_cubic]_f32
@@ -476,6 +501,10 @@ typedef struct {
  * GEMMs, table descriptors); *plan is freed by dpb_bt_step_destroy. The
  * buffers must stay allocated while the plan is used. */
 DPB_API int dpb_bt_step_create(void** plan, const dpb_bt_step_desc* desc);
+/* Runs the plan's descriptor passes on piecewise Chebyshev nets, as
+ * dpb_se_a_descriptor_{fwd,bwd}_cheb_f32 with the plan's quintic tables
+ * (table_degree 5 only); touched as there. */
+DPB_API int dpb_bt_step_set_nets(void* plan, const dpb_cheb_net* nets, unsigned* touched);
 /* One step: env, descriptor, fitting, descriptor backward, forces, virials
  * and energies of every frame in ONE cooperative launch (one CTA per SM),
  * preceded by a 32-byte memset of the barrier and work counters. */
@@ -551,6 +580,23 @@ DPB_API int dpb_se_a_descriptor_bwd_cubic_f32(float* net_deriv, const float* d_d
                                               const float* table_info, const int* sec,
                                               int nsec, int nloc, int last_layer_size,
                                               int axis_neuron, dpb_stream_t stream);
+/* The two descriptor passes on piecewise Chebyshev nets (nets: host array,
+ * one per neighbor type): the sum over the slots is taken in the polynomials
+ * and the channels are products on the tensor cores. Slots whose x lies
+ * outside [lo, hi) are evaluated from tables / table_info, the quintic tables
+ * of dpb_se_a_pack_table_f32. touched (device, [ceil(nloc/8) * (nsec-1)], may be NULL): written by
+ * the forward, the intervals each group of eight atoms uses; the backward of
+ * the same rows evaluates only those (NULL: all). */
+DPB_API int dpb_se_a_descriptor_fwd_cheb_f32(
+    float* xyz, float* descrpt, const int* descrpt_row, const float* em,
+    const float* const* tables, const float* table_info, const dpb_cheb_net* nets,
+    unsigned* touched, const int* sec, int nsec, int nloc, int last_layer_size, int axis_neuron,
+    dpb_stream_t stream);
+DPB_API int dpb_se_a_descriptor_bwd_cheb_f32(
+    float* net_deriv, const float* d_descrpt, const int* descrpt_row, const float* xyz,
+    const float* em, const float* const* tables, const float* table_info,
+    const dpb_cheb_net* nets, const unsigned* touched, const int* sec, int nsec, int nloc,
+    int last_layer_size, int axis_neuron, dpb_stream_t stream);
 /* prod_force_a + prod_virial_a in one pass with FP64 accumulation; ghost
  * forces are added to their owner mapping[j] (force: [nforce, 3], nforce =
  * nloc with a mapping, nall without). atom_virial [nall, 9] may be NULL. */
