@@ -28,6 +28,7 @@
 // library with the elementwise kernels k_fit_*; Adam is k_adam.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "dpb_batch.cuh"
 #include "dpb_envmath.cuh"
@@ -1774,6 +1775,8 @@ static int tr_xbar(T* xb, T* xbd, const T* xyz, const T* xyzd, const T* Dj, cons
 
 }  // namespace dpb
 
+#include "dpb_train_dmma.cuh"
+
 using namespace dpb;
 
 #define DPB_TRAIN_ENTRIES(SUF, T)                                                               \
@@ -1794,6 +1797,8 @@ using namespace dpb;
       set_error("se_a_train_fwd: null buffer");                                                 \
       return DPB_ERR_INVALID;                                                                   \
     }                                                                                           \
+    rc = em_try_fwd<T>(xyz, descrpt, em, net, g, as_stream(stream));                            \
+    if (rc >= 0) return rc;                                                                     \
     auto kern = !tr_std_net(net) ? k_tr_fwd<T, TrTraits<T>::R, 0, 0, 0>                         \
                 : (R == 4 ? k_tr_fwd<T, 4, 25, 50, 100> : k_tr_fwd<T, 8, 25, 50, 100>);\
     int grid;                                                                                   \
@@ -1828,6 +1833,8 @@ using namespace dpb;
     rc = tr_xbar<T>(scratch, nullptr, xyz, nullptr, d_descrpt, nullptr, drow, nrows, net.n3,    \
                     axis, g.nnei, st);                                                          \
     if (rc) return rc;                                                                          \
+    rc = em_try_bwd<T>(net_deriv, em, scratch, net, g, st);                                     \
+    if (rc >= 0) return rc;                                                                     \
     auto kern = !tr_std_net(net) ? k_tr_bwd<T, TrTraits<T>::R, 0, 0, 0>                         \
                 : (R == 4 ? k_tr_bwd<T, 4, 25, 50, 100> : k_tr_bwd<T, 8, 25, 50, 100>);\
     int grid;                                                                                   \

@@ -1,0 +1,589 @@
+// The FP64 embedding passes of the standard net (1 -> 25 -> 50 -> 100) on the
+// FP64 matrix instructions: forward (G, xyz, D) and force backward
+// (dE/d(em)), the same quantities as k_tr_fwd / k_tr_bwd (dpb_train.cu, which
+// includes this file).
+//
+// One warp takes one center atom and 16 neighbor rows at a time through the
+// whole net as mma.m16n8k4 products. The FMA form held one channel per lane
+// and read every operand from shared memory: 8 warps per SM, a third of the
+// FP64 rate. Here the weights lie in shared memory in fragment order and
+// the activations stay in registers between the layers, because the order of
+// a product's k and of its columns is free: lane (g, t) = (lane / 4, lane % 4)
+// owns the layer-1 channels s(j, t) = 4 j + t (j < 7) of rows g and g + 8, and
+// column pair t of layer 2's tile j is the pair s(j, t), s(j, t) + 25, whose
+// residual is that layer-1 channel and which is k = t of layer 3's steps
+// (j, 0) and (j, 1). Layer 3 runs transposed (channels x rows), so its
+// results feed the contraction over rows as A operands. What is left is the
+// FP64 pipe itself: the products at 64 FMA per clock and SM, and 175 tanh per
+// row (tanh_f64 below).
+//
+// Measured, 3,993 atoms: forward 1.17 -> 0.56 ms, backward 2.06 -> 0.91 ms.
+#pragma once
+
+namespace dpb {
+
+constexpr int EM_S1 = 7;                       // layer-1 channels per lane and row
+constexpr int EM_F2 = 7 * 7 * 32;              // fragment doubles: layer 2
+constexpr int EM_F3 = 14 * (6 * 2 + 1) * 32;   // layer 3 (six 16-channel tiles, one of 8)
+constexpr int EM_B3 = 25 * 7 * 32;             // layer 3 adjoint
+constexpr int EM_B2 = 14 * 4 * 32;             // layer 2 adjoint
+constexpr int EM_V = 28 + 28 + 52 + 100;       // W1, b1, b2, b3
+constexpr int EM_FWD_T = EM_F2 + EM_F3 + EM_V;               // per type
+constexpr int EM_BWD_T = EM_F2 + EM_F3 + EM_B3 + EM_B2 + EM_V;
+constexpr int EM_H2S = 50;                     // row stride of the staged layer-2 outputs
+constexpr int EM_TS = 20;                      // row stride of a staged 16 x 16 tile
+constexpr int EM_FWD_W = 16 * 4 + 16 * EM_H2S;               // doubles per warp
+constexpr int EM_BWD_W = 16 * 4 + 400 + 2 * 16 * EM_TS;
+constexpr int EM_FWD_MAXW = 12, EM_BWD_MAXW = 8;
+
+// tanh(x) = E / (E + 2), E = exp(2|x|) - 1 kept as 2^k (e^r - 1) + (2^k - 1),
+// so small arguments keep their relative accuracy: 2|x| = k ln 2 + r, e^r - 1 by
+// its Taylor series to r^13 (|r| <= 0.347: remainder 1e-17), the quotient from
+// a reciprocal estimate, one third-order iteration and one residual
+// correction. Within 2.6 ulp (measured over 1e-9 .. 30); NaN stays NaN.
+__device__ __forceinline__ double tanh_f64(double x) {
+  const double ax = fabs(x);
+  const double y = 2.0 * (ax > 20.0 ? 20.0 : ax);
+  const double magic = 6755399441055744.0;  // 1.5 * 2^52: the sum's low bits are the integer
+  const double kd = fma(y, 1.4426950408889634, magic);
+  const int k = __double2loint(kd);
+  const double kf = kd - magic;
+  // ln 2 as its 40 leading bits and the rest: k times the former is exact
+  double r = fma(-kf, 0.6931471805601177, y);
+  r = fma(-kf, -1.7239444525614835e-13, r);
+  double p = 1.0 / 6227020800.0;  // 1 / 13!
+  p = fma(p, r, 1.0 / 479001600.0);
+  p = fma(p, r, 1.0 / 39916800.0);
+  p = fma(p, r, 1.0 / 3628800.0);
+  p = fma(p, r, 1.0 / 362880.0);
+  p = fma(p, r, 1.0 / 40320.0);
+  p = fma(p, r, 1.0 / 5040.0);
+  p = fma(p, r, 1.0 / 720.0);
+  p = fma(p, r, 1.0 / 120.0);
+  p = fma(p, r, 1.0 / 24.0);
+  p = fma(p, r, 1.0 / 6.0);
+  p = fma(p, r, 0.5);
+  p = fma(r * r, p, r);
+  const double s = __hiloint2double((1023 + k) << 20, 0);
+  const double E = fma(s, p, s - 1.0);
+  const double d = E + 2.0;
+  double q;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(q) : "d"(d));
+  const double e = fma(-d, q, 1.0);
+  q = fma(q, fma(e, e, e), q);
+  double v = E * q;
+  v = fma(fma(-d, v, E), q, v);
+  return copysign(v, x);
+}
+
+__device__ __forceinline__ void dmma16(double (&c)[4], double a0, double a1, double b) {
+  asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
+      "{%0, %1, %2, %3};"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a0), "d"(a1), "d"(b));
+}
+__device__ __forceinline__ void dmma8(double& c0, double& c1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c0), "+d"(c1)
+      : "d"(a), "d"(b));
+}
+
+// layer-2 channel of column / k pair member v owned by lane column u at step j,
+// -1 when the slot is padding
+__device__ __forceinline__ int em_c2(int j, int u, int v) {
+  return 4 * j + u < 25 ? 4 * j + u + 25 * v : -1;
+}
+
+// weights of net t into fragment order
+__device__ inline void em_stage(double* w, const TrNet<double>& net, int t, bool bwd) {
+  double* F2 = w;
+  double* F3 = F2 + EM_F2;
+  double* V = F3 + EM_F3 + (bwd ? EM_B3 + EM_B2 : 0);
+  const double *W2 = net.W[t][1], *W3 = net.W[t][2];
+  const int n = blockDim.x;
+  for (int e = threadIdx.x; e < EM_F2; e += n) {
+    const int lane = e & 31, j = (e >> 5) % 7, s = (e >> 5) / 7, g = lane >> 2;
+    const int k = 4 * s + (lane & 3), c = em_c2(j, g >> 1, g & 1);
+    F2[e] = k < 25 && c >= 0 ? W2[k * 50 + c] : 0.;
+  }
+  for (int e = threadIdx.x; e < EM_F3; e += n) {
+    // tiles 0..5: [tile][step][lane][row g, row g + 8]; tile 6: [step][lane]
+    const bool last = e >= 6 * 14 * 64;
+    const int f = last ? e - 6 * 14 * 64 : e;
+    const int h = last ? 0 : f & 1, lane = last ? f & 31 : (f >> 1) & 31;
+    const int q = last ? f >> 5 : f >> 6;
+    const int step = q % 14, m = (last ? 96 : q / 14 * 16) + 8 * h + (lane >> 2);
+    const int c = em_c2(step >> 1, lane & 3, step & 1);
+    F3[e] = m < 100 && c >= 0 ? W3[c * 100 + m] : 0.;
+  }
+  for (int e = threadIdx.x; e < 28; e += n) {
+    V[e] = e < 25 ? net.W[t][0][e] : 0.;
+    V[28 + e] = e < 25 ? net.b[t][0][e] : 0.;
+  }
+  for (int e = threadIdx.x; e < 50; e += n) V[56 + e] = net.b[t][1][e];
+  for (int e = threadIdx.x; e < 100; e += n) V[108 + e] = net.b[t][2][e];
+  if (!bwd) return;
+  double* B3 = F3 + EM_F3;
+  double* B2 = B3 + EM_B3;
+  for (int e = threadIdx.x; e < EM_B3; e += n) {
+    const int lane = e & 31, j = (e >> 5) % 7, s = (e >> 5) / 7, g = lane >> 2;
+    const int c = em_c2(j, g >> 1, g & 1);
+    B3[e] = c >= 0 ? W3[c * 100 + 4 * s + (lane & 3)] : 0.;
+  }
+  for (int e = threadIdx.x; e < EM_B2; e += n) {
+    const int lane = e & 31, q = (e >> 5) & 3, step = (e >> 5) >> 2, g = lane >> 2;
+    const int c = em_c2(step >> 1, lane & 3, step & 1);
+    const int k = 4 * (2 * q + (g & 1)) + (g >> 1);
+    B2[e] = c >= 0 && k < 25 ? W2[k * 50 + c] : 0.;
+  }
+}
+
+// layers 1 and 2 of 16 rows: h1a / h1b the layer-1 outputs of rows g / g + 8 at
+// the lane's channels, h2[j] the layer-2 outputs (row g: pair members 0, 1;
+// row g + 8: 0, 1), with STAGE stored by row in hs as well
+template <bool STAGE>
+__device__ __forceinline__ void em_layers12(double (&h1a)[EM_S1], double (&h1b)[EM_S1],
+                                            double (&h2)[7][4], double xa, double xb,
+                                            const double* F2, const double* V, double* hs,
+                                            int lane) {
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int s = 0; s < EM_S1; ++s) {
+    const double w = V[4 * s + t], b = V[28 + 4 * s + t];
+    h1a[s] = tanh_f64(fma(xa, w, b));  // padding: tanh(0)
+    h1b[s] = tanh_f64(fma(xb, w, b));
+  }
+#pragma unroll
+  for (int j = 0; j < 7; ++j) {
+    const bool ok = 4 * j + t < 25;
+    h2[j][0] = h2[j][2] = ok ? V[56 + 4 * j + t] : 0.;
+    h2[j][1] = h2[j][3] = ok ? V[56 + 4 * j + t + 25] : 0.;
+  }
+#pragma unroll
+  for (int s = 0; s < EM_S1; ++s)
+#pragma unroll
+    for (int j = 0; j < 7; ++j) dmma16(h2[j], h1a[s], h1b[s], F2[(s * 7 + j) * 32 + lane]);
+#pragma unroll
+  for (int j = 0; j < 7; ++j) {
+    h2[j][0] = tanh_f64(h2[j][0]) + h1a[j];
+    h2[j][1] = tanh_f64(h2[j][1]) + h1a[j];
+    h2[j][2] = tanh_f64(h2[j][2]) + h1b[j];
+    h2[j][3] = tanh_f64(h2[j][3]) + h1b[j];
+    if (STAGE && 4 * j + t < 25) {
+      double* p = hs + g * EM_H2S + 4 * j + t;
+      p[0] = h2[j][0];
+      p[25] = h2[j][1];
+      p[8 * EM_H2S] = h2[j][2];
+      p[8 * EM_H2S + 25] = h2[j][3];
+    }
+  }
+}
+
+// layer 3 of channel tile m, transposed: z[n][..] rows 8 n + 2 t, + 1 of
+// channels 16 m + g ([0], [1]) and + 8 ([2], [3]; absent in tile 6)
+template <int LAST>
+__device__ __forceinline__ void em_layer3(double (&z)[2][4], int m, const double (&h2)[7][4],
+                                          const double* F3, const double* V, int lane) {
+  const int g = lane >> 2, c = 16 * m + g;
+  const double b0 = c < 100 ? V[108 + c] : 0., b1 = LAST ? 0. : V[108 + c + 8];
+#pragma unroll
+  for (int n = 0; n < 2; ++n) {
+    z[n][0] = z[n][1] = b0;
+    z[n][2] = z[n][3] = b1;
+  }
+#pragma unroll
+  for (int j = 0; j < 7; ++j)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const int step = 2 * j + v;
+      if (LAST) {
+        const double a = F3[6 * 14 * 64 + step * 32 + lane];
+        dmma8(z[0][0], z[0][1], a, h2[j][v]);
+        dmma8(z[1][0], z[1][1], a, h2[j][2 + v]);
+      } else {
+        const double2 a = *reinterpret_cast<const double2*>(F3 + ((m * 14 + step) * 32 + lane) * 2);
+        dmma16(z[0], a.x, a.y, h2[j][v]);
+        dmma16(z[1], a.x, a.y, h2[j][2 + v]);
+      }
+    }
+}
+
+// 16 entries of the list from e0 on: env rows (times the multiplicity) to rr
+// [16][4] and each row's x to this lane's rows g, g + 8
+__device__ __forceinline__ void em_rows(double* rr, double& xa, double& xb, const int* ent,
+                                        int e0, int ne, const double* em_row, bool mult,
+                                        int lane) {
+  double x = 0.;
+  if (lane < 16) {
+    double2 u = make_double2(0., 0.), v = u;
+    if (lane < ne) {
+      const int en = ent[e0 + lane];
+      const double2* src = reinterpret_cast<const double2*>(em_row + (size_t)(en & 0xFFFF) * 4);
+      u = src[0];
+      v = src[1];
+      x = u.x;
+      if (mult) {
+        const double mu = (double)(en >> 16);
+        u.x *= mu, u.y *= mu, v.x *= mu, v.y *= mu;
+      }
+    }
+    reinterpret_cast<double2*>(rr)[lane * 2] = u;
+    reinterpret_cast<double2*>(rr)[lane * 2 + 1] = v;
+  }
+  xa = __shfl_sync(0xffffffffu, x, lane >> 2);
+  xb = __shfl_sync(0xffffffffu, x, 8 + (lane >> 2));
+  __syncwarp();
+}
+
+__global__ void __launch_bounds__(32 * EM_FWD_MAXW, 1)
+k_emb_fwd_dmma(double* __restrict__ xyz_out, double* __restrict__ D_out,
+               const double* __restrict__ em, TrNet<double> net, TrGeom g) {
+  extern __shared__ __align__(16) double esm[];
+  pdl_wait();
+  pdl_trigger();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int gr = lane >> 2, t4 = lane & 3;
+  for (int t = 0; t < g.ntypes; ++t) em_stage(esm + (size_t)t * EM_FWD_T, net, t, false);
+  __syncthreads();
+  double* ws = esm + (size_t)g.ntypes * EM_FWD_T + (size_t)w * EM_FWD_W;
+  double* rr = ws;
+  double* hs = ws + 64;
+  int* ent = reinterpret_cast<int*>(esm + (size_t)g.ntypes * EM_FWD_T + (size_t)nw * EM_FWD_W) +
+             (size_t)w * (g.nnei + TR_MAXT + 1);
+  int* secn = ent + g.nnei;
+  for (int row = blockIdx.x * nw + w; row < g.nrows; row += gridDim.x * nw) {
+    tr_entries(ent, secn, g.nlist + (size_t)row * g.nnei, g, g.type[row], true, lane, 0,
+               g.ntypes);
+    double X[7][4];  // xyz: channels 16 m + g (+ 8), env columns 2 t, 2 t + 1 (t < 2)
+#pragma unroll
+    for (int m = 0; m < 7; ++m)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) X[m][k] = 0.;
+    for (int t = 0; t < g.ntypes; ++t) {
+      const double* F2 = esm + (size_t)t * EM_FWD_T;
+      const double* F3 = F2 + EM_F2;
+      const double* V = F3 + EM_F3;
+      for (int e0 = secn[t]; e0 < secn[t + 1]; e0 += 16) {
+        double xa, xb;
+        em_rows(rr, xa, xb, ent, e0, min(16, secn[t + 1] - e0),
+                em + (size_t)row * g.nnei * 4, true, lane);
+        double rb[2][2];  // env column g (< 4) of rows 8 n + 2 t + e
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) rb[n][e] = gr < 4 ? rr[(8 * n + 2 * t4 + e) * 4 + gr] : 0.;
+        double h1a[EM_S1], h1b[EM_S1], h2[7][4];
+        em_layers12<true>(h1a, h1b, h2, xa, xb, F2, V, hs, lane);
+        __syncwarp();
+        auto tile = [&](auto last, int m, double (&x)[4]) {
+          constexpr int LAST = decltype(last)::value;
+          double z[2][4];
+          em_layer3<LAST>(z, m, h2, F3, V, lane);
+          const int c = 16 * m + gr;
+          const int ca = c < 50 ? c : c - 50, cb = c + 8 < 50 ? c + 8 : c - 42;
+#pragma unroll
+          for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const double* hrow = hs + (8 * n + 2 * t4 + e) * EM_H2S;
+              if (LAST) {  // channels 96 .. 99: rows g < 4
+                const double G = gr < 4 ? tanh_f64(z[n][e]) + hrow[gr < 4 ? ca : 0] : 0.;
+                dmma8(x[0], x[1], G, rb[n][e]);
+              } else {
+                const double G0 = tanh_f64(z[n][e]) + hrow[ca];
+                const double G1 = tanh_f64(z[n][2 + e]) + hrow[cb];
+                dmma16(x, G0, G1, rb[n][e]);
+              }
+            }
+        };
+#pragma unroll
+        for (int m = 0; m < 6; ++m) tile(std::integral_constant<int, 0>{}, m, X[m]);
+        tile(std::integral_constant<int, 1>{}, 6, X[6]);
+        __syncwarp();  // rr and hs are rewritten by the next rows
+      }
+    }
+    // xyz / nnei (se_a.py:844), D = xyz^T xyz[:, :ax]
+    const double nn = (double)g.nnei;
+    double* S = hs;  // [4][100]
+    if (t4 < 2)
+#pragma unroll
+      for (int m = 0; m < 7; ++m) {
+        const int c = 16 * m + gr;
+        if (c < 100) {
+          S[(2 * t4) * 100 + c] = X[m][0] / nn;
+          S[(2 * t4 + 1) * 100 + c] = X[m][1] / nn;
+        }
+        if (m < 6) {
+          S[(2 * t4) * 100 + c + 8] = X[m][2] / nn;
+          S[(2 * t4 + 1) * 100 + c + 8] = X[m][3] / nn;
+        }
+      }
+    __syncwarp();
+    for (int e = lane; e < 400; e += 32) xyz_out[(size_t)row * 400 + e] = S[e];
+    double* Dr = D_out + (size_t)g.drow[row] * 100 * g.ax;
+    for (int e = lane; e < 100 * g.ax; e += 32) {
+      const int c = e / g.ax, k = e - c * g.ax;
+      double d = 0.;
+#pragma unroll
+      for (int a = 0; a < 4; ++a) d = fma(S[a * 100 + c], S[a * 100 + k], d);
+      Dr[e] = d;
+    }
+    __syncwarp();
+  }
+}
+
+// CTAs [first[t], first[t + 1]) take neighbor type t (types are independent in
+// the backward, and one net's fragments fill half of shared memory)
+struct EmSplit {
+  int first[TR_MAXT + 1];
+};
+
+__global__ void __launch_bounds__(32 * EM_BWD_MAXW, 1)
+k_emb_bwd_dmma(double* __restrict__ gem, const double* __restrict__ em,
+               const double* __restrict__ xbar, TrNet<double> net, TrGeom g, EmSplit split) {
+  extern __shared__ __align__(16) double esm[];
+  pdl_wait();
+  pdl_trigger();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int gr = lane >> 2, t4 = lane & 3;
+  int t = 0;
+  while (t + 1 < g.ntypes && (int)blockIdx.x >= split.first[t + 1]) ++t;
+  em_stage(esm, net, t, true);
+  __syncthreads();
+  const double* F2 = esm;
+  const double* F3 = F2 + EM_F2;
+  const double* B3 = F3 + EM_F3;
+  const double* B2 = B3 + EM_B3;
+  const double* V = B2 + EM_B2;
+  double* ws = esm + EM_BWD_T + (size_t)w * EM_BWD_W;
+  double* rr = ws;
+  double* xs = rr + 64;              // xbar [4][100]
+  double* zt = xs + 400;             // [16 rows][EM_TS]: zbar of the current channel tile
+  double* yt = zt + 16 * EM_TS;      // its tanh
+  int* ent = reinterpret_cast<int*>(esm + EM_BWD_T + (size_t)nw * EM_BWD_W) +
+             (size_t)w * (g.nnei + TR_MAXT + 1);
+  int* secn = ent + g.nnei;
+  const int b0 = blockIdx.x - split.first[t], nb = split.first[t + 1] - split.first[t];
+  for (int row = b0 * nw + w; row < g.nrows; row += nb * nw) {
+    tr_entries(ent, secn, g.nlist + (size_t)row * g.nnei, g, g.type[row], false, lane, t, t + 1);
+    const int total = secn[t + 1];
+    if (total == 0) continue;
+    for (int e = lane; e < 400; e += 32) xs[e] = xbar[(size_t)row * 400 + e];
+    for (int e0 = 0; e0 < total; e0 += 16) {
+      const int ne = min(16, total - e0);
+      double xa, xb;
+      em_rows(rr, xa, xb, ent, e0, ne, em + (size_t)row * g.nnei * 4, false, lane);
+      double h1a[EM_S1], h1b[EM_S1], h2[7][4];
+      em_layers12<false>(h1a, h1b, h2, xa, xb, F2, V, nullptr, lane);
+      // hb2: adjoint of h2 (the layout of h2); the residual's share first:
+      // sum_a R[row][a] (xbar[a][c] + xbar[a][c + 50])
+      double hb2[7][4];
+      const double ra = rr[gr * 4 + t4], rc = rr[(gr + 8) * 4 + t4];
+#pragma unroll
+      for (int j = 0; j < 7; ++j) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) hb2[j][k] = 0.;
+        const int c = em_c2(j, gr >> 1, gr & 1);
+        dmma16(hb2[j], ra, rc, c >= 0 ? xs[t4 * 100 + c] + xs[t4 * 100 + c + 50] : 0.);
+      }
+      // dE/dR of rows g, g + 8, columns 2 t, 2 t + 1: sum_c G[c] xbar[a][c], first
+      // the residual's share of G
+      double part[4] = {0., 0., 0., 0.};
+#pragma unroll
+      for (int j = 0; j < 7; ++j)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          const int c = em_c2(j, t4, v);
+          dmma16(part, h2[j][v], h2[j][2 + v],
+                 gr < 4 && c >= 0 ? xs[gr * 100 + c] + xs[gr * 100 + c + 50] : 0.);
+        }
+      auto tile = [&](auto last, int m) {
+        constexpr int LAST = decltype(last)::value;
+        const int c = 16 * m + gr;
+        double z[2][4];
+        em_layer3<LAST>(z, m, h2, F3, V, lane);
+        double gb[2][4];  // gbar = sum_a R[row][a] xbar[a][channel]
+        const bool in = !LAST || gr < 4;
+        const double x0 = in ? xs[t4 * 100 + c] : 0., x1 = LAST ? 0. : xs[t4 * 100 + c + 8];
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) gb[n][k] = 0.;
+          const double rv = rr[(8 * n + gr) * 4 + t4];
+          if (LAST)
+            dmma8(gb[n][0], gb[n][1], x0, rv);
+          else
+            dmma16(gb[n], x0, x1, rv);
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int r = 8 * n + 2 * t4 + e;
+            if (in) {
+              const double y = tanh_f64(z[n][e]);
+              zt[r * EM_TS + gr] = gb[n][e] * (1. - y * y);
+              yt[r * EM_TS + gr] = y;
+            }
+            if (!LAST) {
+              const double y = tanh_f64(z[n][2 + e]);
+              zt[r * EM_TS + gr + 8] = gb[n][2 + e] * (1. - y * y);
+              yt[r * EM_TS + gr + 8] = y;
+            }
+          }
+        __syncwarp();
+#pragma unroll
+        for (int s = 0; s < (LAST ? 1 : 4); ++s) {
+          const int k = 4 * s + t4;
+          const double a0 = zt[gr * EM_TS + k], a1 = zt[(gr + 8) * EM_TS + k];
+          const double* bf = B3 + (size_t)((4 * m + s) * 7) * 32 + lane;
+#pragma unroll
+          for (int j = 0; j < 7; ++j) dmma16(hb2[j], a0, a1, bf[j * 32]);
+          dmma16(part, yt[gr * EM_TS + k], yt[(gr + 8) * EM_TS + k],
+                 gr < 4 ? xs[gr * 100 + 16 * m + k] : 0.);
+        }
+        __syncwarp();
+      };
+#pragma unroll 1
+      for (int m = 0; m < 6; ++m) tile(std::integral_constant<int, 0>{}, m);
+      tile(std::integral_constant<int, 1>{}, 6);
+      // layer 2 adjoint: zb2 in h2's place, then hb1 at the lane's channels
+      double h1b_[8], h1d_[8];  // adjoints of h1, rows g and g + 8
+      {
+        double hb1[4][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) hb1[q][k] = 0.;
+#pragma unroll
+        for (int j = 0; j < 7; ++j) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const double y = h2[j][k] - (k < 2 ? h1a[j] : h1b[j]);
+            h2[j][k] = hb2[j][k] * (1. - y * y);
+          }
+#pragma unroll
+          for (int v = 0; v < 2; ++v)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              dmma16(hb1[q], h2[j][v], h2[j][2 + v], B2[((2 * j + v) * 4 + q) * 32 + lane]);
+        }
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          h1b_[s] = hb1[s >> 1][s & 1];
+          h1d_[s] = hb1[s >> 1][2 + (s & 1)];
+        }
+      }
+      double pa = 0., pb = 0.;
+#pragma unroll
+      for (int s = 0; s < EM_S1; ++s) {
+        const double w1 = V[4 * s + t4];  // zero in padding
+        pa = fma((h1b_[s] + hb2[s][0] + hb2[s][1]) * (1. - h1a[s] * h1a[s]), w1, pa);
+        pb = fma((h1d_[s] + hb2[s][2] + hb2[s][3]) * (1. - h1b[s] * h1b[s]), w1, pb);
+      }
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        pa += __shfl_xor_sync(0xffffffffu, pa, o);
+        pb += __shfl_xor_sync(0xffffffffu, pb, o);
+      }
+      if (t4 == 0) {
+        part[0] += pa;
+        part[2] += pb;
+      }
+      if (t4 < 2) {
+        double* out = gem + (size_t)row * g.nnei * 4 + 2 * t4;
+        if (gr < ne)
+          *reinterpret_cast<double2*>(out + (size_t)(ent[e0 + gr] & 0xFFFF) * 4) =
+              make_double2(part[0], part[1]);
+        if (gr + 8 < ne)
+          *reinterpret_cast<double2*>(out + (size_t)(ent[e0 + gr + 8] & 0xFFFF) * 4) =
+              make_double2(part[2], part[3]);
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// most warps per CTA whose rows come out even: the smallest
+// ceil(rows / (blocks * n)) * n, within shared memory
+static int em_warps(int rows, int blocks, int maxw, size_t base, size_t per_warp) {
+  int best = 0;
+  long long cost = 0;
+  for (int n = maxw; n >= 4; --n) {
+    if (base + per_warp * n > 227 * 1024) continue;
+    const long long c = (long long)ceil_div(rows, (long long)blocks * n) * n;
+    if (best == 0 || c < cost) best = n, cost = c;
+  }
+  return best;
+}
+
+// The passes on the FP64 matrix instructions, for the standard net, 16-byte
+// aligned env rows and at most three types (their fragments must fit in shared
+// memory). em_try_* return -1 when the general kernels have to run.
+static bool em_takes(const TrNet<double>& net, const TrGeom& g, const double* em,
+                     const double* gem) {
+  return net.n1 == 25 && net.n2 == 50 && net.n3 == 100 && g.ntypes <= 3 &&
+         ((reinterpret_cast<uintptr_t>(em) | reinterpret_cast<uintptr_t>(gem)) & 15) == 0;
+}
+
+static int em_fwd(double* xyz, double* D, const double* em, const TrNet<double>& net,
+                  const TrGeom& g, cudaStream_t st) {
+  const size_t base = (size_t)g.ntypes * EM_FWD_T * 8;
+  const size_t per = EM_FWD_W * 8 + (size_t)(g.nnei + TR_MAXT + 1) * 4;
+  const int nw = em_warps(g.nrows, sm_count(), EM_FWD_MAXW, base, per);
+  if (nw == 0) return -1;
+  const size_t smem = base + per * nw;
+  DPB_CUDA(cudaFuncSetAttribute(k_emb_fwd_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)smem),
+           "se_a_train_fwd");
+  const int grid = std::min(sm_count(), ceil_div(g.nrows, nw));
+  DPB_CUDA(launch_pdl(k_emb_fwd_dmma, dim3(grid), dim3(32 * nw), smem, st, xyz, D, em, net, g),
+           "se_a_train_fwd");
+  return DPB_OK;
+}
+
+static int em_bwd(double* gem, const double* em, const double* xbar, const TrNet<double>& net,
+                  const TrGeom& g, cudaStream_t st) {
+  // CTAs per type in proportion to its slots
+  EmSplit sp{};
+  const int sms = std::max(sm_count(), g.ntypes);
+  int used = 0;
+  for (int t = 0; t < g.ntypes; ++t) {
+    sp.first[t] = used;
+    const int left = g.ntypes - 1 - t;
+    int n = (int)((long long)sms * (g.sec[t + 1] - g.sec[t]) / g.nnei);
+    n = t + 1 == g.ntypes ? sms - used : std::max(1, std::min(n, sms - used - left));
+    used += n;
+  }
+  sp.first[g.ntypes] = used;
+  const size_t base = (size_t)EM_BWD_T * 8;
+  const size_t per = EM_BWD_W * 8 + (size_t)(g.nnei + TR_MAXT + 1) * 4;
+  const int nw = em_warps(g.nrows, std::max(1, sms / g.ntypes), EM_BWD_MAXW, base, per);
+  if (nw == 0) return -1;
+  const size_t smem = base + per * nw;
+  DPB_CUDA(cudaFuncSetAttribute(k_emb_bwd_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)smem),
+           "se_a_train_bwd");
+  DPB_CUDA(launch_pdl(k_emb_bwd_dmma, dim3(used), dim3(32 * nw), smem, st, gem, em, xbar, net, g,
+                      sp),
+           "se_a_train_bwd");
+  return DPB_OK;
+}
+
+template <typename T>
+static int em_try_fwd(T* xyz, T* D, const T* em, const TrNet<T>& net, const TrGeom& g,
+                      cudaStream_t st) {
+  if constexpr (std::is_same_v<T, double>)
+    if (em_takes(net, g, em, nullptr)) return em_fwd(xyz, D, em, net, g, st);
+  return -1;
+}
+
+template <typename T>
+static int em_try_bwd(T* gem, const T* em, const T* xbar, const TrNet<T>& net, const TrGeom& g,
+                      cudaStream_t st) {
+  if constexpr (std::is_same_v<T, double>)
+    if (em_takes(net, g, em, gem)) return em_bwd(gem, em, xbar, net, g, st);
+  return -1;
+}
+
+}  // namespace dpb
