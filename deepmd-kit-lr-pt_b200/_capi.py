@@ -107,9 +107,11 @@ _FUNCS = {
     "dpb_se_a_descriptor_bwd_f32": "ppppp" "pp" "pi" "iiip",
     "dpb_se_a_descriptor_fwd_cubic_f32": "pppp" "pp" "pi" "iiip",
     "dpb_se_a_descriptor_bwd_cubic_f32": "ppppp" "pp" "pi" "iiip",
-    "dpb_se_a_descriptor_fwd_cheb_f32": "pppp" "pppp" "pi" "iiip",
+    "dpb_se_a_descriptor_fwd_cheb_f32": "pppp" "ppppp" "pi" "iiip",
+    "dpb_gemm_f16x3_f32": "piipppp" "ipii" "pppp" "pppp" "pp",
     "dpb_se_a_descriptor_bwd_cheb_f32": "ppppp" "pppp" "pi" "iiip",
-    "dpb_bt_step_set_nets": "ppp",
+    "dpb_bt_step_set_nets": "ppppppp",
+    "dpb_se_a_row_scale_f32": "pppiip",
     "dpb_force_virial_a_f32": "pppppp" "pp" "iiiip",
     "dpb_force_virial_a_f64": "pppppp" "pp" "iiiip",
     "dpb_build_nlist_noalloc_f64": "ppppp" "iiif" "i" "pp",

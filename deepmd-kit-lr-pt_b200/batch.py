@@ -206,20 +206,23 @@ class BatchEvaluator:
             return g
 
         layers = [
-            layer(self.D, din, E.B1f, w, E.EPI_TANH, E.H1, bias=E.b1),
-            layer(E.H1, w, E.B2f, w, E.EPI_RES_DT, E.Y2, E.H2, aux0=E.H1, bias=E.b2, idt=E.d2),
-            layer(E.H2, w, E.B3f, w, E.EPI_LAST, E.G3, aux0=E.H2, bias=E.b3, idt=E.d3,
+            layer(self.D, din, E.tf32("1f"), w, E.EPI_TANH, E.H1, bias=E.b1),
+            layer(E.H1, w, E.tf32("2f"), w, E.EPI_RES_DT, E.Y2, E.H2, aux0=E.H1, bias=E.b2,
+                  idt=E.d2),
+            layer(E.H2, w, E.tf32("3f"), w, E.EPI_LAST, E.G3, aux0=E.H2, bias=E.b3, idt=E.d3,
                   wv=E.w4),
-            layer(E.G3, w, E.B3b, w, E.EPI_BWD_DT, E.G2, E.g2, aux0=E.Y2, idt=E.d2, wv=E.w4),
-            layer(E.G2, w, E.B2b, w, E.EPI_BWD_RES, E.G1, aux0=E.H1, aux1=E.g2),
-            layer(E.G1, w, E.B1b, din, E.EPI_STORE, self.dD)]
+            layer(E.G3, w, E.tf32("3b"), w, E.EPI_BWD_DT, E.G2, E.g2, aux0=E.Y2, idt=E.d2, wv=E.w4),
+            layer(E.G2, w, E.tf32("2b"), w, E.EPI_BWD_RES, E.G1, aux0=E.H1, aux1=E.g2),
+            layer(E.G1, w, E.tf32("1b"), din, E.EPI_STORE, self.dD)]
         for k, g in enumerate(layers):
             d.fit[k] = g
         self._desc = d
         handle = ctypes.c_void_p()
         call("dpb_bt_step_create", ctypes.byref(handle), ctypes.byref(d))
         if pt.nets is not None:
-            call("dpb_bt_step_set_nets", handle, pt.nets, ptr(pt.touched))
+            b, a_scale, b_scale = fit.f16_layers()
+            call("dpb_bt_step_set_nets", handle, pt.nets, ptr(pt.touched), ptr(pt.row_scale), b,
+                 a_scale.ctypes.data, b_scale.ctypes.data)
         self._split = _capi.lib().dpb_tune_get(b"batch_fused_split") != 0
         self.plan = handle
 
@@ -267,7 +270,7 @@ class BatchEvaluator:
              cfg.sec.size, ptr(self.status), s)
         pt = self.ptab
         pt.forward(self.xyz, self.D, self.drow, self.em, cfg.sec, N, M, ax, s)
-        self.fit.layers(self.D, self.dD)
+        self.fit.layers(self.D, self.dD, row_scale=pt.row_scale)
         pt.backward(self.net_deriv, self.dD, self.drow, self.xyz, self.em, cfg.sec, N, M, ax, s)
         call("dpb_batch_force_virial_a", ptr(self.force), ptr(self.virial),
              ptr(self.net_deriv), ptr(self.cw), ptr(self.type), ptr(self.std),

@@ -34,6 +34,7 @@
 #include <stddef.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "dpb_batch_dev.cuh"
 #include "dpb_cheb_dev.cuh"
@@ -61,7 +62,9 @@ constexpr unsigned long long BS_WAIT_NS = 500000000ull;  // per barrier
 // the weights are pre-split, so no weight-splitting warps, and 8 epilogue
 // warps (40 or 48 chunk sums a thread).
 using CfgBS = GemmCfg<80, 3, 4, 2, 8, false>;
-static_assert(CfgBS::THREADS <= BS_THREADS, "the GEMM passes fit in the step kernel's warps");
+// with the piecewise Chebyshev nets the GEMMs run in the FP16 form
+using CfgBSH = GemmCfg<80, 6, 4, 2, 8, false, true>;
+static_assert(CfgBS::THREADS <= BS_THREADS && CfgBSH::THREADS <= BS_THREADS, "the GEMM passes fit in the step kernel's warps");
 
 struct BtStepArgs {
   GemmMaps maps[BS_PASSES];
@@ -72,6 +75,7 @@ struct BtStepArgs {
   TypeTables tt;
   ChebTables ct;      // piecewise Chebyshev nets (rows then go in groups of four)
   unsigned* touched;
+  float* row_scale;
   double* cw;
   int* cell_of;
   int* cell_start;
@@ -194,7 +198,7 @@ __device__ __forceinline__ void bs_rows_fwd(const BtStepArgs& a, int row, int wa
                                             float* gsm) {
   cheb_fwd_group<BS_CH, 6, COH>(row, a.nrows, warp % CHEB_A, lane, BS_BAR0 + warp / CHEB_A, gsm,
                                 a.xyz, a.D, a.drow, a.em, a.ct, a.tt, a.M, a.naxis, a.inv_nnei,
-                                a.touched);
+                                a.touched, a.row_scale);
 }
 
 __device__ __forceinline__ void bs_rows_bwd(const BtStepArgs& a, int row, int warp, int lane,
@@ -219,16 +223,17 @@ __device__ __forceinline__ void bs_row_force(const BtStepArgs& a, int row, int l
                            a.nlist, a.fr, a.sec.ntypes, a.sec.nnei, a.rcut, a.rcut_smth);
 }
 
-template <int MODE>
+template <class CFG, int MODE>
 __device__ __forceinline__ void bs_gemm(const BtStepArgs& a, int l, unsigned char* smem,
                                      GemmBars& bars, uint32_t tmem) {
-  gemm_run<CfgBS, MODE, true>(a.maps[l], a.shp[l], a.epi[l], a.status, smem, bars, tmem);
+  gemm_run<CFG, MODE, true>(a.maps[l], a.shp[l], a.epi[l], a.status, smem, bars, tmem);
 }
 
 // CHEB: the descriptor passes on the piecewise Chebyshev nets; a work item is
 // then CHEB_A rows for a group of as many warps
 template <int NC, bool CHEB>
 __global__ void __launch_bounds__(BS_THREADS, 1) k_bt_step(const __grid_constant__ BtStepArgs a) {
+  using Cfg = std::conditional_t<CHEB, CfgBSH, CfgBS>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ GemmBars bars[BS_PASSES];
@@ -305,32 +310,32 @@ __global__ void __launch_bounds__(BS_THREADS, 1) k_bt_step(const __grid_constant
 
   // ---- P2-P7: the fitting GEMMs
   if (ok) {
-    bs_gemm<EPI_TANH>(a, 0, smem, bars[0], tmem);
+    bs_gemm<Cfg, EPI_TANH>(a, 0, smem, bars[0], tmem);
     ok = bs_sync(a, ++k, &s_ok);
     bs_stamp(a, k);
   }
   if (ok) {
-    bs_gemm<EPI_RES_DT>(a, 1, smem, bars[1], tmem);
+    bs_gemm<Cfg, EPI_RES_DT>(a, 1, smem, bars[1], tmem);
     ok = bs_sync(a, ++k, &s_ok);
     bs_stamp(a, k);
   }
   if (ok) {
-    bs_gemm<EPI_LAST>(a, 2, smem, bars[2], tmem);
+    bs_gemm<Cfg, EPI_LAST>(a, 2, smem, bars[2], tmem);
     ok = bs_sync(a, ++k, &s_ok);
     bs_stamp(a, k);
   }
   if (ok) {
-    bs_gemm<EPI_BWD_DT>(a, 3, smem, bars[3], tmem);
+    bs_gemm<Cfg, EPI_BWD_DT>(a, 3, smem, bars[3], tmem);
     ok = bs_sync(a, ++k, &s_ok);
     bs_stamp(a, k);
   }
   if (ok) {
-    bs_gemm<EPI_BWD_RES>(a, 4, smem, bars[4], tmem);
+    bs_gemm<Cfg, EPI_BWD_RES>(a, 4, smem, bars[4], tmem);
     ok = bs_sync(a, ++k, &s_ok);
     bs_stamp(a, k);
   }
   if (ok) {
-    bs_gemm<EPI_STORE>(a, 5, smem, bars[5], tmem);
+    bs_gemm<Cfg, EPI_STORE>(a, 5, smem, bars[5], tmem);
     bs_smem_switch();
     ok = bs_sync(a, ++k, &s_ok);
     bs_stamp(a, k);
@@ -405,7 +410,7 @@ static const void* bs_kernel(int nc, bool cheb) {
 // the kernel with the smallest carve-out that holds it (the rest is L1)
 static int bs_set_smem(BtStepArgs& a, int nc, bool cheb, size_t wf, size_t& smem) {
   wf = (std::max(wf, (sizeof(BtEnvSmem) + 3) / 4) + 3) / 4 * 4;
-  smem = std::max({(size_t)CfgBS::SMEM, wf * 4 * BS_WARPS + 1024,
+  smem = std::max({(size_t)(cheb ? CfgBSH::SMEM : CfgBS::SMEM), wf * 4 * BS_WARPS + 1024,
                    (size_t)4 * (BT_MAXCELLS + 1) + 1024});
   if (smem + 4096 > 232448) {
     set_error("bt_step: the per-warp descriptor staging (%zu B) does not fit", wf * 4);
@@ -543,10 +548,14 @@ int dpb_bt_step_create(void** plan, const dpb_bt_step_desc* d) {
   return DPB_OK;
 }
 
-int dpb_bt_step_set_nets(void* plan, const dpb_cheb_net* nets, unsigned* touched) {
+int dpb_bt_step_set_nets(void* plan, const dpb_cheb_net* nets, unsigned* touched,
+                         float* row_scale, const void* const* b, const float* a_scale,
+                         const float* b_scale) {
   BtStepPlan* p = static_cast<BtStepPlan*>(plan);
-  if (p == nullptr || p->nc != 6) {
-    set_error("bt_step_set_nets: needs a plan with quintic tables");
+  if (p == nullptr || p->nc != 6 || row_scale == nullptr || b == nullptr || a_scale == nullptr ||
+      b_scale == nullptr) {
+    set_error("bt_step_set_nets: needs a plan with quintic tables, the row scales and the FP16 "
+              "weights with their scales");
     return DPB_ERR_INVALID;
   }
   ChebTables ct;
@@ -559,8 +568,15 @@ int dpb_bt_step_set_nets(void* plan, const dpb_cheb_net* nets, unsigned* touched
                          CHEB_A - 1) / CHEB_A,
                         smem)))
     return rc;
+  for (int l = 0; l < BS_PASSES; ++l) {
+    const int o = l * p->a.shp[l].ntypes;
+    if ((rc = gemm_set_f16(b + o, a_scale + o, b_scale + o, l == 0 ? row_scale : nullptr,
+                           CfgBSH::BN, p->a.maps[l], p->a.shp[l], p->a.epi[l])))
+      return rc;
+  }
   p->a.ct = ct;
   p->a.touched = touched;
+  p->a.row_scale = row_scale;
   p->cheb = true;
   p->smem = smem;
   return DPB_OK;

@@ -31,9 +31,8 @@
 // the linear tails) are added from the table, a warp per slot.
 #pragma once
 
-#include <cuda_fp16.h>
-
 #include "dpb_desc_dev.cuh"
+#include "dpb_f16split.cuh"
 
 namespace dpb {
 
@@ -76,24 +75,6 @@ __device__ __forceinline__ void mma_split(float (&d)[4], const unsigned (&ah)[4]
   mma_f16(d, al, b.x, b.y, zero);
   mma_f16(d, ah, b.z, b.w, d);
   mma_f16(d, ah, b.x, b.y, d);
-}
-
-// (x, y) as two FP16 pairs, hi + lo
-__device__ __forceinline__ void split_f16(float x, float y, unsigned& hi, unsigned& lo) {
-  const __half2 h = __floats2half2_rn(x, y);
-  const float2 f = __half22float2(h);
-  const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
-  hi = *reinterpret_cast<const unsigned*>(&h);
-  lo = *reinterpret_cast<const unsigned*>(&l);
-}
-
-// power of two s with bound * s < 2^14 (exponent field clamped so that 1 / s
-// is normal too), and its reciprocal
-__device__ __forceinline__ float cheb_scale(float bound, float& inv) {
-  const int e = (__float_as_int(bound) >> 23) & 255;  // bound < 2^(e - 126)
-  const int se = min(253, max(1, 267 - e));
-  inv = __int_as_float((254 - se) << 23);
-  return __int_as_float(se << 23);
 }
 
 __device__ __forceinline__ float warp_max(float v) {
@@ -148,6 +129,17 @@ __device__ __forceinline__ bool cheb_locate(const ChebNet& c, float x, int& r, f
   return true;
 }
 
+// power of two that brings a descriptor row below 2^14, from its atom's x
+// [4][M]: |D[m, a]| <= max_m sum_d x[d, m]^2
+__device__ __forceinline__ float descriptor_scale(const float* x, int M, int lane) {
+  float mx = 0.f;
+  for (int m = lane; m < M; m += 32)
+    mx = fmaxf(mx, x[m] * x[m] + x[M + m] * x[M + m] + x[2 * M + m] * x[2 * M + m] +
+                       x[3 * M + m] * x[3 * M + m]);
+  float inv;
+  return f16_scale(warp_max(mx), inv);
+}
+
 // floats of shared memory per group of CHEB_A warps
 static size_t cheb_fwd_floats(int M, int wstride) {
   const size_t w = (size_t)CHEB_A * 4 * wstride, x = (size_t)CHEB_A * 4 * M;
@@ -179,7 +171,8 @@ __device__ __forceinline__ void frag_a(unsigned (&h)[4], unsigned (&l)[4], const
 // Descriptor forward of atoms i0 .. i0 + 7 (those below nrow): warp w of the
 // group sums atom i0 + w's slots into W, then all warps share the products.
 // touched: the intervals that hold a slot of any of the eight, per type (may
-// be NULL).
+// be NULL); row_scale: per descriptor row, the power of two that brings it
+// below 2^14 (the operand scale of the FP16 fitting GEMM; may be NULL).
 template <int CH, int NC, bool COH = false>
 __device__ __forceinline__ void cheb_fwd_group(int i0, int nrow, int w, int lane, int bar,
                                                float* gsm, float* __restrict__ xyz_out,
@@ -187,7 +180,8 @@ __device__ __forceinline__ void cheb_fwd_group(int i0, int nrow, int w, int lane
                                                const int* __restrict__ drow,
                                                const float* __restrict__ em,
                                                const ChebTables& ct, const TypeTables& tt, int M,
-                                               int naxis, float inv_nnei, unsigned* touched) {
+                                               int naxis, float inv_nnei, unsigned* touched,
+                                               float* row_scale) {
   constexpr int NTW = MAXM / 8 / CHEB_A;  // channel tiles per warp
   const int nnei = tt.nnei, wst = ct.wstride, ntile = (M + 7) / 8;
   const int i = i0 + w;
@@ -291,7 +285,7 @@ __device__ __forceinline__ void cheb_fwd_group(int i0, int nrow, int w, int lane
       __syncwarp();
       // |T_k| <= 1 (to rounding), so sum |e| bounds every entry of W; the
       // touched entries become (hi pair, lo pair) words in place
-      const float sc = cheb_scale(warp_sum(bound), inv);
+      const float sc = f16_scale(warp_sum(bound), inv);
       for (unsigned m = mask; m; m &= m - 1u) {
         float2* p = reinterpret_cast<float2*>(Wa + cd * wst + (__ffs(m) - 1) * CHEB_K + 2 * cp);
         const float2 v = *p;
@@ -410,6 +404,10 @@ __device__ __forceinline__ void cheb_fwd_group(int i0, int nrow, int w, int lane
     }
     float4* xo = reinterpret_cast<float4*>(xyz_out + (size_t)i * 4 * M);
     for (int q = lane; q < M; q += 32) xo[q] = reinterpret_cast<const float4*>(xa)[q];
+    if (row_scale != nullptr) {
+      const float sc = descriptor_scale(xa, M, lane);
+      if (lane == 0) row_scale[drow[i]] = sc;
+    }
     write_descriptor(D + (size_t)drow[i] * M * naxis, xa, M, naxis, lane);
   }
 }
@@ -450,7 +448,7 @@ __device__ __forceinline__ void cheb_bwd_group(int i0, int nrow, int w, int lane
       for (int ch = 0; ch < 4; ++ch)
 #pragma unroll
         for (int k = 0; k < 4; ++k) mx = fmaxf(mx, fabsf(dyr[ch][k]));
-      sc = cheb_scale(warp_max(mx), inv);
+      sc = f16_scale(warp_max(mx), inv);
     }
     if (m0 < ksteps * 16) {  // zero beyond M and for atoms beyond the last
 #pragma unroll

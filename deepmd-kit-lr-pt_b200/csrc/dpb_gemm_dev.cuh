@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include "dpb_common.cuh"
+#include "dpb_f16split.cuh"
 
 namespace dpb {
 
@@ -24,21 +25,27 @@ constexpr uint32_t TM_COLS = 512;
 // BSPLIT: with the four warps that split FP32 weights into TF32 hi / lo in
 // shared memory (false: pre-split weights only, the epilogue warps follow
 // the A-split warps)
-template <int BN_, int STAGES_, int ASLOTS_, int ACCBUF_, int EPIW_, bool BSPLIT_ = true>
+// F16: operands as two FP16 terms (kind::f16, K = 16 per instruction) instead of
+// two TF32 terms (K = 8); a weight row's k-block then holds 32 hi and 32 lo
+// halves side by side, one 128-byte row as well
+template <int BN_, int STAGES_, int ASLOTS_, int ACCBUF_, int EPIW_, bool BSPLIT_ = true,
+          bool F16_ = false>
 struct GemmCfg {
   static constexpr int BN = BN_, STAGES = STAGES_, ASLOTS = ASLOTS_, ACCBUF = ACCBUF_,
                        EPIW = EPIW_;
-  static constexpr bool BSPLIT = BSPLIT_;
+  static constexpr bool BSPLIT = BSPLIT_, F16 = F16_;
   static constexpr int EPI0 = BSPLIT ? 10 : 6;  // first epilogue warp
   static constexpr int THREADS = 32 * EPI0 + 32 * EPIW;
   static constexpr uint32_t ACC_STRIDE = BN <= 128 ? 128u : (uint32_t)((BN + 31) / 32 * 32);
   static constexpr uint32_t A0 = ACCBUF * ACC_STRIDE;
   static constexpr int A_BYTES = GT_BM * GT_BK * 4;  // 16 KB
   static constexpr int B_BYTES = BN * GT_BK * 4;
-  static constexpr int STAGE_BYTES = A_BYTES + 2 * B_BYTES;
+  static constexpr int STAGE_BYTES = A_BYTES + (F16 ? 1 : 2) * B_BYTES;
+  static constexpr uint32_t ASW = F16 ? 32u : 64u;  // TMEM columns of an A slot (hi, lo)
   static constexpr int SMEM = STAGES * STAGE_BYTES + 1024;
   static_assert(BN % 16 == 0 && BN <= 256, "MMA N");
-  static_assert(A0 + 64u * ASLOTS <= TM_COLS, "tensor memory columns");
+  static_assert(A0 + ASW * ASLOTS <= TM_COLS, "tensor memory columns");
+  static_assert(!(F16 && BSPLIT), "FP16 weights come split");
   static_assert(STAGE_BYTES % 1024 == 0, "stage alignment for the 128-byte swizzle");
   static_assert(SMEM <= 232448, "shared memory per CTA");
   static_assert(EPIW == 4 || EPIW == 8, "epilogue warps");
@@ -57,6 +64,14 @@ using CfgN240 = GemmCfg<240, 2, 4, 1, 8>;
 // hi x hi products are issued) still leaves loads in flight for the next;
 // eight epilogue warps drain the chunk accumulators
 using CfgN80C = GemmCfg<80, 6, 4, 2, 8>;
+// the FP16 forms: half the weight bytes and half the TMEM columns per A slot
+// leave room for deeper rings; CfgH80 drains chunks or whole tiles. Measured,
+// 331,776 rows, TF32 -> FP16: K = 1600 layer 1.56 -> 1.26 ms, N = 1600 1.58 -> 1.33 ms
+// (the MMAs halved; the K = 1600 layer now reads its operands from L2 at 8 TB/s),
+// the 240 x 240 layers unchanged (their epilogues bound them)
+using CfgH80 = GemmCfg<80, 8, 8, 2, 8, false, true>;
+using CfgH160 = GemmCfg<160, 6, 6, 2, 8, false, true>;
+using CfgH240 = GemmCfg<240, 4, 8, 1, 8, false, true>;
 
 enum : int {
   ST_MMA_TIMEOUT = 1 << 8,
@@ -83,6 +98,11 @@ struct GemmEpi {
   const float* idt[GT_MAXT];
   const float* w[GT_MAXT];
   float* e;
+  // FP16 form: power-of-two scale of A's rows per type (times row_scale[row]
+  // where given) and its product's reciprocal with the weights' scale
+  const float* row_scale;
+  float a_scale[GT_MAXT];
+  float inv_scale[GT_MAXT];
 };
 
 struct GemmShape {
@@ -105,7 +125,7 @@ struct GemmMaps {
 };
 
 // the mbarriers of one GEMM pass (sized for every configuration below)
-constexpr int GB_MAXS = 6, GB_MAXA = 4, GB_MAXACC = 2;
+constexpr int GB_MAXS = 8, GB_MAXA = 8, GB_MAXACC = 2;
 struct GemmBars {
   uint64_t full[GB_MAXS], conv[GB_MAXS], empty[GB_MAXS];
   uint64_t afree[GB_MAXA];
@@ -183,6 +203,17 @@ __device__ __forceinline__ void mma_tf32_ta(uint32_t tmem_d, uint32_t tmem_a, ui
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u),
+      "r"(0u), "r"(0u));
+}
+
+// the same with FP16 pairs (two k per TMEM column)
+__device__ __forceinline__ void mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t b,
+                                           uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
       ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u),
       "r"(0u), "r"(0u));
 }
@@ -286,9 +317,22 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
   constexpr int A_BYTES = CFG::A_BYTES;
   constexpr int B_BYTES = CFG::B_BYTES;
   constexpr int STAGE_BYTES = CFG::STAGE_BYTES;
+  constexpr bool F16 = CFG::F16;
+  constexpr uint32_t ASW = CFG::ASW;
+  constexpr uint32_t ALO = ASW / 2;          // TMEM columns from hi to lo
+  constexpr int KS = F16 ? GT_BK / 16 : GT_BK / 8;  // MMAs per k-block and product
+  // byte offset of the weights' lo part from hi: the second half of the 128-byte
+  // rows (FP16), or a second tile (TF32)
+  constexpr uint64_t BLO = (F16 ? 64 : B_BYTES) >> 4;
+  auto mma = [](uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    if constexpr (F16)
+      mma_f16_ta(d, a, b, idesc, accumulate);
+    else
+      mma_tf32_ta(d, a, b, idesc, accumulate);
+  };
   constexpr uint32_t IDESC = (1u << 4)            // D: FP32
-                             | (2u << 7)          // A: TF32
-                             | (2u << 10)         // B: TF32
+                             | ((F16 ? 0u : 2u) << 7)   // A: FP16 or TF32
+                             | ((F16 ? 0u : 2u) << 10)  // B: the same
                              | ((uint32_t)(BN >> 3) << 17)  // N
                              | ((uint32_t)(GT_BM >> 4) << 24);  // M = 128
   static_assert(STAGES <= GB_MAXS && ASLOTS <= GB_MAXA && ACCBUF <= GB_MAXACC, "barrier set");
@@ -346,10 +390,11 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
         }
         if (elect_one()) {
           unsigned char* st = smem + s * STAGE_BYTES;
-          mbar_expect_tx(&full_bar[s], A_BYTES + (shp.split_b ? 1 : 2) * B_BYTES);
+          mbar_expect_tx(&full_bar[s], A_BYTES + (F16 || shp.split_b ? 1 : 2) * B_BYTES);
           tma_load_2d(st, &maps.a, &full_bar[s], kb * GT_BK, tc.row0);
-          tma_load_2d(st + A_BYTES, &maps.bh[tc.ty], &full_bar[s], kb * GT_BK, tc.n0);
-          if (!shp.split_b)
+          tma_load_2d(st + A_BYTES, &maps.bh[tc.ty], &full_bar[s], (F16 ? 2 : 1) * kb * GT_BK,
+                      tc.n0);
+          if (!F16 && !shp.split_b)
             tma_load_2d(st + A_BYTES + B_BYTES, &maps.bl[tc.ty], &full_bar[s], kb * GT_BK,
                         tc.n0);
         }
@@ -398,18 +443,17 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             unsigned char* st = smem + s * STAGE_BYTES;
-            const uint32_t ah = tmem + TM_A0 + 64u * (uint32_t)as, al = ah + 32u;
-            const uint64_t bh = smem_desc(st + A_BYTES);
-            const uint64_t bl = smem_desc(st + A_BYTES + B_BYTES);
+            const uint32_t ah = tmem + TM_A0 + ASW * (uint32_t)as, al = ah + ALO;
+            const uint64_t bh = smem_desc(st + A_BYTES), bl = bh + BLO;
             if (elect_one()) {
 #pragma unroll
-              for (int j = 0; j < GT_BK / 8; ++j) {
+              for (int j = 0; j < KS; ++j) {
                 const uint32_t ca = 8u * (uint32_t)j;
                 const uint64_t ob = (uint64_t)(j * 32) >> 4;
-                mma_tf32_ta(d, al + ca, bh + ob, IDESC, (i > 0 || j > 0) ? 1u : 0u);
-                mma_tf32_ta(d, ah + ca, bl + ob, IDESC, 1u);
-                if (shp.terms == 4) mma_tf32_ta(d, al + ca, bl + ob, IDESC, 1u);
-                if (!shp.cross_first) mma_tf32_ta(d, ah + ca, bh + ob, IDESC, 1u);
+                mma(d, al + ca, bh + ob, IDESC, (i > 0 || j > 0) ? 1u : 0u);
+                mma(d, ah + ca, bl + ob, IDESC, 1u);
+                if (shp.terms == 4) mma(d, al + ca, bl + ob, IDESC, 1u);
+                if (!shp.cross_first) mma(d, ah + ca, bh + ob, IDESC, 1u);
               }
               if (!shp.cross_first) {  // k-block order: its stage is free once read
                 mma_commit(&empty_bar[s]);
@@ -424,12 +468,11 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
             for (int i = 0; i < nkc && shp.cross_first; ++i) {  // pass 2: Ah Bh
               const int gi = g + i, s = gi % STAGES, as = gi % ASLOTS;
               unsigned char* st = smem + s * STAGE_BYTES;
-              const uint32_t ah = tmem + TM_A0 + 64u * (uint32_t)as;
+              const uint32_t ah = tmem + TM_A0 + ASW * (uint32_t)as;
               const uint64_t bh = smem_desc(st + A_BYTES);
 #pragma unroll
-              for (int j = 0; j < GT_BK / 8; ++j)
-                mma_tf32_ta(d, ah + 8u * (uint32_t)j, bh + ((uint64_t)(j * 32) >> 4), IDESC,
-                            1u);
+              for (int j = 0; j < KS; ++j)
+                mma(d, ah + 8u * (uint32_t)j, bh + ((uint64_t)(j * 32) >> 4), IDESC, 1u);
               mma_commit(&empty_bar[s]);
               mma_commit(&afree_bar[as]);
             }
@@ -460,19 +503,18 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           unsigned char* st = smem + s * STAGE_BYTES;
           const int as = g % ASLOTS;
-          const uint32_t ah = tmem + TM_A0 + 64u * (uint32_t)as, al = ah + 32u;
-          const uint64_t bh = smem_desc(st + A_BYTES);
-          const uint64_t bl = smem_desc(st + A_BYTES + B_BYTES);
+          const uint32_t ah = tmem + TM_A0 + ASW * (uint32_t)as, al = ah + ALO;
+          const uint64_t bh = smem_desc(st + A_BYTES), bl = bh + BLO;
           if (elect_one()) {
 #pragma unroll
-            for (int j = 0; j < GT_BK / 8; ++j) {  // K = 8 per instruction
+            for (int j = 0; j < KS; ++j) {  // 32 bytes of k per instruction
               const uint32_t ca = 8u * (uint32_t)j;           // TMEM columns
               const uint64_t ob = (uint64_t)(j * 32) >> 4;    // +32 B in the swizzled row
               const uint32_t acc = (kb > 0 || j > 0) ? 1u : 0u;
-              mma_tf32_ta(d, ah + ca, bh + ob, IDESC, acc);
-              mma_tf32_ta(d, al + ca, bh + ob, IDESC, 1u);
-              mma_tf32_ta(d, ah + ca, bl + ob, IDESC, 1u);
-              if (shp.terms == 4) mma_tf32_ta(d, al + ca, bl + ob, IDESC, 1u);
+              mma(d, ah + ca, bh + ob, IDESC, acc);
+              mma(d, al + ca, bh + ob, IDESC, 1u);
+              mma(d, ah + ca, bl + ob, IDESC, 1u);
+              if (shp.terms == 4) mma(d, al + ca, bl + ob, IDESC, 1u);
             }
             mma_commit(&empty_bar[s]);    // frees the shared-memory stage once read
             mma_commit(&afree_bar[as]);   // and the TMEM A slot
@@ -502,6 +544,13 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
     int g = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < n_total && ok; t += gridDim.x) {
+      float sc = 1.f;
+      if constexpr (F16) {
+        const TileCoord tc = tile_coord(shp, t, BN);
+        sc = epi.a_scale[tc.ty];
+        if (epi.row_scale != nullptr && tc.row0 + r < tc.row_end)
+          sc *= __ldg(epi.row_scale + tc.row0 + r);
+      }
       for (int kb = 0; kb < nk; ++kb, ++g) {
         const int s = g % STAGES;
         const uint32_t ph = (g / STAGES) & 1;
@@ -516,23 +565,29 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // row r of the 128-byte-swizzled tile: 16-byte chunk c at c ^ (r & 7)
         const unsigned char* rowp = smem + s * STAGE_BYTES + r * 128;
-        uint32_t hi[32], lo[32];
+        const uint32_t ta = tmem + (lane_base << 16) + TM_A0 + ASW * (uint32_t)as;
+        uint32_t hi[ALO], lo[ALO];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           const float4 x = *reinterpret_cast<const float4*>(rowp + ((c ^ (r & 7)) << 4));
-          const float xs[4] = {x.x, x.y, x.z, x.w};
+          if constexpr (F16) {
+            split_f16(x.x * sc, x.y * sc, hi[2 * c], lo[2 * c]);
+            split_f16(x.z * sc, x.w * sc, hi[2 * c + 1], lo[2 * c + 1]);
+          } else {
+            const float xs[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float h = tf32_hi(xs[u]);
-            hi[4 * c + u] = __float_as_uint(h);
-            lo[4 * c + u] = __float_as_uint(tf32_hi(xs[u] - h));
+            for (int u = 0; u < 4; ++u) {
+              const float h = tf32_hi(xs[u]);
+              hi[4 * c + u] = __float_as_uint(h);
+              lo[4 * c + u] = __float_as_uint(tf32_hi(xs[u] - h));
+            }
           }
         }
-        const uint32_t ta = tmem + (lane_base << 16) + TM_A0 + 64u * (uint32_t)as;
-        tmem_st16(ta, hi);
-        tmem_st16(ta + 16u, hi + 16);
-        tmem_st16(ta + 32u, lo);
-        tmem_st16(ta + 48u, lo + 16);
+#pragma unroll
+        for (uint32_t q = 0; q < ALO; q += 16) {
+          tmem_st16(ta + q, hi + q);
+          tmem_st16(ta + ALO + q, lo + q);
+        }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         mbar_arrive(&conv_bar[s]);
@@ -644,6 +699,11 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
       const float* bias = epi.bias[tc.ty];
       const float* idt = epi.idt[tc.ty];
       const float* wv = epi.w[tc.ty];
+      float inv = 1.f;
+      if constexpr (F16) {
+        inv = epi.inv_scale[tc.ty];
+        if (epi.row_scale != nullptr && ok) inv /= __ldg(epi.row_scale + row);  // powers of two
+      }
       constexpr bool NEED0 = MODE >= EPI_RES_DT, NEED1 = MODE == EPI_BWD_RES;
       const uint32_t acc_base = tmem + ((uint32_t)lane_base << 16) + (uint32_t)b * TM_ACC;
       float esum = 0.f;
@@ -660,6 +720,9 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
         }
         float v[16];
         load_acc(v);
+        if constexpr (F16)
+#pragma unroll
+          for (int k = 0; k < 16; ++k) v[k] *= inv;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int cj = n0 + c0 + 4 * j;
@@ -740,7 +803,10 @@ int gemm_prepare(const float* A, int M, int K, const float* const* b_hi,
                  const float* const* b_lo, int N, const int* type_rows, int ntypes, int mode,
                  float* out0, float* out1, const float* aux0, const float* aux1,
                  const float* const* bias, const float* const* idt, const float* const* w,
-                 float* e, int force_bn, GemmMaps& maps, GemmShape& shp, GemmEpi& ep, int& BN);
+                 float* e, int force_bn, GemmMaps& maps, GemmShape& shp, GemmEpi& ep, int& BN,
+                 bool f16 = false);
+int gemm_set_f16(const void* const* b, const float* a_scale, const float* b_scale,
+                 const float* row_scale, int BN, GemmMaps& maps, GemmShape& shp, GemmEpi& ep);
 
 __device__ __forceinline__ void tmem_alloc_all(uint32_t* slot) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(

@@ -51,6 +51,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "dpb_gemm_dev.cuh"
 
@@ -120,7 +121,7 @@ static int launch(const GemmMaps& maps, GemmShape shp, const GemmEpi& epi, int* 
   shp.kchunk = 0;
   shp.cross_first = 0;
   if constexpr (CFG::BN == 80) {
-    using C = CfgN80C;
+    using C = std::conditional_t<CFG::F16, CFG, CfgN80C>;
     const int nk = (shp.K + GT_BK - 1) / GT_BK;
     shp.cross_first = tune_value("fit_kchunk_cross_first", 0) != 0;
     int P = tune_value("fit_kchunk", 8);
@@ -149,17 +150,19 @@ static int get_encoder() {
   return DPB_OK;
 }
 
-// 2-D FP32 row-major [rows, cols] (cols contiguous), box rows x 32 cols, SW128
-static int make_map(CUtensorMap* m, const float* base, int rows, int cols, int box_rows) {
+// 2-D FP32 row-major [rows, cols] (cols contiguous), box rows x 32 cols, SW128;
+// f16: the same bytes as pairs of halves
+static int make_map(CUtensorMap* m, const float* base, int rows, int cols, int box_rows,
+                    bool f16 = false) {
   if (((uintptr_t)base & 15) != 0 || (cols * 4) % 16 != 0) {
     set_error("gemm: operand base must be 16-byte aligned and rows a multiple of 16 bytes");
     return DPB_ERR_INVALID;
   }
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t dims[2] = {(cuuint64_t)cols * (f16 ? 2 : 1), (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)cols * 4};
-  cuuint32_t box[2] = {(cuuint32_t)GT_BK, (cuuint32_t)box_rows};
+  cuuint32_t box[2] = {(cuuint32_t)(f16 ? 2 * GT_BK : GT_BK), (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = g_encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)base, dims, strides, box,
+  CUresult r = g_encode(m, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)base, dims, strides, box,
                         estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
@@ -221,7 +224,8 @@ int gemm_prepare(const float* A, int M, int K, const float* const* b_hi,
                  const float* const* b_lo, int N, const int* type_rows, int ntypes, int mode,
                  float* out0, float* out1, const float* aux0, const float* aux1,
                  const float* const* bias, const float* const* idt, const float* const* w,
-                 float* e, int force_bn, GemmMaps& maps, GemmShape& shp, GemmEpi& ep, int& BN) {
+                 float* e, int force_bn, GemmMaps& maps, GemmShape& shp, GemmEpi& ep, int& BN,
+                 bool f16) {
   if (ntypes < 1 || ntypes > GT_MAXT || M < 0 || K <= 0 || N <= 0 || mode < 0 ||
       mode > EPI_BWD_RES || type_rows == nullptr || b_hi == nullptr) {
     set_error("gemm_tf32x3: invalid arguments (ntypes=%d M=%d K=%d N=%d mode=%d)", ntypes, M,
@@ -262,8 +266,12 @@ int gemm_prepare(const float* A, int M, int K, const float* const* b_hi,
   shp.split_b = b_lo == nullptr ? 1 : 0;
   shp.terms = tune_value("fit_terms", 3) == 4 ? 4 : 3;
   for (int t = 0; t < ntypes; ++t) {
-    if ((rc = make_map(&maps.bh[t], b_hi[t], N, K, BN))) return rc;
-    if ((rc = make_map(&maps.bl[t], shp.split_b ? b_hi[t] : b_lo[t], N, K, BN))) return rc;
+    // FP16 weights: rows of 32 hi and 32 lo halves per k-block, as many bytes
+    // as 32 FP32 values
+    const int cols = f16 ? (K + GT_BK - 1) / GT_BK * GT_BK : K;
+    if ((rc = make_map(&maps.bh[t], b_hi[t], N, cols, BN, f16))) return rc;
+    if (!f16 && (rc = make_map(&maps.bl[t], shp.split_b ? b_hi[t] : b_lo[t], N, K, BN)))
+      return rc;
   }
   auto misaligned = [](const void* q) { return ((uintptr_t)q & 15) != 0; };
   bool bad = misaligned(out0) || misaligned(out1) || misaligned(aux0) || misaligned(aux1);
@@ -287,6 +295,21 @@ int gemm_prepare(const float* A, int M, int K, const float* const* b_hi,
     ep.idt[t] = idt ? idt[t] : nullptr;
     ep.w[t] = w ? w[t] : nullptr;
   }
+  return DPB_OK;
+}
+
+// Turns a GEMM prepared with TF32 weights into its FP16 form (maps, scales).
+int gemm_set_f16(const void* const* b, const float* a_scale, const float* b_scale,
+                 const float* row_scale, int BN, GemmMaps& maps, GemmShape& shp, GemmEpi& ep) {
+  const int cols = (shp.K + GT_BK - 1) / GT_BK * GT_BK;
+  for (int t = 0; t < shp.ntypes; ++t) {
+    const int rc = make_map(&maps.bh[t], static_cast<const float*>(b[t]), shp.N, cols, BN, true);
+    if (rc) return rc;
+    ep.a_scale[t] = a_scale[t];
+    ep.inv_scale[t] = 1.f / (a_scale[t] * b_scale[t]);
+  }
+  ep.row_scale = row_scale;
+  shp.split_b = 0;
   return DPB_OK;
 }
 
@@ -315,6 +338,36 @@ int dpb_gemm_tf32x3_f32(const float* A, int M, int K, const float* const* b_hi,
   if (BN == CfgN240::BN) return launch<CfgN240>(maps, shp, ep, status, st);
   if (BN == CfgN160::BN) return launch<CfgN160>(maps, shp, ep, status, st);
   return launch<CfgN80>(maps, shp, ep, status, st);
+}
+
+int dpb_gemm_f16x3_f32(const float* A, int M, int K, const float* row_scale,
+                       const float* a_scale, const void* const* b, const float* b_scale, int N,
+                       const int* type_rows, int ntypes, int mode, float* out0, float* out1,
+                       const float* aux0, const float* aux1, const float* const* bias,
+                       const float* const* idt, const float* const* w, float* e, int* status,
+                       dpb_stream_t stream) {
+  if (status == nullptr || a_scale == nullptr || b_scale == nullptr) {
+    set_error("gemm_f16x3: a status word and the operand scales are required");
+    return DPB_ERR_INVALID;
+  }
+  GemmMaps maps;
+  GemmShape shp;
+  GemmEpi ep;
+  int BN = 0;
+  const int rc = gemm_prepare(A, M, K, reinterpret_cast<const float* const*>(b), nullptr, N,
+                              type_rows, ntypes, mode, out0, out1, aux0, aux1, bias, idt, w, e, 0,
+                              maps, shp, ep, BN, true);
+  if (rc || M == 0) return rc;
+  shp.split_b = 0;
+  ep.row_scale = row_scale;
+  for (int t = 0; t < ntypes; ++t) {
+    ep.a_scale[t] = a_scale[t];
+    ep.inv_scale[t] = 1.f / (a_scale[t] * b_scale[t]);
+  }
+  cudaStream_t st = as_stream(stream);
+  if (BN == CfgH240::BN) return launch<CfgH240>(maps, shp, ep, status, st);
+  if (BN == CfgH160::BN) return launch<CfgH160>(maps, shp, ep, status, st);
+  return launch<CfgH80>(maps, shp, ep, status, st);
 }
 
 long long dpb_fit_energy_sum_work_bytes(void) {

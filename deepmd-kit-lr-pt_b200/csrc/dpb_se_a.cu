@@ -209,13 +209,13 @@ __global__ void __launch_bounds__(CHEB_A * 32, 4)
 k_desc_fwd_cheb(float* __restrict__ xyz_out, float* __restrict__ D,
                 const int* __restrict__ drow, const float* __restrict__ em,
                 const __grid_constant__ ChebTables ct, const __grid_constant__ TypeTables tt,
-                int nloc, int M, int naxis, float inv_nnei, unsigned* touched) {
+                int nloc, int M, int naxis, float inv_nnei, unsigned* touched, float* row_scale) {
   extern __shared__ float4 dsm4[];
   pdl_wait();
   pdl_trigger();
   cheb_fwd_group<CH, NC>(blockIdx.x * CHEB_A, nloc, threadIdx.x >> 5, threadIdx.x & 31, 0,
                          reinterpret_cast<float*>(dsm4), xyz_out, D, drow, em, ct, tt, M, naxis,
-                         inv_nnei, touched);
+                         inv_nnei, touched, row_scale);
 }
 
 template <int CH, int NC>
@@ -231,6 +231,19 @@ k_desc_bwd_cheb(float* __restrict__ net_deriv, const float* __restrict__ dD,
   cheb_bwd_group<CH, NC>(blockIdx.x * CHEB_A, nloc, threadIdx.x >> 5, threadIdx.x & 31, 0,
                          reinterpret_cast<float*>(dsm4), net_deriv, dD, drow, xyz, em, ct, tt, M,
                          naxis, inv_nnei, touched);
+}
+
+// the operand scales of the descriptor rows from xyz, for the passes that do
+// not write them themselves
+__global__ void __launch_bounds__(256)
+k_row_scale(float* __restrict__ row_scale, const float* __restrict__ xyz,
+            const int* __restrict__ drow, int nloc, int M) {
+  pdl_wait();
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (i >= nloc) return;
+  const float sc = descriptor_scale(xyz + (size_t)i * 4 * M, M, lane);
+  if (lane == 0) row_scale[drow[i]] = sc;
 }
 
 template <typename T>
@@ -557,8 +570,8 @@ static int cheb_args(TypeTables& tt, ChebTables& ct, const float* const* tables,
 
 static int desc_fwd_cheb(float* xyz, float* descrpt, const int* descrpt_row, const float* em,
                          const float* const* tables, const float* table_info,
-                         const dpb_cheb_net* nets, unsigned* touched, const int* sec, int nsec,
-                         int nloc, int M, int naxis, cudaStream_t st) {
+                         const dpb_cheb_net* nets, unsigned* touched, float* row_scale,
+                         const int* sec, int nsec, int nloc, int M, int naxis, cudaStream_t st) {
   TypeTables tt;
   ChebTables ct;
   int rc = cheb_args(tt, ct, tables, table_info, nets, sec, nsec, M, naxis);
@@ -569,7 +582,7 @@ static int desc_fwd_cheb(float* xyz, float* descrpt, const int* descrpt_row, con
   DPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
            "se_a_descriptor_fwd_cheb");
   DPB_CUDA(launch_pdl(kern, dim3(ceil_div(nloc, CHEB_A)), dim3(CHEB_A * 32), smem, st, xyz,
-                      descrpt, descrpt_row, em, ct, tt, nloc, M, naxis, inv, touched),
+                      descrpt, descrpt_row, em, ct, tt, nloc, M, naxis, inv, touched, row_scale),
            "se_a_descriptor_fwd_cheb");
   return DPB_OK;
 }
@@ -598,14 +611,28 @@ static int desc_bwd_cheb(float* net_deriv, const float* d_descrpt, const int* de
 
 extern "C" {
 
+int dpb_se_a_row_scale_f32(float* row_scale, const float* xyz, const int* descrpt_row, int nloc,
+                           int last_layer_size, dpb_stream_t stream) {
+  if (nloc < 0 || last_layer_size < 1 ||
+      (nloc > 0 && (row_scale == nullptr || xyz == nullptr || descrpt_row == nullptr))) {
+    set_error("se_a_row_scale: invalid arguments");
+    return DPB_ERR_INVALID;
+  }
+  if (nloc == 0) return DPB_OK;
+  DPB_CUDA(launch_pdl(k_row_scale, dim3(ceil_div(nloc, 8)), dim3(256), 0, as_stream(stream),
+                      row_scale, xyz, descrpt_row, nloc, last_layer_size),
+           "se_a_row_scale");
+  return DPB_OK;
+}
+
 int dpb_se_a_descriptor_fwd_cheb_f32(float* xyz, float* descrpt, const int* descrpt_row,
                                      const float* em, const float* const* tables,
                                      const float* table_info, const dpb_cheb_net* nets,
-                                     unsigned* touched, const int* sec, int nsec, int nloc,
-                                     int last_layer_size, int axis_neuron,
+                                     unsigned* touched, float* row_scale, const int* sec,
+                                     int nsec, int nloc, int last_layer_size, int axis_neuron,
                                      dpb_stream_t stream) {
-  return desc_fwd_cheb(xyz, descrpt, descrpt_row, em, tables, table_info, nets, touched, sec,
-                       nsec, nloc, last_layer_size, axis_neuron, as_stream(stream));
+  return desc_fwd_cheb(xyz, descrpt, descrpt_row, em, tables, table_info, nets, touched,
+                       row_scale, sec, nsec, nloc, last_layer_size, axis_neuron, as_stream(stream));
 }
 
 int dpb_se_a_descriptor_bwd_cheb_f32(float* net_deriv, const float* d_descrpt,

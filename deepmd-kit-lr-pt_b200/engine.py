@@ -113,7 +113,7 @@ class ForwardLower:
              ptr(self.status), s)
         pt = self.ptab
         pt.forward(self.xyz, self.D, self.drow, self.em, sec, nloc, M, ax, s)
-        self.fit.forward_backward(self.D[:nloc], self.dD[:nloc], energy)
+        self.fit.forward_backward(self.D[:nloc], self.dD[:nloc], energy, pt.row_scale)
         pt.backward(self.net_deriv, self.dD, self.drow, self.xyz, self.em, sec, nloc, M, ax, s)
         call("dpb_force_virial_a_env_mixed_acc", ptr(force), ptr(virial), ptr(self.net_deriv),
              ptr(c), ptr(t), ptr(self.std), ptr(self.nlist), ptr(self.identity), nloc, nall,

@@ -503,8 +503,13 @@ typedef struct {
 DPB_API int dpb_bt_step_create(void** plan, const dpb_bt_step_desc* desc);
 /* Runs the plan's descriptor passes on piecewise Chebyshev nets, as
  * dpb_se_a_descriptor_{fwd,bwd}_cheb_f32 with the plan's quintic tables
- * (table_degree 5 only); touched as there. */
-DPB_API int dpb_bt_step_set_nets(void* plan, const dpb_cheb_net* nets, unsigned* touched);
+ * (table_degree 5 only), and its GEMMs in the form of dpb_gemm_f16x3_f32.
+ * touched, row_scale as there (row_scale is required); b, a_scale, b_scale: the
+ * six GEMMs' weights and scales one after another, ntypes each (a failure
+ * leaves the plan unusable). */
+DPB_API int dpb_bt_step_set_nets(void* plan, const dpb_cheb_net* nets, unsigned* touched,
+                                 float* row_scale, const void* const* b, const float* a_scale,
+                                 const float* b_scale);
 /* One step: env, descriptor, fitting, descriptor backward, forces, virials
  * and energies of every frame in ONE cooperative launch (one CTA per SM),
  * preceded by a 32-byte memset of the barrier and work counters. */
@@ -586,17 +591,22 @@ DPB_API int dpb_se_a_descriptor_bwd_cubic_f32(float* net_deriv, const float* d_d
  * outside [lo, hi) are evaluated from tables / table_info, the quintic tables
  * of dpb_se_a_pack_table_f32. touched (device, [ceil(nloc/8) * (nsec-1)], may be NULL): written by
  * the forward, the intervals each group of eight atoms uses; the backward of
- * the same rows evaluates only those (NULL: all). */
+ * the same rows evaluates only those (NULL: all). row_scale (device, may be
+ * NULL): per descriptor row, the operand scale of dpb_gemm_f16x3_f32. */
 DPB_API int dpb_se_a_descriptor_fwd_cheb_f32(
     float* xyz, float* descrpt, const int* descrpt_row, const float* em,
     const float* const* tables, const float* table_info, const dpb_cheb_net* nets,
-    unsigned* touched, const int* sec, int nsec, int nloc, int last_layer_size, int axis_neuron,
+    unsigned* touched, float* row_scale, const int* sec, int nsec, int nloc, int last_layer_size, int axis_neuron,
     dpb_stream_t stream);
 DPB_API int dpb_se_a_descriptor_bwd_cheb_f32(
     float* net_deriv, const float* d_descrpt, const int* descrpt_row, const float* xyz,
     const float* em, const float* const* tables, const float* table_info,
     const dpb_cheb_net* nets, const unsigned* touched, const int* sec, int nsec, int nloc,
     int last_layer_size, int axis_neuron, dpb_stream_t stream);
+/* The operand scales of dpb_gemm_f16x3_f32 for descriptor rows made by the
+ * other forward passes, from their xyz. */
+DPB_API int dpb_se_a_row_scale_f32(float* row_scale, const float* xyz, const int* descrpt_row,
+                                   int nloc, int last_layer_size, dpb_stream_t stream);
 /* prod_force_a + prod_virial_a in one pass with FP64 accumulation; ghost
  * forces are added to their owner mapping[j] (force: [nforce, 3], nforce =
  * nloc with a mapping, nall without). atom_virial [nall, 9] may be NULL. */
@@ -661,6 +671,20 @@ DPB_API int dpb_gemm_tf32x3_f32(const float* A, int M, int K,
                                 const float* aux1, const float* const* bias,
                                 const float* const* idt, const float* const* w,
                                 float* e, int* status, dpb_stream_t stream);
+/* The same GEMM and epilogues with the operands as two FP16 terms (three
+ * products, twice the tensor-core rate of TF32 at the same 22-23 significant
+ * bits). Row r of A, of type t, is multiplied by a_scale[t] (host, a power of
+ * two) and, where row_scale (device [M], powers of two) is not NULL, by
+ * row_scale[r]; the scaled values must stay below 2^15. b (host array of
+ * device pointers): B[n, k] * b_scale[t] as halves, per row n and block of 32 k
+ * (zero beyond K) the 32 hi terms, then the 32 lo terms. */
+DPB_API int dpb_gemm_f16x3_f32(const float* A, int M, int K, const float* row_scale,
+                               const float* a_scale, const void* const* b, const float* b_scale,
+                               int N, const int* type_rows, int ntypes, int mode, float* out0,
+                               float* out1, const float* aux0, const float* aux1,
+                               const float* const* bias, const float* const* idt,
+                               const float* const* w, float* e, int* status,
+                               dpb_stream_t stream);
 /* energy[0] = e_const + sum of e[0, n) in FP64 (fixed summation order), then
  * e[0, n) = 0: the per-row energies the mode-3 epilogue accumulates, reduced
  * and cleared for the next step's accumulation. work: device buffer of
