@@ -28,13 +28,16 @@ constexpr uint32_t TM_COLS = 512;
 // F16: operands as two FP16 terms (kind::f16, K = 16 per instruction) instead of
 // two TF32 terms (K = 8); a weight row's k-block then holds 32 hi and 32 lo
 // halves side by side, one 128-byte row as well
+// CONVG: groups of four warps that split A, k-blocks in turn
 template <int BN_, int STAGES_, int ASLOTS_, int ACCBUF_, int EPIW_, bool BSPLIT_ = true,
-          bool F16_ = false>
+          bool F16_ = false, int CONVG_ = 1>
 struct GemmCfg {
   static constexpr int BN = BN_, STAGES = STAGES_, ASLOTS = ASLOTS_, ACCBUF = ACCBUF_,
                        EPIW = EPIW_;
   static constexpr bool BSPLIT = BSPLIT_, F16 = F16_;
-  static constexpr int EPI0 = BSPLIT ? 10 : 6;  // first epilogue warp
+  static constexpr int CONVG = CONVG_;
+  static constexpr int CONV1 = 2 + 4 * CONVG;            // end of the A-split warps
+  static constexpr int EPI0 = CONV1 + (BSPLIT ? 4 : 0);  // first epilogue warp
   static constexpr int THREADS = 32 * EPI0 + 32 * EPIW;
   static constexpr uint32_t ACC_STRIDE = BN <= 128 ? 128u : (uint32_t)((BN + 31) / 32 * 32);
   static constexpr uint32_t A0 = ACCBUF * ACC_STRIDE;
@@ -46,6 +49,7 @@ struct GemmCfg {
   static_assert(BN % 16 == 0 && BN <= 256, "MMA N");
   static_assert(A0 + ASW * ASLOTS <= TM_COLS, "tensor memory columns");
   static_assert(!(F16 && BSPLIT), "FP16 weights come split");
+  static_assert(CONVG == 1 || !BSPLIT, "the B-split warps follow one A-split group");
   static_assert(STAGE_BYTES % 1024 == 0, "stage alignment for the 128-byte swizzle");
   static_assert(SMEM <= 232448, "shared memory per CTA");
   static_assert(EPIW == 4 || EPIW == 8, "epilogue warps");
@@ -69,9 +73,9 @@ using CfgN80C = GemmCfg<80, 6, 4, 2, 8>;
 // 331,776 rows, TF32 -> FP16: K = 1600 layer 1.56 -> 1.26 ms, N = 1600 1.58 -> 1.33 ms
 // (the MMAs halved; the K = 1600 layer now reads its operands from L2 at 8 TB/s),
 // the 240 x 240 layers unchanged (their epilogues bound them)
-using CfgH80 = GemmCfg<80, 8, 8, 2, 8, false, true>;
-using CfgH160 = GemmCfg<160, 6, 6, 2, 8, false, true>;
-using CfgH240 = GemmCfg<240, 4, 8, 1, 8, false, true>;
+using CfgH80 = GemmCfg<80, 8, 8, 2, 8, false, true, 2>;
+using CfgH160 = GemmCfg<160, 6, 6, 2, 8, false, true, 2>;
+using CfgH240 = GemmCfg<240, 4, 8, 1, 8, false, true, 2>;
 
 enum : int {
   ST_MMA_TIMEOUT = 1 << 8,
@@ -537,8 +541,9 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
         if (mbar_try(drain, 0)) break;
     }
     __syncwarp();
-  } else if (warp < 6) {
+  } else if (warp < CFG::CONV1) {
     // ------------------------------------------- split A into TMEM hi / lo
+    const int grp = (warp - 2) >> 2;  // takes the k-blocks g = grp modulo CONVG
     const uint32_t lane_base = 32u * (uint32_t)(warp & 3);
     const int r = (int)lane_base + lane;  // tile row of this thread
     int g = 0;
@@ -552,6 +557,7 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
           sc *= __ldg(epi.row_scale + tc.row0 + r);
       }
       for (int kb = 0; kb < nk; ++kb, ++g) {
+        if (CFG::CONVG > 1 && g % CFG::CONVG != grp) continue;
         const int s = g % STAGES;
         const uint32_t ph = (g / STAGES) & 1;
         const int as = g % ASLOTS;
@@ -593,7 +599,7 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
         mbar_arrive(&conv_bar[s]);
       }
     }
-  } else if (CFG::BSPLIT && warp < 10) {
+  } else if (CFG::BSPLIT && warp < CFG::EPI0) {
     // ------------------------------------- split FP32 B tiles into hi / lo
     // (only with FP32 weights): TF32 hi in place, lo into the lo buffer at the
     // same swizzled offset; rows r and r + 128 of the BN-row tile
