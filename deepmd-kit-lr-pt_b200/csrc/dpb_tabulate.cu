@@ -1,13 +1,20 @@
 // Compressed se_a embedding: the quintic table G_m(x) fused with the
 // contraction over neighbors (tabulate_fusion_se_a and its two gradients).
 //
-// Layout: one warp per (center atom, block of up to 128 embedding channels m);
-// lane l owns channels m = mb + 32c + l. A neighbor's table row is read once
-// per warp as contiguous 24-byte (FP32) / 48-byte (FP64) coefficient groups,
-// so a warp-wide load covers a contiguous 768 B / 1.5 KB span of the row.
-// The forward and grad_grad accumulate over neighbors in registers; the
-// gradient reduces over channels with a butterfly and keeps the result in the
-// lane that owns the neighbor, flushing 32 neighbors per coalesced store.
+// Layout: one warp per (center atom, block of 64 embedding channels). The
+// reference's table row holds a channel's six coefficients side by side; read
+// per channel (24 or 48 bytes per lane) every line of the row went through L1
+// three times, and one warp per atom left small systems waiting on each row.
+// Here a row is read as it lies, 16 bytes per lane, and a lane works on
+// coefficient pairs: pair q of the row belongs to channel q / 3 and powers
+// 2 (q % 3), + 1, so its term is a.x t^k + a.y t^(k + 1), summed over slots per
+// pair and over a channel's three pairs once at the end (forward), or multiplied
+// by the channel's gradient at once (backward). Slots are located 32 at a time,
+// one per lane, and the next slot's row is in flight while one is summed.
+// Measured, 92 slots, M = 100, FP32: forward 192 atoms 68 -> 19 us, 12,288 atoms
+// 234 -> 191 us (now FP32 issue and the L2 reads of the rows), grad_grad 70 -> 21
+// and 260 -> 258 us, gradient 78 -> 31 us at 192 atoms (k_tab_grad below; many
+// atoms stay on k_tab_grad_channels).
 //
 // Semantics follow the CPU reference (source/lib/src/tabulate.cc): locate_xx
 // (:45-73) with the nextafter upper bound (:21-30), linear extrapolation
@@ -70,6 +77,345 @@ __device__ __forceinline__ void locate(const TabInfo<T>& t, T x, int& idx, T& xx
   }
 }
 
+// First slot of the sorted padding tail, or nnei when there is none.
+template <typename T>
+__device__ __forceinline__ int fold_start(const T* em_x, const T* em, int nnei, int lane) {
+  const T last = em_x[nnei - 1];
+  for (int base = 0; base < nnei; base += 32) {
+    int jj = base + lane;
+    bool c = false;
+    if (jj < nnei) {
+      const T* e = em + (size_t)jj * 4;
+      c = em_x[jj] == last && e[1] == (T)0. && e[2] == (T)0. && e[3] == (T)0.;
+    }
+    unsigned b = __ballot_sync(0xffffffffu, c);
+    if (b) return base + __ffs(b) - 1;
+  }
+  return nnei;
+}
+
+constexpr int TW = 4;     // warps per block
+constexpr int TB = 64;    // channels per warp
+constexpr int TP = 6;     // coefficient pairs per lane (3 TB / 32)
+constexpr int TS = 12;    // staged values per slot: six weights of the value, six of
+                          // the slope
+
+template <typename T>
+struct Pair;
+template <>
+struct Pair<float> {
+  using type = float2;
+};
+template <>
+struct Pair<double> {
+  using type = double2;
+};
+
+// The pairs a lane owns. VW = 4: FP32 rows read as float4 (M even and the table
+// 16-byte aligned), two neighboring pairs per load; VW = 2: one pair per load
+// (float2 or double2).
+template <int VW>
+__device__ __forceinline__ int pair_index(int p, int lane) {
+  return VW == 4 ? 2 * (lane + 32 * (p >> 1)) + (p & 1) : lane + 32 * p;
+}
+// acc[0..3] += u e[0..3]; FP32 two at a time
+__device__ __forceinline__ void axpy4(float (&acc)[4], float u, const float (&e)[4]) {
+  const float2 uu = make_float2(u, u);
+  const float2 lo = __ffma2_rn(uu, make_float2(e[0], e[1]), make_float2(acc[0], acc[1]));
+  const float2 hi = __ffma2_rn(uu, make_float2(e[2], e[3]), make_float2(acc[2], acc[3]));
+  acc[0] = lo.x, acc[1] = lo.y, acc[2] = hi.x, acc[3] = hi.y;
+}
+__device__ __forceinline__ void axpy4(double (&acc)[4], double u, const double (&e)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) acc[k] = fma(u, e[k], acc[k]);
+}
+
+// four consecutive staged values (16-byte aligned)
+template <typename T>
+__device__ __forceinline__ void load4(T (&v)[4], const T* p) {
+  using T2 = typename Pair<T>::type;
+  if constexpr (sizeof(T) == 4) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+  } else {
+    const T2 a = reinterpret_cast<const T2*>(p)[0], b = reinterpret_cast<const T2*>(p)[1];
+    v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+  }
+}
+
+// which of the lane's three staged power pairs pair p uses: the staged pairs are
+// rotated by the lane's class, pair_index(0, lane) % 3
+template <int VW>
+__host__ __device__ constexpr int pair_power(int p) {
+  return VW == 4 ? (64 * (p >> 1) + (p & 1)) % 3 : (32 * p) % 3;
+}
+
+template <typename T, int VW>
+__device__ __forceinline__ void load_row(typename Pair<T>::type (&a)[TP], const T* row, int npair,
+                                         int lane) {
+  using T2 = typename Pair<T>::type;
+  if constexpr (VW == 4) {
+#pragma unroll
+    for (int i = 0; i < TP / 2; ++i) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (2 * (lane + 32 * i) < npair)  // M even: npair is even too
+        v = __ldg(reinterpret_cast<const float4*>(row) + lane + 32 * i);
+      a[2 * i] = make_float2(v.x, v.y);
+      a[2 * i + 1] = make_float2(v.z, v.w);
+    }
+  } else {
+#pragma unroll
+    for (int p = 0; p < TP; ++p) {
+      a[p].x = a[p].y = (T)0;
+      if (lane + 32 * p < npair) a[p] = __ldg(reinterpret_cast<const T2*>(row) + lane + 32 * p);
+    }
+  }
+}
+
+// one slot per lane: its row and the weights w_k of the value (with the linear
+// extrapolation, tabulate.cc:116-144: v + g delta) and dw_k of the slope
+template <typename T>
+__device__ __forceinline__ int stage_weights(T* sw, const TabInfo<T>& ti, T x, int lane) {
+  int idx;
+  T t, delta;
+  locate(ti, x, idx, t, delta);
+  T p = (T)1, d = (T)0;  // t^k, k t^(k - 1)
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    sw[lane * TS + k] = d != (T)0 ? p + delta * d : p;  // an infinite delta stays out of
+                                                        // the powers that have no slope
+    sw[lane * TS + 6 + k] = d;
+    d = (T)(k + 1) * p;
+    p *= t;
+  }
+  return idx;
+}
+
+// out[i,k,m] = sum_jj w_jj * (G_m(x_jj) * em[jj,k])              (forward)
+// out[i,k,m] = sum_jj w_jj * (G_m * dz_dem[jj,k] + dz_dem_x[jj] * G'_m * em[jj,k])
+//                                                   (GG: grad_grad)
+template <typename T, int VW, bool GG>
+__global__ void __launch_bounds__(TW * 32)
+k_tab_fwd(T* __restrict__ out, const T* __restrict__ table, TabInfo<T> ti,
+          const T* __restrict__ em_x, const T* __restrict__ em, int nloc, int nnei, int M,
+          const T* __restrict__ dz_dem_x, const T* __restrict__ dz_dem) {
+  using T2 = typename Pair<T>::type;
+  // per warp: weights [32][TS], env rows [32][4] (GG: and the two multipliers of
+  // value and slope); the pair sums of one env column at the end
+  __shared__ __align__(16) T s_w[TW][32 * TS];
+  __shared__ __align__(16) T s_e[TW][32 * (GG ? 8 : 4)];
+  __shared__ int s_row[TW][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * TW + w;
+  if (i >= nloc) return;
+  const int m0 = blockIdx.y * TB, npair = 3 * min(TB, M - m0);
+  const int cls = pair_index<VW>(0, lane) % 3;
+  const int off[3] = {2 * cls, 2 * ((cls + 1) % 3), 2 * ((cls + 2) % 3)};
+  T acc[TP][4];
+#pragma unroll
+  for (int p = 0; p < TP; ++p)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[p][k] = (T)0;
+  const T* ex = em_x + (size_t)i * nnei;
+  const T* ee = em + (size_t)i * nnei * 4;
+  const int brk = fold_start(ex, ee, nnei, lane);
+  const int last = brk < nnei ? brk : nnei - 1;
+  for (int base = 0; base <= last; base += 32) {
+    const int cnt = min(32, last + 1 - base), jj = base + lane;
+    if (lane < cnt) {
+      const T rep = jj == brk ? (T)(nnei - jj) : (T)1;
+      s_row[w][lane] = stage_weights(s_w[w], ti, ex[jj], lane);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (GG) {
+          const size_t at = (size_t)i * nnei + jj;
+          s_e[w][lane * 8 + k] = rep * dz_dem[at * 4 + k];
+          s_e[w][lane * 8 + 4 + k] = rep * dz_dem_x[at] * ee[jj * 4 + k];
+        } else {
+          s_e[w][lane * 4 + k] = rep * ee[jj * 4 + k];
+        }
+      }
+    }
+    __syncwarp();
+    const T* tab = table + (size_t)m0 * 6;
+    const int rs = M * 6;
+    T2 a[2][TP];  // two rows in turn: the next slot's is in flight
+    auto fetch = [&](T2 (&v)[TP], int q) {
+      load_row<T, VW>(v, tab + (size_t)s_row[w][q] * rs, npair, lane);
+    };
+    auto slot = [&](const T2 (&v)[TP], int q) {
+      T2 pw[3], dw[3];
+      const T* sw = s_w[w] + q * TS;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        pw[j] = *reinterpret_cast<const T2*>(sw + off[j]);
+        if (GG) dw[j] = *reinterpret_cast<const T2*>(sw + 6 + off[j]);
+      }
+      T e[4], f[4];
+      load4(e, s_e[w] + q * (GG ? 8 : 4));
+      if (GG) load4(f, s_e[w] + q * 8 + 4);
+#pragma unroll
+      for (int p = 0; p < TP; ++p) {
+        const T2 z = pw[pair_power<VW>(p)];
+        axpy4(acc[p], fma(v[p].x, z.x, v[p].y * z.y), e);
+        if (GG) {
+          const T2 dz = dw[pair_power<VW>(p)];
+          axpy4(acc[p], fma(v[p].x, dz.x, v[p].y * dz.y), f);
+        }
+      }
+    };
+    fetch(a[0], 0);
+    for (int q = 0; q < cnt; q += 2) {
+      if (q + 1 < cnt) fetch(a[1], q + 1);
+      slot(a[0], q);
+      if (q + 2 < cnt) fetch(a[0], q + 2);
+      if (q + 1 < cnt) slot(a[1], q + 1);
+    }
+    __syncwarp();
+  }
+  // a channel's three pairs, one env column at a time
+  T* red = s_w[w];
+  static_assert(32 * TS >= 3 * TB, "the pair sums reuse the staging");
+  T* o = out + (size_t)i * 4 * M + m0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+#pragma unroll
+    for (int p = 0; p < TP; ++p) red[pair_index<VW>(p, lane)] = acc[p][k];
+    __syncwarp();
+    for (int c = lane; 3 * c < npair; c += 32)
+      o[k * M + c] = red[3 * c] + red[3 * c + 1] + red[3 * c + 2];
+    __syncwarp();
+  }
+}
+
+// dy_dem_x[i,jj] = sum_m G'_m * sum_k em[jj,k] dy[k,m]
+// dy_dem[i,jj,k] = sum_m G_m * dy[k,m]           (tabulate.cc:234-341)
+// A CTA holds the nmb channel blocks of blockDim / (32 nmb) atoms; a warp's
+// five sums per slot are reduced over its lanes in groups of four slots and
+// over the blocks in shared memory.
+template <typename T, int VW>
+__global__ void __launch_bounds__(512)
+k_tab_grad(T* __restrict__ dy_dem_x, T* __restrict__ dy_dem, const T* __restrict__ table,
+           TabInfo<T> ti, const T* __restrict__ em_x, const T* __restrict__ em,
+           const T* __restrict__ dy, int nloc, int nnei, int M, int nmb) {
+  using T2 = typename Pair<T>::type;
+  extern __shared__ __align__(16) unsigned char tab_smem[];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  T* s_w = reinterpret_cast<T*>(tab_smem) + (size_t)w * 32 * (TS + 4 + 5);
+  T* s_e = s_w + 32 * TS;
+  T* s_r = s_e + 32 * 4;  // [32][5]
+  int* s_row = reinterpret_cast<int*>(reinterpret_cast<T*>(tab_smem) +
+                                      (size_t)nw * 32 * (TS + 4 + 5)) + w * 32;
+  const int mb = w % nmb;
+  const int i = blockIdx.x * (nw / nmb) + w / nmb;
+  const bool act = i < nloc;
+  const int m0 = mb * TB, npair = 3 * min(TB, M - m0);
+  const int cls = pair_index<VW>(0, lane) % 3;
+  const int off[3] = {2 * cls, 2 * ((cls + 1) % 3), 2 * ((cls + 2) % 3)};
+  const T* ex = em_x + (size_t)(act ? i : 0) * nnei;
+  const T* ee = em + (size_t)(act ? i : 0) * nnei * 4;
+  T dyr[TP][4];
+#pragma unroll
+  for (int p = 0; p < TP; ++p) {
+    const int q = pair_index<VW>(p, lane);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      dyr[p][k] = act && q < npair ? dy[(size_t)i * 4 * M + k * M + m0 + q / 3] : (T)0;
+  }
+  const int brk = fold_start(ex, ee, nnei, lane);
+  const int last = brk < nnei ? brk : nnei - 1;
+  const int b4 = (lane >> 4) & 1, b3 = (lane >> 3) & 1;
+  for (int base = 0; base < nnei; base += 32) {
+    const int cnt = act ? max(0, min(32, last + 1 - base)) : 0, jj = base + lane;
+    if (lane < cnt) {
+      s_row[lane] = stage_weights(s_w, ti, ex[jj], lane);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) s_e[lane * 4 + k] = ee[jj * 4 + k];
+    }
+    __syncwarp();
+    // two rows in turn, the next slot's in flight (FP64: one, the registers of a
+    // second would not fit a 16-warp CTA)
+    constexpr int NB = sizeof(T) == 4 ? 2 : 1;
+    const T* tab = table + (size_t)m0 * 6;
+    const int rs = M * 6;
+    T2 a[NB][TP];
+    auto fetch = [&](T2 (&v)[TP], int q) {
+      load_row<T, VW>(v, tab + (size_t)s_row[q] * rs, npair, lane);
+    };
+    if (NB == 2 && cnt > 0) fetch(a[0], 0);
+    for (int q0 = 0; q0 < cnt; q0 += 4) {
+      T S[4][5];  // per slot: the slope's sum, then the value's per env column
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int q = q0 + u;
+        T V[4] = {(T)0, (T)0, (T)0, (T)0}, Q[4] = {(T)0, (T)0, (T)0, (T)0}, sl = (T)0;
+        if (q < cnt) {
+          if (NB == 1)
+            fetch(a[0], q);
+          else if (q + 1 < cnt)
+            fetch(a[(u + 1) % NB], q + 1);
+          const T2(&v)[TP] = a[u % NB];
+          const T* sw = s_w + q * TS;
+          T2 pw[3], dw[3];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            pw[j] = *reinterpret_cast<const T2*>(sw + off[j]);
+            dw[j] = *reinterpret_cast<const T2*>(sw + 6 + off[j]);
+          }
+#pragma unroll
+          for (int p = 0; p < TP; ++p) {
+            const T2 z = pw[pair_power<VW>(p)], dz = dw[pair_power<VW>(p)];
+            axpy4(V, fma(v[p].x, z.x, v[p].y * z.y), dyr[p]);
+            axpy4(Q, fma(v[p].x, dz.x, v[p].y * dz.y), dyr[p]);
+          }
+          T e[4];
+          load4(e, s_e + q * 4);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) sl = fma(e[k], Q[k], sl);
+        }
+        S[u][0] = sl;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) S[u][k + 1] = V[k];
+      }
+      // the xor-16 and -8 steps leave slot 2 b4 + b3 in a lane, summed over 8
+      // lanes; xor-4, -2 and -1 finish the sum
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        T r0 = (b4 ? S[2][k] : S[0][k]) +
+               __shfl_xor_sync(0xffffffffu, b4 ? S[0][k] : S[2][k], 16);
+        T r1 = (b4 ? S[3][k] : S[1][k]) +
+               __shfl_xor_sync(0xffffffffu, b4 ? S[1][k] : S[3][k], 16);
+        T v = (b3 ? r1 : r0) + __shfl_xor_sync(0xffffffffu, b3 ? r0 : r1, 8);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        const int q = q0 + 2 * b4 + b3;
+        if ((lane & 7) == 0 && q < cnt) s_r[q * 5 + k] = v;
+      }
+    }
+    __syncthreads();
+    // the atom's first warp adds the channel blocks; slots after the fold point
+    // keep the zero of the reference's memset
+    if (act && mb == 0 && jj < nnei) {
+      T v[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
+      if (lane < cnt) {
+        for (int b = 0; b < nmb; ++b)
+#pragma unroll
+          for (int k = 0; k < 5; ++k) v[k] += s_r[(size_t)b * 32 * (TS + 4 + 5) + lane * 5 + k];
+        const T rep = jj == brk ? (T)(nnei - jj) : (T)1;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) v[k] *= rep;
+      }
+      dy_dem_x[(size_t)i * nnei + jj] = v[0];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) dy_dem[((size_t)i * nnei + jj) * 4 + k] = v[k + 1];
+    }
+    __syncthreads();
+  }
+}
+
+// The gradient by channels, for many atoms: one warp per atom, lane l owns the
+// channels mb + 32 c + l and reads a channel's six coefficients itself. With the
+// chip full of atoms the smaller instruction count wins over the wide loads.
 template <typename T>
 struct Coef {
   T a0, a1, a2, a3, a4, a5;
@@ -94,95 +440,9 @@ __device__ __forceinline__ void poly(const Coef<T>& a, T xx, T delta, T& v, T& g
   v = v + g * delta;
 }
 
-// First slot of the sorted padding tail, or nnei when there is none.
-template <typename T>
-__device__ __forceinline__ int fold_start(const T* em_x, const T* em, int nnei, int lane) {
-  const T last = em_x[nnei - 1];
-  for (int base = 0; base < nnei; base += 32) {
-    int jj = base + lane;
-    bool c = false;
-    if (jj < nnei) {
-      const T* e = em + (size_t)jj * 4;
-      c = em_x[jj] == last && e[1] == (T)0. && e[2] == (T)0. && e[3] == (T)0.;
-    }
-    unsigned b = __ballot_sync(0xffffffffu, c);
-    if (b) return base + __ffs(b) - 1;
-  }
-  return nnei;
-}
-
-constexpr int TW = 4;  // warps per block
-
 template <typename T, int MC>
 __global__ void __launch_bounds__(TW * 32)
-k_tab_fwd(T* __restrict__ out, const T* __restrict__ table, TabInfo<T> ti,
-          const T* __restrict__ em_x, const T* __restrict__ em, int nloc,
-          int nnei, int M, const T* __restrict__ dz_dem_x,
-          const T* __restrict__ dz_dem) {
-  // out[i,k,m] = sum_jj w_jj * (G_m(x_jj) * em[jj,k])              (forward)
-  // out[i,k,m] = sum_jj w_jj * (G_m * dz_dem[jj,k] + dz_dem_x[jj] * G'_m * em[jj,k])
-  //                                                   (grad_grad, dz_* != NULL)
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int i = blockIdx.x * TW + w;
-  if (i >= nloc) return;
-  const int m0 = blockIdx.y * 32 * MC;
-  const bool gg = dz_dem != nullptr;
-  T acc[MC][4];
-#pragma unroll
-  for (int c = 0; c < MC; ++c)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) acc[c][k] = (T)0.;
-  const T* ex = em_x + (size_t)i * nnei;
-  const T* ee = em + (size_t)i * nnei * 4;
-  const int brk = nnei > 0 ? fold_start(ex, ee, nnei, lane) : 0;
-  for (int jj = 0; jj < nnei; ++jj) {
-    const T x = ex[jj];
-    T e[4] = {ee[jj * 4 + 0], ee[jj * 4 + 1], ee[jj * 4 + 2], ee[jj * 4 + 3]};
-    T h[4] = {(T)0., (T)0., (T)0., (T)0.}, dzx = (T)0.;
-    if (gg) {
-      const T* hz = dz_dem + ((size_t)i * nnei + jj) * 4;
-      h[0] = hz[0]; h[1] = hz[1]; h[2] = hz[2]; h[3] = hz[3];
-      dzx = dz_dem_x[(size_t)i * nnei + jj];
-    }
-    int idx;
-    T xx, delta;
-    locate(ti, x, idx, xx, delta);
-    const T rep = jj == brk ? (T)(nnei - jj) : (T)1.;
-    const T* row = table + (size_t)idx * M * 6;
-#pragma unroll
-    for (int c = 0; c < MC; ++c) {
-      const int m = m0 + c * 32 + lane;
-      if (m < M) {
-        Coef<T> a = load_coef(row + (size_t)m * 6);
-        T v, g;
-        poly(a, xx, delta, v, g);
-        if (!gg) {
-          const T sc = rep * v;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) acc[c][k] += sc * e[k];
-        } else {
-          const T dg = dzx * g;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) acc[c][k] += rep * (v * h[k] + dg * e[k]);
-        }
-      }
-    }
-    if (jj == brk) break;
-  }
-  T* o = out + (size_t)i * 4 * M;
-#pragma unroll
-  for (int c = 0; c < MC; ++c) {
-    const int m = m0 + c * 32 + lane;
-    if (m < M) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) o[k * M + m] = acc[c][k];
-    }
-  }
-}
-
-template <typename T, int MC>
-__global__ void __launch_bounds__(TW * 32)
-k_tab_grad(T* __restrict__ dy_dem_x, T* __restrict__ dy_dem,
+k_tab_grad_channels(T* __restrict__ dy_dem_x, T* __restrict__ dy_dem,
            const T* __restrict__ table, TabInfo<T> ti,
            const T* __restrict__ em_x, const T* __restrict__ em,
            const T* __restrict__ dy, int nloc, int nnei, int M) {
@@ -265,13 +525,21 @@ k_tab_grad(T* __restrict__ dy_dem_x, T* __restrict__ dy_dem,
   }
 }
 
-template <typename T, int MC>
+// 16-byte row loads need an even M (rows of 24 M bytes) and an aligned table;
+// FP64 pairs are 16 bytes (as the reference's double2 loads, an aligned table is
+// required)
+template <typename T>
+static bool wide_rows(const T* table, int M) {
+  return sizeof(T) == 4 && (M & 1) == 0 && (reinterpret_cast<uintptr_t>(table) & 15) == 0;
+}
+
+template <typename T, int VW>
 static void launch_fwd(T* out, const T* table, const TabInfo<T>& ti, const T* em_x,
                        const T* em, int nloc, int nnei, int M, const T* dzx,
                        const T* dze, cudaStream_t st) {
-  dim3 grid(ceil_div(nloc, TW), ceil_div(M, 32 * MC));
-  k_tab_fwd<T, MC><<<grid, TW * 32, 0, st>>>(out, table, ti, em_x, em, nloc, nnei, M,
-                                             dzx, dze);
+  const dim3 grid(ceil_div(nloc, TW), ceil_div(M, TB));
+  auto kern = dze != nullptr ? k_tab_fwd<T, VW, true> : k_tab_fwd<T, VW, false>;
+  kern<<<grid, TW * 32, 0, st>>>(out, table, ti, em_x, em, nloc, nnei, M, dzx, dze);
 }
 
 template <typename T>
@@ -291,10 +559,14 @@ static int tab_fwd(T* out, const T* table, const T* info, const T* em_x,
     DPB_CUDA(cudaMemsetAsync(out, 0, sizeof(T) * (size_t)nloc * 4 * M, st), name);
     return DPB_OK;
   }
-  if (M <= 32) launch_fwd<T, 1>(out, table, ti, em_x, em, nloc, nnei, M, dzx, dze, st);
-  else if (M <= 64) launch_fwd<T, 2>(out, table, ti, em_x, em, nloc, nnei, M, dzx, dze, st);
-  else if (M <= 96) launch_fwd<T, 3>(out, table, ti, em_x, em, nloc, nnei, M, dzx, dze, st);
-  else launch_fwd<T, 4>(out, table, ti, em_x, em, nloc, nnei, M, dzx, dze, st);
+  if constexpr (sizeof(T) == 4) {
+    if (wide_rows(table, M)) {
+      launch_fwd<T, 4>(out, table, ti, em_x, em, nloc, nnei, M, dzx, dze, st);
+      DPB_CHECK_LAUNCH(name);
+      return DPB_OK;
+    }
+  }
+  launch_fwd<T, 2>(out, table, ti, em_x, em, nloc, nnei, M, dzx, dze, st);
   DPB_CHECK_LAUNCH(name);
   return DPB_OK;
 }
@@ -311,11 +583,37 @@ static int tab_grad(T* dy_dem_x, T* dy_dem, const T* table, const T* info,
     return DPB_ERR_INVALID;
   }
   if (nloc == 0 || nnei == 0) return DPB_OK;  // tabulate.cc:251-256
-  dim3 grid(ceil_div(nloc, TW));
-  if (M <= 32) k_tab_grad<T, 1><<<grid, TW * 32, 0, st>>>(dy_dem_x, dy_dem, table, ti, em_x, em, dy, nloc, nnei, M);
-  else if (M <= 64) k_tab_grad<T, 2><<<grid, TW * 32, 0, st>>>(dy_dem_x, dy_dem, table, ti, em_x, em, dy, nloc, nnei, M);
-  else if (M <= 96) k_tab_grad<T, 3><<<grid, TW * 32, 0, st>>>(dy_dem_x, dy_dem, table, ti, em_x, em, dy, nloc, nnei, M);
-  else k_tab_grad<T, 4><<<grid, TW * 32, 0, st>>>(dy_dem_x, dy_dem, table, ti, em_x, em, dy, nloc, nnei, M);
+  // Pairs or channels (us, 92 slots, M = 100, FP32 | FP64): 192 atoms 31 against 78
+  // | 57 against 107, 3,000 atoms 108 against 108 | 211 against 207, 12,288 atoms 367
+  // against 307 | 768 against 588
+  if (nloc > 16 * sm_count()) {
+    const dim3 grid(ceil_div(nloc, TW));
+    auto by = [&](auto kern) {
+      kern<<<grid, TW * 32, 0, st>>>(dy_dem_x, dy_dem, table, ti, em_x, em, dy, nloc, nnei, M);
+    };
+    if (M <= 32) by(k_tab_grad_channels<T, 1>);
+    else if (M <= 64) by(k_tab_grad_channels<T, 2>);
+    else if (M <= 96) by(k_tab_grad_channels<T, 3>);
+    else by(k_tab_grad_channels<T, 4>);
+    DPB_CHECK_LAUNCH("tabulate_fusion_se_a_grad");
+    return DPB_OK;
+  }
+  const int nmb = ceil_div(M, TB);  // at most 16 warps per atom
+  const int atoms = nmb < TW ? TW / nmb : 1, nw = atoms * nmb;
+  const size_t smem = (size_t)nw * 32 * ((TS + 4 + 5) * sizeof(T) + sizeof(int));
+  auto run = [&](auto kern) -> int {
+    if (smem > 48 * 1024)
+      DPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+               "tabulate_fusion_se_a_grad");
+    kern<<<ceil_div(nloc, atoms), nw * 32, smem, st>>>(dy_dem_x, dy_dem, table, ti, em_x, em, dy,
+                                                       nloc, nnei, M, nmb);
+    return DPB_OK;
+  };
+  if constexpr (sizeof(T) == 4)
+    rc = wide_rows(table, M) ? run(k_tab_grad<T, 4>) : run(k_tab_grad<T, 2>);
+  else
+    rc = run(k_tab_grad<T, 2>);
+  if (rc) return rc;
   DPB_CHECK_LAUNCH("tabulate_fusion_se_a_grad");
   return DPB_OK;
 }
