@@ -187,23 +187,38 @@ __device__ __forceinline__ void bt_env_row(int row, int lane, BtEnvSmem& sm,
     }
     tstart = x - tstart;
   }
-  for (int q = 0; q * 32 < n; ++q) {
-    const int kk = q * 32 + lane;
-    const unsigned long long own = kk < n ? sm.keys[kk] : ~0ull;
-    int r = 0;
-    const ulonglong2* k2 = reinterpret_cast<const ulonglong2*>(sm.keys);
+  // rank every key, three of a lane per pass over the list
+  const ulonglong2* k2 = reinterpret_cast<const ulonglong2*>(sm.keys);
+  for (int q = 0; q * 96 < n; ++q) {
+    unsigned long long own[3];
+    int r[3] = {0, 0, 0};
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      const int kk = q * 96 + u * 32 + lane;
+      own[u] = kk < n ? sm.keys[kk] : ~0ull;
+    }
     int p = 0;
     for (; 2 * p + 1 < n; ++p) {  // two keys per 16-byte load (broadcast)
       const ulonglong2 v = k2[p];
-      r += (v.x < own ? 1 : 0) + (v.y < own ? 1 : 0);
+#pragma unroll
+      for (int u = 0; u < 3; ++u) r[u] += (v.x < own[u] ? 1 : 0) + (v.y < own[u] ? 1 : 0);
     }
-    if (2 * p < n) r += sm.keys[2 * p] < own ? 1 : 0;
-    const int t = (int)(own >> 56) & 31;
-    const int ts = __shfl_sync(0xffffffffu, tstart, t);
-    if (kk < n) {
-      const int rr = r - ts;
-      if (rr < sec.sec[t + 1] - sec.sec[t]) sm.row[sec.sec[t] + rr] = (int)(own & 0xFFFFFFull);
-      else atomicOr(status, ST_SEL_OVERFLOW);
+    if (2 * p < n) {
+      const unsigned long long v = sm.keys[2 * p];
+#pragma unroll
+      for (int u = 0; u < 3; ++u) r[u] += v < own[u] ? 1 : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      const int t = (int)(own[u] >> 56) & 31;
+      const int ts = __shfl_sync(0xffffffffu, tstart, t);
+      if (q * 96 + u * 32 + lane < n) {
+        const int rr = r[u] - ts;
+        if (rr < sec.sec[t + 1] - sec.sec[t])
+          sm.row[sec.sec[t] + rr] = (int)(own[u] & 0xFFFFFFull);
+        else
+          atomicOr(status, ST_SEL_OVERFLOW);
+      }
     }
   }
   __syncwarp();

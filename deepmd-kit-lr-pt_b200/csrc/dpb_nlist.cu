@@ -332,25 +332,39 @@ __device__ bool env_one(const EnvIO<CT, OT>& io, const SecInfo& sec, int row,
     tstart = x - tstart;
   }
   // ---- rank every key (keys are unique: they contain the index)
-  for (int q = 0; q * 32 < n; ++q) {
-    int kk = q * 32 + lane;
-    unsigned long long own = kk < n ? keys[kk] : ~0ull;
-    int r = 0;
+  // (three keys of a lane share each pass over the list: a cutoff sphere of
+  // liquid or metal density holds 65-96 atoms)
+  const ulonglong2* k2 = reinterpret_cast<const ulonglong2*>(keys);
+  for (int q = 0; q * 96 < n; ++q) {
+    unsigned long long own[3];
+    int r[3] = {0, 0, 0};
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      const int kk = q * 96 + u * 32 + lane;
+      own[u] = kk < n ? keys[kk] : ~0ull;
+    }
     // two keys per 16-byte shared-memory load (broadcast to the warp)
-    const ulonglong2* k2 = reinterpret_cast<const ulonglong2*>(keys);
     int p = 0;
     for (; 2 * p + 1 < n; ++p) {
       const ulonglong2 v = k2[p];
-      r += (v.x < own ? 1 : 0) + (v.y < own ? 1 : 0);
+#pragma unroll
+      for (int u = 0; u < 3; ++u) r[u] += (v.x < own[u] ? 1 : 0) + (v.y < own[u] ? 1 : 0);
     }
-    if (2 * p < n) r += keys[2 * p] < own ? 1 : 0;
-    int t = (int)(own >> 56) & 31;
-    int ts = __shfl_sync(0xffffffffu, tstart, t);
-    if (kk < n) {
-      int rr = r - ts;
-      int selt = sec.sec[t + 1] - sec.sec[t];
-      if (rr < selt) srow[sec.sec[t] + rr] = (int)(own & 0xFFFFFFull);
-      else atomicOr(io.status, ST_SEL_OVERFLOW);
+    if (2 * p < n) {
+      const unsigned long long v = keys[2 * p];
+#pragma unroll
+      for (int u = 0; u < 3; ++u) r[u] += v < own[u] ? 1 : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      const int t = (int)(own[u] >> 56) & 31;
+      const int ts = __shfl_sync(0xffffffffu, tstart, t);
+      if (q * 96 + u * 32 + lane < n) {
+        const int rr = r[u] - ts;
+        const int selt = sec.sec[t + 1] - sec.sec[t];
+        if (rr < selt) srow[sec.sec[t] + rr] = (int)(own[u] & 0xFFFFFFull);
+        else atomicOr(io.status, ST_SEL_OVERFLOW);
+      }
     }
   }
   __syncwarp();
@@ -486,12 +500,19 @@ static int env_inlist(OT* em, OT* em_deriv, OT* rij, int* nlist, const CT* coord
   GridView g{};
   EnvIO<CT, OT> io{em, em_deriv, rij, nlist, coord, type, g, ilist, numneigh, firstneigh,
                    avg, std_, nloc, nall, rcut, rcut_smth, status};
-  if (max_nbor_size <= 1024) {
-    constexpr int W = 4;
+  // A row's candidates within rcut go to a key buffer in shared memory, at most
+  // max_nbor_size of them; the smallest buffer that holds them lets the most
+  // warps run (20 per SM with 1,024 keys, 32 with 256)
+  constexpr int W = 4;
+  if (max_nbor_size <= ENV_SMALL_CAP)
+    k_env<CT, OT, ENV_SMALL_CAP, W, false><<<ceil_div(inum, W), W * 32, 0, st>>>(io, s, inum,
+                                                                                nullptr);
+  else if (max_nbor_size <= 512)
+    k_env<CT, OT, 512, W, false><<<ceil_div(inum, W), W * 32, 0, st>>>(io, s, inum, nullptr);
+  else if (max_nbor_size <= 1024)
     k_env<CT, OT, 1024, W, false><<<ceil_div(inum, W), W * 32, 0, st>>>(io, s, inum, nullptr);
-  } else {
+  else
     k_env<CT, OT, ENV_LARGE_CAP, 1, false><<<inum, 32, 0, st>>>(io, s, inum, nullptr);
-  }
   DPB_CHECK_LAUNCH("prod_env_mat_a");
   return DPB_OK;
 }
@@ -508,7 +529,7 @@ k_build_nlist(int* ilist, int* numneigh, int** firstneigh, int* max_size,
   // build_nlist_cpu semantics (neighbor_list.cc:875-928): j != i, both types
   // >= 0 when type is given, strict |c_i - c_j|^2 < (T)(rcut*rcut), rows in
   // ascending j.
-  __shared__ int s_c[4][NL_CAP];
+  __shared__ __align__(16) int s_c[4][NL_CAP + 4];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * 4 + w;
   if (i >= nloc) return;
@@ -566,12 +587,20 @@ k_build_nlist(int* ilist, int* numneigh, int** firstneigh, int* max_size,
   if (count > NL_CAP) atomicOr(status, ST_NLIST_CAPACITY);
   const int n = count < NL_CAP ? count : NL_CAP;
   int* out = firstneigh[row];
-  for (int q = 0; q * 32 < n; ++q) {
-    int kk = q * 32 + lane;
-    int own = kk < n ? cand[kk] : 0x7fffffff;
-    int r = 0;
-    for (int p = 0; p < n; ++p) r += cand[p] < own ? 1 : 0;
-    if (kk < n && r < mem_size) out[r] = own;
+  if (lane < 4) cand[n + lane] = 0x7fffffff;  // whole groups of four below
+  __syncwarp();
+  const int4* c4 = reinterpret_cast<const int4*>(cand);
+  for (int q = 0; q * 64 < n; ++q) {  // two candidates per lane share each read
+    const int k0 = q * 64 + lane, k1 = k0 + 32;
+    const int o0 = k0 < n ? cand[k0] : 0x7fffffff, o1 = k1 < n ? cand[k1] : 0x7fffffff;
+    int r0 = 0, r1 = 0;
+    for (int p = 0; 4 * p < n; ++p) {
+      const int4 v = c4[p];
+      r0 += (v.x < o0) + (v.y < o0) + (v.z < o0) + (v.w < o0);
+      r1 += (v.x < o1) + (v.y < o1) + (v.z < o1) + (v.w < o1);
+    }
+    if (k0 < n && r0 < mem_size) out[r0] = o0;
+    if (k1 < n && r1 < mem_size) out[r1] = o1;
   }
 }
 
