@@ -112,6 +112,7 @@ _FUNCS = {
     "dpb_se_a_descriptor_bwd_cheb_f32": "ppppp" "pppp" "pi" "iiip",
     "dpb_bt_step_set_nets": "ppppppp",
     "dpb_se_a_row_scale_f32": "pppiip",
+    "dpb_row_pointers": "ppiip",
     "dpb_force_virial_a_f32": "pppppp" "pp" "iiiip",
     "dpb_force_virial_a_f64": "pppppp" "pp" "iiiip",
     "dpb_build_nlist_noalloc_f64": "ppppp" "iiif" "i" "pp",

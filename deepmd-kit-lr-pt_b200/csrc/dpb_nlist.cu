@@ -653,10 +653,27 @@ template int build_nlist<double>(int*, int*, int**, int*, void*, long long, cons
 template int build_nlist<float>(int*, int*, int**, int*, void*, long long, const float*, int,
                                 int, int, float, int, const int*, cudaStream_t);
 
+// firstneigh of a list stored as one [n, width] array
+__global__ void k_row_pointers(int** out, int* rows, int n, int width) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = rows + (size_t)i * width;
+}
+
 }  // namespace dpb
 
 using namespace dpb;
 extern "C" {
+
+int dpb_row_pointers(int** firstneigh, int* rows, int n, int width, dpb_stream_t stream) {
+  if (n < 0 || width < 0 || (n > 0 && (firstneigh == nullptr || rows == nullptr))) {
+    set_error("row_pointers: invalid arguments (n=%d width=%d)", n, width);
+    return DPB_ERR_INVALID;
+  }
+  if (n == 0) return DPB_OK;
+  k_row_pointers<<<ceil_div(n, 256), 256, 0, as_stream(stream)>>>(firstneigh, rows, n, width);
+  DPB_CHECK_LAUNCH("row_pointers");
+  return DPB_OK;
+}
 
 long long dpb_build_nlist_scratch_bytes(int nloc, int nall) {
   (void)nloc;

@@ -31,7 +31,8 @@ _ENV_CAP = 1024
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle: building a torch.cuda.Stream for it costs ~5 us a call
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _need_cuda(*ts: torch.Tensor, what: str) -> None:
@@ -149,8 +150,8 @@ def build_nlist(c_cpy: torch.Tensor, nloc: int, rcut: float, atype: torch.Tensor
 def _row_pointers(rows: torch.Tensor) -> torch.Tensor:
     """Device array of row addresses (the firstneigh of a device InputNlist)."""
     n, w = rows.shape
-    base = rows.data_ptr()
-    addr = base + torch.arange(n, dtype=torch.int64, device=rows.device) * (w * 4)
+    addr = torch.empty(n, dtype=torch.int64, device=rows.device)
+    call("dpb_row_pointers", ptr(addr), ptr(rows), n, w, _stream())
     return addr
 
 
@@ -400,6 +401,64 @@ def _tab_grad_grad_impl(table, table_info, em_x, em, dz_dy_dem_x, dz_dy_dem, des
     return [out]
 
 
+# Autograd of the ops as two autograd functions at the Autograd dispatch key
+# (torch.library.register_autograd flattens the Tensor[] results as a tree on
+# every call, ~60 us each way).
+
+class _TabForward(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, table, table_info, em_x, em, last_layer_size):
+        with torch._C._AutoDispatchBelowAutograd():
+            out, = torch.ops.deepmd.tabulate_fusion_se_a(table, table_info, em_x, em,
+                                                         last_layer_size)
+        ctx.save_for_backward(table, table_info, em_x, em, out)
+        return out
+
+    @staticmethod
+    def backward(ctx, dy):
+        table, table_info, em_x, em, desc = ctx.saved_tensors
+        dx, de = torch.ops.deepmd.tabulate_fusion_se_a_grad(table, table_info, em_x, em,
+                                                           dy.contiguous(), desc)
+        return None, None, dx, de, None
+
+
+class _TabGrad(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, table, table_info, em_x, em, dy, desc):
+        with torch._C._AutoDispatchBelowAutograd():
+            dx, de = torch.ops.deepmd.tabulate_fusion_se_a_grad(table, table_info, em_x, em, dy,
+                                                               desc)
+        ctx.save_for_backward(table, table_info, em_x, em, desc)
+        return dx, de
+
+    @staticmethod
+    def backward(ctx, gx, ge):
+        table, table_info, em_x, em, desc = ctx.saved_tensors
+        dz, = torch.ops.deepmd.tabulate_fusion_se_a_grad_grad(
+            table, table_info, em_x, em, gx.contiguous(), ge.contiguous(), desc, True)
+        return None, None, None, None, dz, None
+
+
+def _needs_grad(*ts) -> bool:
+    return torch.is_grad_enabled() and any(t.requires_grad for t in ts)
+
+
+def _tab_fwd_autograd(table, table_info, em_x, em, last_layer_size):
+    if _needs_grad(table, table_info, em_x, em):
+        return [_TabForward.apply(table, table_info, em_x, em, last_layer_size)]
+    with torch._C._AutoDispatchBelowAutograd():
+        return torch.ops.deepmd.tabulate_fusion_se_a(table, table_info, em_x, em,
+                                                     last_layer_size)
+
+
+def _tab_grad_autograd(table, table_info, em_x, em, dy, descriptor):
+    if _needs_grad(table, table_info, em_x, em, dy, descriptor):
+        return list(_TabGrad.apply(table, table_info, em_x, em, dy, descriptor))
+    with torch._C._AutoDispatchBelowAutograd():
+        return torch.ops.deepmd.tabulate_fusion_se_a_grad(table, table_info, em_x, em, dy,
+                                                          descriptor)
+
+
 _LIB = None
 
 
@@ -432,33 +491,8 @@ def register_torch_ops() -> None:
 
     # autograd: forward -> grad (tabulate_multi_device.cc:961-995),
     # grad -> grad_grad w.r.t. dy only (:818-863)
-    def fwd_setup(ctx, inputs, output):
-        table, table_info, em_x, em, _ = inputs
-        ctx.save_for_backward(table, table_info, em_x, em, output[0])
-
-    def fwd_backward(ctx, grads):
-        table, table_info, em_x, em, desc = ctx.saved_tensors
-        dy = grads[0].contiguous()
-        dx, de = torch.ops.deepmd.tabulate_fusion_se_a_grad(table, table_info, em_x, em, dy,
-                                                           desc)
-        return None, None, dx, de, None
-
-    def grad_setup(ctx, inputs, output):
-        table, table_info, em_x, em, dy, desc = inputs
-        ctx.save_for_backward(table, table_info, em_x, em, desc)
-
-    def grad_backward(ctx, grads):
-        table, table_info, em_x, em, desc = ctx.saved_tensors
-        gx = grads[0] if grads[0] is not None else torch.zeros_like(em_x)
-        ge = grads[1] if grads[1] is not None else torch.zeros_like(em)
-        dz = torch.ops.deepmd.tabulate_fusion_se_a_grad_grad(
-            table, table_info, em_x, em, gx.contiguous(), ge.contiguous(), desc, True)[0]
-        return None, None, None, None, dz, None
-
-    torch.library.register_autograd("deepmd::tabulate_fusion_se_a", fwd_backward,
-                                    setup_context=fwd_setup, lib=lib)
-    torch.library.register_autograd("deepmd::tabulate_fusion_se_a_grad", grad_backward,
-                                    setup_context=grad_setup, lib=lib)
+    lib.impl("tabulate_fusion_se_a", _tab_fwd_autograd, "Autograd")
+    lib.impl("tabulate_fusion_se_a_grad", _tab_grad_autograd, "Autograd")
     _LIB = lib
 
 

@@ -121,6 +121,9 @@ DPB_API int dpb_build_nlist_f32(int* ilist, int* numneigh, int** firstneigh,
                                 int nloc, int nall, int mem_size, float rcut,
                                 int nframes, const int* type,
                                 dpb_stream_t stream);
+/* firstneigh[i] = rows + i * width: the row pointers of a list kept as one
+ * [n, width] device array. */
+DPB_API int dpb_row_pointers(int** firstneigh, int* rows, int n, int width, dpb_stream_t stream);
 
 /* ----------------------------------------------------- environment matrix -- */
 
