@@ -1940,6 +1940,8 @@ using namespace dpb;
     rc = tr_xbar<T>(xb, xbd, xyz, xyz_t, d_descrpt, d_descrpt_t, drow, nrows, net.n3, axis,     \
                     g.nnei, st);                                                                \
     if (rc) return rc;                                                                          \
+    rc = em_try_rev<T>(gr, xb, xbd, avg, std_, force_bar, virial_bar, net, g, st);              \
+    if (rc >= 0) return rc;                                                                     \
     auto kern = !tr_std_net(net) ? k_tr_rev<T, TrTraits<T>::R, 0, 0, 0>                         \
                 : (R == 4 ? k_tr_rev<T, 4, 25, 50, 100> : k_tr_rev<T, 8, 25, 50, 100>);\
     int grid;                                                                                   \

@@ -1,7 +1,8 @@
 // The FP64 embedding passes of the standard net (1 -> 25 -> 50 -> 100) on the
-// FP64 matrix instructions: forward (G, xyz, D) and force backward
-// (dE/d(em)), the same quantities as k_tr_fwd / k_tr_bwd (dpb_train.cu, which
-// includes this file).
+// FP64 matrix instructions: forward (G, xyz, D), force backward (dE/d(em)) and
+// the reverse pass over primal and tangent (weight gradients), the same
+// quantities as k_tr_fwd / k_tr_bwd / k_tr_rev (dpb_train.cu, which includes
+// this file).
 //
 // One warp takes one center atom and 16 neighbor rows at a time through the
 // whole net as mma.m16n8k4 products. The FMA form held one channel per lane
@@ -94,6 +95,30 @@ __device__ __forceinline__ int em_c2(int j, int u, int v) {
   return 4 * j + u < 25 ? 4 * j + u + 25 * v : -1;
 }
 
+// layer 2 and its adjoint in fragment order, W1 and b1 padded to 28
+__device__ inline void em_stage_f2(double* F2, const double* W2) {
+  for (int e = threadIdx.x; e < EM_F2; e += blockDim.x) {
+    const int lane = e & 31, j = (e >> 5) % 7, s = (e >> 5) / 7, g = lane >> 2;
+    const int k = 4 * s + (lane & 3), c = em_c2(j, g >> 1, g & 1);
+    F2[e] = k < 25 && c >= 0 ? W2[k * 50 + c] : 0.;
+  }
+}
+__device__ inline void em_stage_b2(double* B2, const double* W2) {
+  for (int e = threadIdx.x; e < EM_B2; e += blockDim.x) {
+    const int lane = e & 31, q = (e >> 5) & 3, step = (e >> 5) >> 2, g = lane >> 2;
+    const int c = em_c2(step >> 1, lane & 3, step & 1);
+    const int k = 4 * (2 * q + (g & 1)) + (g >> 1);
+    B2[e] = c >= 0 && k < 25 ? W2[k * 50 + c] : 0.;
+  }
+}
+__device__ inline void em_stage_v(double* V, const TrNet<double>& net, int t) {
+  for (int e = threadIdx.x; e < 28; e += blockDim.x) {
+    V[e] = e < 25 ? net.W[t][0][e] : 0.;
+    V[28 + e] = e < 25 ? net.b[t][0][e] : 0.;
+  }
+  for (int e = threadIdx.x; e < 50; e += blockDim.x) V[56 + e] = net.b[t][1][e];
+}
+
 // weights of net t into fragment order
 __device__ inline void em_stage(double* w, const TrNet<double>& net, int t, bool bwd) {
   double* F2 = w;
@@ -101,11 +126,7 @@ __device__ inline void em_stage(double* w, const TrNet<double>& net, int t, bool
   double* V = F3 + EM_F3 + (bwd ? EM_B3 + EM_B2 : 0);
   const double *W2 = net.W[t][1], *W3 = net.W[t][2];
   const int n = blockDim.x;
-  for (int e = threadIdx.x; e < EM_F2; e += n) {
-    const int lane = e & 31, j = (e >> 5) % 7, s = (e >> 5) / 7, g = lane >> 2;
-    const int k = 4 * s + (lane & 3), c = em_c2(j, g >> 1, g & 1);
-    F2[e] = k < 25 && c >= 0 ? W2[k * 50 + c] : 0.;
-  }
+  em_stage_f2(F2, W2);
   for (int e = threadIdx.x; e < EM_F3; e += n) {
     // tiles 0..5: [tile][step][lane][row g, row g + 8]; tile 6: [step][lane]
     const bool last = e >= 6 * 14 * 64;
@@ -116,26 +137,16 @@ __device__ inline void em_stage(double* w, const TrNet<double>& net, int t, bool
     const int c = em_c2(step >> 1, lane & 3, step & 1);
     F3[e] = m < 100 && c >= 0 ? W3[c * 100 + m] : 0.;
   }
-  for (int e = threadIdx.x; e < 28; e += n) {
-    V[e] = e < 25 ? net.W[t][0][e] : 0.;
-    V[28 + e] = e < 25 ? net.b[t][0][e] : 0.;
-  }
-  for (int e = threadIdx.x; e < 50; e += n) V[56 + e] = net.b[t][1][e];
+  em_stage_v(V, net, t);
   for (int e = threadIdx.x; e < 100; e += n) V[108 + e] = net.b[t][2][e];
   if (!bwd) return;
   double* B3 = F3 + EM_F3;
-  double* B2 = B3 + EM_B3;
   for (int e = threadIdx.x; e < EM_B3; e += n) {
     const int lane = e & 31, j = (e >> 5) % 7, s = (e >> 5) / 7, g = lane >> 2;
     const int c = em_c2(j, g >> 1, g & 1);
     B3[e] = c >= 0 ? W3[c * 100 + 4 * s + (lane & 3)] : 0.;
   }
-  for (int e = threadIdx.x; e < EM_B2; e += n) {
-    const int lane = e & 31, q = (e >> 5) & 3, step = (e >> 5) >> 2, g = lane >> 2;
-    const int c = em_c2(step >> 1, lane & 3, step & 1);
-    const int k = 4 * (2 * q + (g & 1)) + (g >> 1);
-    B2[e] = c >= 0 && k < 25 ? W2[k * 50 + c] : 0.;
-  }
+  em_stage_b2(B3 + EM_B3, W2);
 }
 
 // layers 1 and 2 of 16 rows: h1a / h1b the layer-1 outputs of rows g / g + 8 at
@@ -504,6 +515,428 @@ k_emb_bwd_dmma(double* __restrict__ gem, const double* __restrict__ em,
   }
 }
 
+// ------------------------------------------------- reverse over tangent --
+// The weight gradients of J = sum Ebar E + <u, g> (k_tr_rev's) on the FP64
+// matrix instructions. The FMA form adds every row group's share of the 6,250
+// weight gradients to shared memory: the atomics and the operand reads around
+// them held it at a seventh of the FP64 rate. Here the eight warps of a CTA
+// take one 16-row tile each, of any atoms, and go through the net in step: layer
+// 3 one 16-channel tile at a time, whose adjoints of all 128 rows meet in
+// shared memory, and warp w adds their product with the rows' layer-2 outputs
+// and tangents for 8 of the 50 units to registers that it keeps to the end.
+//
+// Shared memory holds one net (so a CTA stays with one neighbor type): W3
+// once, rows of 100 with the second pair members 26 rows down, which makes the
+// reads as layer-3 and as adjoint operand free of bank conflicts; row 25 is b3
+// and meets the constant 1 at position 50 of the layer-2 outputs, which also
+// collects the gradient of b3. Position 2 (c % 25) + c / 25 holds unit c.
+//
+// Tiles are numbered tile-in-atom first, so the empty ones (beyond an atom's
+// neighbors) are the last and the rest come out even over the warps.
+//
+// Measured, 4 frames of 192 atoms: 1666 -> 461 us (FP64 matrix pipe 44 % busy, the
+// FMA pipe 10 %; the eight warps' waits for each other and for operands are the rest).
+constexpr int EM_REV_NW = 8;
+constexpr int EM_REV_W3 = 54 * 100 + 4;
+constexpr int EM_REV_V = 28 + 28 + 52;
+constexpr int EM_P2S = 52;                     // row stride of staged layer-2 vectors
+constexpr int EM_P1S = 28;                     // of layer-1 vectors
+constexpr int EM_REV_H = 2 * 16 * EM_P2S;      // per warp: outputs, tangents
+constexpr int EM_REV_Z = 2 * 16 * EM_TS;       // layer-3 adjoints of a channel tile
+constexpr int EM_REV_R = 16 * 8;               // env rows and their tangents
+constexpr int EM_REV_N = EM_REV_W3 + EM_F2 + EM_B2 + EM_REV_V +
+                         EM_REV_NW * (EM_REV_H + EM_REV_Z + EM_REV_R + 56) + 4;
+
+__global__ void __launch_bounds__(32 * EM_REV_NW, 1)
+k_emb_rev_dmma(TrGrad<double> grad, const double* __restrict__ xbar,
+               const double* __restrict__ xbard, const double* __restrict__ avg,
+               const double* __restrict__ std_, const double* __restrict__ fbar,
+               const double* __restrict__ vbar, TrNet<double> net, TrGeom g, EmSplit split) {
+  extern __shared__ __align__(16) double esm[];
+  pdl_wait();
+  pdl_trigger();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int gr = lane >> 2, t4 = lane & 3;
+  int t = 0;
+  while (t + 1 < g.ntypes && (int)blockIdx.x >= split.first[t + 1]) ++t;
+  double* W3 = esm;
+  double* F2 = W3 + EM_REV_W3;
+  double* B2 = F2 + EM_F2;
+  double* V = B2 + EM_B2;
+  double* H = V + EM_REV_V;
+  double* Z = H + EM_REV_NW * EM_REV_H;
+  double* R = Z + EM_REV_NW * EM_REV_Z;
+  double* G1 = R + EM_REV_NW * EM_REV_R;
+  int* act = reinterpret_cast<int*>(G1 + EM_REV_NW * 56);
+  for (int e = threadIdx.x; e < EM_REV_W3; e += blockDim.x) {
+    const int r = e / 100, c = e - r * 100;
+    W3[e] = r < 25 ? net.W[t][2][e]
+            : r == 25 ? net.b[t][2][c]
+            : r < 51 ? net.W[t][2][(r - 1) * 100 + c] : 0.;
+  }
+  em_stage_f2(F2, net.W[t][1]);
+  em_stage_b2(B2, net.W[t][1]);
+  em_stage_v(V, net, t);
+  for (int e = threadIdx.x; e < EM_REV_NW * 56; e += blockDim.x) G1[e] = 0.;
+  double* hs = H + w * EM_REV_H;
+  double* hd = hs + 16 * EM_P2S;
+  double* zs = Z + w * EM_REV_Z;
+  double* zd = zs + 16 * EM_TS;
+  double* rr = R + w * EM_REV_R;
+  double* g1 = G1 + w * 56;
+  int* ent = reinterpret_cast<int*>(zs);  // read before the first adjoints are written
+  int* secn = ent + g.nnei;
+  double gw3[7][4], gw2[2][4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    gw2[0][k] = gw2[1][k] = 0.;
+#pragma unroll
+    for (int m = 0; m < 7; ++m) gw3[m][k] = 0.;
+  }
+  const int nb = split.first[t + 1] - split.first[t];
+  const long long ntile = (long long)g.nrows * ((g.sec[t + 1] - g.sec[t] + 15) / 16);
+  long long idx = (long long)w * nb + (blockIdx.x - split.first[t]);
+  bool any = false;
+  for (;;) {
+    __syncthreads();  // the previous round's last products have read Z
+    int ne = 0, e0 = 0, row = 0;
+    while (idx < ntile) {
+      row = (int)(idx % g.nrows);
+      e0 = 16 * (int)(idx / g.nrows);
+      idx += (long long)nb * EM_REV_NW;
+      tr_entries(ent, secn, g.nlist + (size_t)row * g.nnei, g, g.type[row], true, lane, t, t + 1);
+      ne = max(0, min(16, secn[t + 1] - e0));
+      if (ne > 0) break;
+      __syncwarp();
+    }
+    if (lane == 0) act[w] = ne > 0;
+    if (!__syncthreads_or(ne > 0)) break;
+    any = true;
+    const double* xb = xbar + (size_t)row * 400;
+    const double* xd = xbard + (size_t)row * 400;
+    double x0 = 0., x1 = 0., d0 = 0., d1 = 0.;  // input and tangent of rows g, g + 8
+    double hb2[7][4], hbd2[7][4];               // adjoints of layer 2's output and tangent
+    auto layer1 = [&](double (&ha)[EM_S1], double (&hb)[EM_S1]) {
+#pragma unroll
+      for (int s = 0; s < EM_S1; ++s) {
+        const double w1 = V[4 * s + t4], b1 = V[28 + 4 * s + t4];
+        ha[s] = tanh_f64(fma(x0, w1, b1));
+        hb[s] = tanh_f64(fma(x1, w1, b1));
+      }
+    };
+    if (ne > 0) {
+      double x = 0., d = 0.;
+      if (lane < 16) {
+        double Rv[4] = {0., 0., 0., 0.}, Rd[4] = {0., 0., 0., 0.}, mu = 0.;
+        if (lane < ne) {
+          const TrAtom A = tr_atom(g, row);
+          const int en = ent[e0 + lane];
+          tr_env_tangent<double>(Rv, Rd, g, A, en & 0xFFFF, avg + (size_t)A.ti * g.nnei * 4,
+                                 std_ + (size_t)A.ti * g.nnei * 4, fbar, vbar);
+          mu = (double)(en >> 16);
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          rr[lane * 8 + a] = mu * Rv[a];
+          rr[lane * 8 + 4 + a] = mu * Rd[a];
+        }
+        x = Rv[0];
+        d = Rd[0];
+      }
+      x0 = __shfl_sync(0xffffffffu, x, gr);
+      x1 = __shfl_sync(0xffffffffu, x, 8 + gr);
+      d0 = __shfl_sync(0xffffffffu, d, gr);
+      d1 = __shfl_sync(0xffffffffu, d, 8 + gr);
+      __syncwarp();
+      // layers 1 and 2, outputs and tangents staged at their positions
+      double h1a[EM_S1], h1b[EM_S1], h2[7][4], ht[7][4];
+      layer1(h1a, h1b);
+#pragma unroll
+      for (int j = 0; j < 7; ++j) {
+        const bool ok = 4 * j + t4 < 25;
+        h2[j][0] = h2[j][2] = ok ? V[56 + 4 * j + t4] : 0.;
+        h2[j][1] = h2[j][3] = ok ? V[56 + 4 * j + t4 + 25] : 0.;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ht[j][k] = 0.;
+      }
+#pragma unroll
+      for (int s = 0; s < EM_S1; ++s) {
+        const double w1 = V[4 * s + t4];
+        const double ta = (1. - h1a[s] * h1a[s]) * (d0 * w1);
+        const double tb = (1. - h1b[s] * h1b[s]) * (d1 * w1);
+#pragma unroll
+        for (int j = 0; j < 7; ++j) {
+          const double b = F2[(s * 7 + j) * 32 + lane];
+          dmma16(h2[j], h1a[s], h1b[s], b);
+          dmma16(ht[j], ta, tb, b);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 7; ++j) {
+        const double w1 = V[4 * j + t4];
+        const double ta = (1. - h1a[j] * h1a[j]) * (d0 * w1);
+        const double tb = (1. - h1b[j] * h1b[j]) * (d1 * w1);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const double y = tanh_f64(h2[j][k]);
+          h2[j][k] = y + (k < 2 ? h1a[j] : h1b[j]);
+          ht[j][k] = (1. - y * y) * ht[j][k] + (k < 2 ? ta : tb);
+        }
+        if (j == 6 && t4 == 1) {  // positions 50 (the constant), 51
+          h2[j][0] = h2[j][2] = 1.;
+          h2[j][1] = h2[j][3] = 0.;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) ht[j][k] = 0.;
+        }
+        if (j < 6 || t4 < 2) {
+          const int o = gr * EM_P2S + 8 * j + 2 * t4;
+          *reinterpret_cast<double2*>(hs + o) = make_double2(h2[j][0], h2[j][1]);
+          *reinterpret_cast<double2*>(hs + o + 8 * EM_P2S) = make_double2(h2[j][2], h2[j][3]);
+          *reinterpret_cast<double2*>(hd + o) = make_double2(ht[j][0], ht[j][1]);
+          *reinterpret_cast<double2*>(hd + o + 8 * EM_P2S) = make_double2(ht[j][2], ht[j][3]);
+        }
+      }
+      // the layer-3 residual's share of the layer-2 adjoints
+      const double ra = rr[gr * 8 + t4], rb = rr[(gr + 8) * 8 + t4];
+      const double qa = rr[gr * 8 + 4 + t4], qb = rr[(gr + 8) * 8 + 4 + t4];
+#pragma unroll
+      for (int j = 0; j < 7; ++j) {
+        const int c = em_c2(j, gr >> 1, gr & 1), o = t4 * 100 + (c < 0 ? 0 : c);
+        const double u = c < 0 ? 0. : xb[o] + xb[o + 50], v = c < 0 ? 0. : xd[o] + xd[o + 50];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) hb2[j][k] = hbd2[j][k] = 0.;
+        dmma16(hb2[j], ra, rb, u);
+        dmma16(hb2[j], qa, qb, v);
+        dmma16(hbd2[j], ra, rb, v);
+      }
+      __syncwarp();
+    }
+    auto tile = [&](auto last, int m) {
+      constexpr int LAST = decltype(last)::value;
+      if (ne > 0) {
+        const int c = 16 * m + gr;
+        const bool in = !LAST || gr < 4;
+        const int o = t4 * 100 + c;
+        const double xb0 = in ? xb[o] : 0., xb1 = LAST ? 0. : xb[o + 8];
+        const double xd0 = in ? xd[o] : 0., xd1 = LAST ? 0. : xd[o + 8];
+#pragma unroll 1
+        for (int n = 0; n < 2; ++n) {
+          double z[4] = {0., 0., 0., 0.}, zt[4] = {0., 0., 0., 0.};
+          const double* hr = hs + (8 * n + gr) * EM_P2S + 2 * t4;
+#pragma unroll
+          for (int j = 0; j < 7; ++j) {
+            double2 h = *reinterpret_cast<const double2*>(hr + 8 * j);
+            double2 q = *reinterpret_cast<const double2*>(hr + 16 * EM_P2S + 8 * j);
+            if (j == 6) {  // positions past 50: the next row's
+              h.x = t4 < 2 ? h.x : 0.;
+              q.x = t4 < 2 ? q.x : 0.;
+              h.y = t4 < 1 ? h.y : 0.;
+              q.y = t4 < 1 ? q.y : 0.;
+            }
+            const double* a = W3 + (4 * j + t4) * 100 + c;
+            const double* b = a + 2600;
+            if (LAST) {
+              dmma8(z[0], z[1], a[0], h.x);
+              dmma8(zt[0], zt[1], a[0], q.x);
+              dmma8(z[0], z[1], b[0], h.y);
+              dmma8(zt[0], zt[1], b[0], q.y);
+            } else {
+              const double a0 = a[0], a1 = a[8], b0 = b[0], b1 = b[8];
+              dmma16(z, a0, a1, h.x);
+              dmma16(zt, a0, a1, q.x);
+              dmma16(z, b0, b1, h.y);
+              dmma16(zt, b0, b1, q.y);
+            }
+          }
+          double gb[4] = {0., 0., 0., 0.}, gd[4] = {0., 0., 0., 0.};
+          const double rv = rr[(8 * n + gr) * 8 + t4], rd = rr[(8 * n + gr) * 8 + 4 + t4];
+          if (LAST) {
+            dmma8(gb[0], gb[1], xb0, rv);
+            dmma8(gb[0], gb[1], xd0, rd);
+            dmma8(gd[0], gd[1], xd0, rv);
+          } else {
+            dmma16(gb, xb0, xb1, rv);
+            dmma16(gb, xd0, xd1, rd);
+            dmma16(gd, xd0, xd1, rv);
+          }
+#pragma unroll
+          for (int k = 0; k < (LAST ? 2 : 4); ++k)
+            if (in) {
+              const double y = tanh_f64(z[k]), q = 1. - y * y;
+              const int p = (8 * n + 2 * t4 + (k & 1)) * EM_TS + gr + 8 * (k >> 1);
+              zs[p] = (gb[k] - 2. * y * zt[k] * gd[k]) * q;
+              zd[p] = gd[k] * q;
+            }
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int s = 0; s < (LAST ? 1 : 4); ++s) {
+          const int k = 4 * s + t4;
+          const double a0 = zs[gr * EM_TS + k], a1 = zs[(gr + 8) * EM_TS + k];
+          const double e0_ = zd[gr * EM_TS + k], e1_ = zd[(gr + 8) * EM_TS + k];
+          const double* bp = W3 + ((gr >> 1) + 26 * (gr & 1)) * 100 + 16 * m + k;
+#pragma unroll
+          for (int j = 0; j < 7; ++j) {
+            const double b = bp[400 * j];
+            dmma16(hb2[j], a0, a1, b);
+            dmma16(hbd2[j], e0_, e1_, b);
+          }
+        }
+      }
+      __syncthreads();
+      // W3 gradient of this tile's channels, units at positions 8 w ..
+      if (w < 7) {
+        double c[2][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) c[0][k] = c[1][k] = 0.;
+#pragma unroll 1
+        for (int v = 0; v < EM_REV_NW; ++v) {
+          if (!act[v]) continue;
+          const double* zp = Z + v * EM_REV_Z + t4 * EM_TS + gr;
+          const double* hp = H + v * EM_REV_H + t4 * EM_P2S + 8 * w + gr;
+#pragma unroll
+          for (int s = 0; s < 8; ++s) {  // four steps of outputs, four of tangents
+            const double* zq = zp + 4 * s * EM_TS;
+            const double b = hp[4 * s * EM_P2S];
+            if (LAST)
+              dmma8(c[s & 1][0], c[s & 1][1], zq[0], b);
+            else
+              dmma16(c[s & 1], zq[0], zq[8], b);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 7; ++q)
+          if (q == m)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) gw3[q][k] += c[0][k] + c[1][k];
+      }
+      __syncthreads();
+    };
+#pragma unroll 1
+    for (int m = 0; m < 6; ++m) tile(std::integral_constant<int, 0>{}, m);
+    tile(std::integral_constant<int, 1>{}, 6);
+    // layer 2's pre-activation adjoints take the place of its outputs and tangents
+    double h1a[EM_S1], h1b[EM_S1];
+    if (ne > 0) {
+      layer1(h1a, h1b);
+      double u[4][4], v[4][4];  // layer 1's: channel 4 s + t of row g at [s / 2][s % 2]
+#pragma unroll
+      for (int j = 0; j < 7; ++j) {
+        u[j >> 1][j & 1] = hb2[j][0] + hb2[j][1];
+        u[j >> 1][2 + (j & 1)] = hb2[j][2] + hb2[j][3];
+        v[j >> 1][j & 1] = hbd2[j][0] + hbd2[j][1];
+        v[j >> 1][2 + (j & 1)] = hbd2[j][2] + hbd2[j][3];
+        if (j == 6 && t4 > 0) continue;
+        const double w1 = V[4 * j + t4];
+        double* ho = hs + gr * EM_P2S + 8 * j + 2 * t4;
+        double* po = hd + gr * EM_P2S + 8 * j + 2 * t4;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int o = (k >> 1) * 8 * EM_P2S + (k & 1);
+          const double h = k < 2 ? h1a[j] : h1b[j];
+          const double y = ho[o] - h, q = 1. - y * y;
+          const double yt = po[o] - (1. - h * h) * ((k < 2 ? d0 : d1) * w1);  // q times zdot
+          ho[o] = hb2[j][k] * q - 2. * y * yt * hbd2[j][k];
+          po[o] = hbd2[j][k] * q;
+        }
+      }
+      u[3][1] = u[3][3] = v[3][1] = v[3][3] = 0.;
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 7; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int o = gr * EM_P2S + 8 * j + 2 * t4 + e;
+          const bool ok = j < 6 || t4 == 0;
+          const double a0 = ok ? hs[o] : 0., a1 = ok ? hs[o + 8 * EM_P2S] : 0.;
+          const double b0 = ok ? hd[o] : 0., b1 = ok ? hd[o + 8 * EM_P2S] : 0.;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const double b = B2[((2 * j + e) * 4 + q) * 32 + lane];
+            dmma16(u[q], a0, a1, b);
+            dmma16(v[q], b0, b1, b);
+          }
+        }
+#pragma unroll
+      for (int s = 0; s < EM_S1; ++s) {
+        const double w1 = V[4 * s + t4];
+        const double qa = 1. - h1a[s] * h1a[s], qb = 1. - h1b[s] * h1b[s];
+        const double ta = v[s >> 1][s & 1], tb = v[s >> 1][2 + (s & 1)];
+        const double za = (u[s >> 1][s & 1] - 2. * h1a[s] * (d0 * w1) * ta) * qa;
+        const double zb = (u[s >> 1][2 + (s & 1)] - 2. * h1b[s] * (d1 * w1) * tb) * qb;
+        double gws = fma(x0, za, fma(d0, ta * qa, fma(x1, zb, d1 * (tb * qb)))), gbs = za + zb;
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) {
+          gws += __shfl_xor_sync(0xffffffffu, gws, o);
+          gbs += __shfl_xor_sync(0xffffffffu, gbs, o);
+        }
+        if (gr == 0) {
+          g1[4 * s + t4] += gws;
+          g1[28 + 4 * s + t4] += gbs;
+        }
+      }
+    }
+    // W2 gradient: positions 16 (w / 2) .. of layer 2, channels 16 (w % 2) .. of
+    // layer 1, whose outputs (and the constant 1 as channel 25, for b2), then
+    // tangents, take the place of Z
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+      if (half) __syncthreads();
+      if (ne > 0) {
+        double* p = Z + (w * 16 + gr) * EM_P1S + t4;
+#pragma unroll
+        for (int s = 0; s < EM_S1; ++s) {
+          const bool one = s == 6 && t4 == 1;
+          const double w1 = V[4 * s + t4];
+          p[4 * s] = half ? (1. - h1a[s] * h1a[s]) * (d0 * w1) : one ? 1. : h1a[s];
+          p[8 * EM_P1S + 4 * s] = half ? (1. - h1b[s] * h1b[s]) * (d1 * w1) : one ? 1. : h1b[s];
+        }
+      }
+      __syncthreads();
+#pragma unroll 1
+      for (int v = 0; v < EM_REV_NW; ++v) {
+        if (!act[v]) continue;
+        const double* ap = H + v * EM_REV_H + half * 16 * EM_P2S + t4 * EM_P2S + 16 * (w >> 1) + gr;
+        const double* bp = Z + (v * 16 + t4) * EM_P1S + 16 * (w & 1) + gr;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const double a0 = ap[4 * s * EM_P2S], a1 = ap[4 * s * EM_P2S + 8];
+          dmma16(gw2[0], a0, a1, bp[4 * s * EM_P1S]);
+          dmma16(gw2[1], a0, a1, bp[4 * s * EM_P1S + 8]);
+        }
+      }
+    }
+  }
+  if (!any) return;
+  if (w < 7)
+#pragma unroll
+    for (int m = 0; m < 7; ++m)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int c = 16 * m + gr + 8 * (k >> 1), p = 8 * w + 2 * t4 + (k & 1);
+        if (c >= 100 || p > 50) continue;
+        atomicAdd(p == 50 ? grad.b[t][2] + c : grad.W[t][2] + ((p >> 1) + 25 * (p & 1)) * 100 + c,
+                  gw3[m][k]);
+      }
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int p = 16 * (w >> 1) + gr + 8 * (k >> 1);
+      const int i = 16 * (w & 1) + 8 * n + 2 * t4 + (k & 1);
+      if (p >= 50 || i > 25) continue;
+      const int c = (p >> 1) + 25 * (p & 1);
+      atomicAdd(i == 25 ? grad.b[t][1] + c : grad.W[t][1] + i * 50 + c, gw2[n][k]);
+    }
+  for (int e = threadIdx.x; e < 56; e += blockDim.x) {
+    const int i = e % 28;
+    if (i >= 25) continue;
+    double s = 0.;
+    for (int v = 0; v < EM_REV_NW; ++v) s += G1[v * 56 + e];
+    atomicAdd((e < 28 ? grad.W[t][0] : grad.b[t][0]) + i, s);
+  }
+}
+
 // most warps per CTA whose rows come out even: the smallest
 // ceil(rows / (blocks * n)) * n, within shared memory
 static int em_warps(int rows, int blocks, int maxw, size_t base, size_t per_warp) {
@@ -542,12 +975,11 @@ static int em_fwd(double* xyz, double* D, const double* em, const TrNet<double>&
   return DPB_OK;
 }
 
-static int em_bwd(double* gem, const double* em, const double* xbar, const TrNet<double>& net,
-                  const TrGeom& g, cudaStream_t st) {
-  // CTAs per type in proportion to its slots
+// CTAs per type in proportion to its slots
+static EmSplit em_split(const TrGeom& g, int& sms, int& used) {
   EmSplit sp{};
-  const int sms = std::max(sm_count(), g.ntypes);
-  int used = 0;
+  sms = std::max(sm_count(), g.ntypes);
+  used = 0;
   for (int t = 0; t < g.ntypes; ++t) {
     sp.first[t] = used;
     const int left = g.ntypes - 1 - t;
@@ -556,6 +988,13 @@ static int em_bwd(double* gem, const double* em, const double* xbar, const TrNet
     used += n;
   }
   sp.first[g.ntypes] = used;
+  return sp;
+}
+
+static int em_bwd(double* gem, const double* em, const double* xbar, const TrNet<double>& net,
+                  const TrGeom& g, cudaStream_t st) {
+  int sms, used;
+  const EmSplit sp = em_split(g, sms, used);
   const size_t base = (size_t)EM_BWD_T * 8;
   const size_t per = EM_BWD_W * 8 + (size_t)(g.nnei + TR_MAXT + 1) * 4;
   const int nw = em_warps(g.nrows, std::max(1, sms / g.ntypes), EM_BWD_MAXW, base, per);
@@ -567,6 +1006,21 @@ static int em_bwd(double* gem, const double* em, const double* xbar, const TrNet
   DPB_CUDA(launch_pdl(k_emb_bwd_dmma, dim3(used), dim3(32 * nw), smem, st, gem, em, xbar, net, g,
                       sp),
            "se_a_train_bwd");
+  return DPB_OK;
+}
+
+static int em_rev(const TrGrad<double>& gr, const double* xb, const double* xbd, const double* avg,
+                  const double* std_, const double* fbar, const double* vbar,
+                  const TrNet<double>& net, const TrGeom& g, cudaStream_t st) {
+  int sms, used;
+  const EmSplit sp = em_split(g, sms, used);
+  const size_t smem = (size_t)EM_REV_N * 8;
+  DPB_CUDA(cudaFuncSetAttribute(k_emb_rev_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)smem),
+           "se_a_train_rev");
+  DPB_CUDA(launch_pdl(k_emb_rev_dmma, dim3(used), dim3(32 * EM_REV_NW), smem, st, gr, xb, xbd, avg,
+                      std_, fbar, vbar, net, g, sp),
+           "se_a_train_rev");
   return DPB_OK;
 }
 
@@ -583,6 +1037,19 @@ static int em_try_bwd(T* gem, const T* em, const T* xbar, const TrNet<T>& net, c
                       cudaStream_t st) {
   if constexpr (std::is_same_v<T, double>)
     if (em_takes(net, g, em, gem)) return em_bwd(gem, em, xbar, net, g, st);
+  return -1;
+}
+
+// the reverse pass keeps one net per CTA, so any number of types; the entry list
+// of an atom has to fit where the adjoints of a tile go later
+template <typename T>
+static int em_try_rev(const TrGrad<T>& gr, const T* xb, const T* xbd, const T* avg, const T* std_,
+                      const double* fbar, const double* vbar, const TrNet<T>& net, const TrGeom& g,
+                      cudaStream_t st) {
+  if constexpr (std::is_same_v<T, double>)
+    if (net.n1 == 25 && net.n2 == 50 && net.n3 == 100 &&
+        g.nnei + TR_MAXT + 1 <= EM_REV_Z * 2)
+      return em_rev(gr, xb, xbd, avg, std_, fbar, vbar, net, g, st);
   return -1;
 }
 

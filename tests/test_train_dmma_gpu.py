@@ -73,3 +73,99 @@ def test_embedding_passes_match_autograd(dpb, n, sel, ax):
             got, want = got.detach(), want.detach()
             assert float((got - want).abs().max()) <= 1e-12 * max(1.0, float(want.abs().max()))
     assert bool((out[2][~real] == 0).all())
+
+
+def _env(r, rmin, rmax):
+    """env rows (s, s x / d, ...) of displacements r, s = sw(d) / d"""
+    d = r.norm(dim=-1, keepdim=True)
+    u = ((d - rmin) / (rmax - rmin)).clamp(0, 1)
+    s = (u ** 3 * (-6 * u ** 2 + 15 * u - 10) + 1) / d
+    return torch.cat([s, s * r / d], -1)
+
+
+@pytest.mark.parametrize("n,sel,ax", [(1, (5,), 16), (2, (16, 17), 4), (9, (33, 1, 48), 16),
+                                      (260, (20, 40), 16), (6, (15, 32, 3, 9), 8)])
+def test_embedding_tangent_and_weight_gradients_match_autograd(dpb, n, sel, ax):
+    """xyz' and D' along a displacement field, and the gradient of
+    <dD, D> + <dDt, D'> by every embedding weight: 1e-12 of the largest for the
+    tangents (100 x sum(sel) products), 1e-11 for the gradients, whose sums run
+    over the atoms as well and cancel."""
+    cap = dpb._capi
+    wl = importlib.import_module("deepmd_kit_lr_pt_b200.workload")
+    cfg = wl.SeAConfig(sel=sel, axis_neuron=ax)
+    p = wl.init_params(cfg, seed=n)
+    nt, nn, M = len(sel), sum(sel), 100
+    rmin, rmax = 1.5, 4.0
+    rng = np.random.default_rng(n)
+    grid = np.stack(np.meshgrid(*[np.arange(7)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    dev = lambda a: torch.tensor(np.asarray(a), device="cuda")  # noqa: E731
+    vp = lambda xs: (ctypes.c_void_p * len(xs))(*[x.data_ptr() for x in xs])  # noqa: E731
+    x = dev(1.1 * grid + rng.uniform(-0.2, 0.2, (n, 3)))
+    fbar, vbar = dev(rng.normal(0, 1, (n, 3))), dev(rng.normal(0, 0.3, (1, 3, 3)))
+    ty = np.sort(rng.integers(0, nt, n)).astype(np.int32)
+    avg, std = dev(rng.normal(0, .1, (nt, nn, 4))), dev(rng.uniform(.5, 1.5, (nt, nn, 4)))
+    # one mean and deviation per section and column: pads of a section are alike
+    for a, b in zip(cfg.sec[:-1], cfg.sec[1:]):
+        avg[:, a:b], std[:, a:b] = avg[:, a:a + 1].clone(), std[:, a:a + 1].clone()
+    nb = np.full((n, nn), -1, np.int32)
+    for i in range(n if n > 1 else 0):
+        for a, b in zip(cfg.sec[:-1], cfg.sec[1:]):
+            full = int(rng.integers(0, b - a + 1))
+            nb[i, a:a + full] = (i + rng.integers(1, n, full)) % n
+    packed = np.where(nb >= 0, nb * 27 + 13, -1).astype(np.int32)
+    j, real = dev(np.maximum(nb, 0)).long(), dev(nb >= 0)[..., None]
+    r = torch.where(real, x[j] - x[:, None], 1.0)
+    w = torch.where(real, fbar[j] - fbar[:, None] + r @ vbar[0].T, 0.0)
+    R, Rd = torch.func.jvp(lambda q: _env(q, rmin, rmax), (r,), (w,))
+    tl = dev(ty).long()
+    R = (torch.where(real, R, 0.0) - avg[tl]) / std[tl]
+    Rd = -torch.where(real, Rd, 0.0) / std[tl]  # the env derivative is by the center atom
+    Ws = [dev(W) for net in p.emb for W, _ in net]
+    bs = [dev(b) for net in p.emb for _, b in net]
+    leaf = [q.clone().requires_grad_() for q in Ws + bs]
+
+    def xyz_of(R):
+        out = 0
+        for t, (a, b) in enumerate(zip(cfg.sec[:-1], cfg.sec[1:])):
+            h = R[:, a:b, :1]
+            for k in range(3):
+                W, bias = leaf[3 * t + k], leaf[len(Ws) + 3 * t + k]
+                y = torch.tanh(h @ W + bias)
+                h = _res(W, h, y) if k else y
+            out = out + R[:, a:b].transpose(1, 2) @ h
+        return out / nn
+
+    def D_of(X):
+        return (X.transpose(1, 2) @ X[:, :, :ax]).reshape(n, -1)
+
+    xyz, xyz_t = torch.func.jvp(xyz_of, (R,), (Rd,))
+    D, Dt = torch.func.jvp(D_of, (xyz,), (xyz_t,))
+    dD, dDt = (dev(rng.normal(0, 1, (n, M * ax))) for _ in range(2))
+    want = torch.autograd.grad((D * dD).sum() + (Dt * dDt).sum(), leaf)
+    drow = np.arange(n, dtype=np.int32)[::-1].copy()
+    dr, cw, box = dev(drow), x.contiguous(), dev(np.full((1, 3), 50.0))
+    off, rf = dev(np.array([0, n], np.int32)), dev(np.zeros(n, np.int32))
+    widths, sec = np.array([1, 25, 50, 100], np.int32), cfg.sec
+    fold = np.ones(nt * nt, np.uint8)
+    s = torch.cuda.current_stream().cuda_stream
+    got_x = torch.full((n, 4, M), float("nan"), dtype=torch.float64, device="cuda")
+    got_d = torch.full((n, M * ax), float("nan"), dtype=torch.float64, device="cuda")
+    xc, xtc, nl, tyd = xyz.detach().contiguous(), xyz_t.detach().contiguous(), dev(packed), dev(ty)
+    cap.call("dpb_se_a_train_tan_f64", cap.ptr(got_x), cap.ptr(got_d), cap.ptr(xc), cap.ptr(avg),
+             cap.ptr(std), cap.ptr(fbar), cap.ptr(vbar), cap.ptr(cw), cap.ptr(nl), cap.ptr(tyd),
+             cap.ptr(dr), cap.ptr(off), cap.ptr(box), cap.ptr(rf), 1, vp(Ws), vp(bs),
+             widths.ctypes.data, sec.ctypes.data, sec.size, n, ax,
+             ctypes.c_float(rmax), ctypes.c_float(rmin), s)
+    g = [torch.zeros_like(q) for q in Ws + bs]
+    scratch = torch.empty(8 * n * M, dtype=torch.float64, device="cuda")
+    a1, a2 = dD[dr.long()].contiguous(), dDt[dr.long()].contiguous()
+    cap.call("dpb_se_a_train_rev_f64", vp(g[:len(Ws)]), vp(g[len(Ws):]), cap.ptr(scratch),
+             cap.ptr(xc), cap.ptr(xtc), cap.ptr(a1), cap.ptr(a2), cap.ptr(avg), cap.ptr(std),
+             cap.ptr(fbar), cap.ptr(vbar), cap.ptr(cw), cap.ptr(nl), cap.ptr(tyd), cap.ptr(dr),
+             cap.ptr(off), cap.ptr(box), cap.ptr(rf), 1, vp(Ws), vp(bs), widths.ctypes.data,
+             sec.ctypes.data, sec.size, n, ax, fold.ctypes.data, ctypes.c_float(rmax),
+             ctypes.c_float(rmin), s)
+    for a, b in ((got_x, xyz_t.detach()), (got_d[dr.long()], Dt.detach())):
+        assert float((a - b).abs().max()) <= 1e-12 * max(1.0, float(b.abs().max()))
+    for a, b in zip(g, want):
+        assert float((a - b).abs().max()) <= 1e-11 * max(1.0, float(b.abs().max()))
