@@ -251,9 +251,10 @@ __device__ __forceinline__ void tr_load_col(T (&a)[R], const T* base, int c) {
 
 // acc[r] += a[r] w for the R rows of a group. FP32 rows go two at a time (packed
 // FMA): the warp-per-atom kernels are bound by issue slots and the latency between
-// them (reverse pass: 8 warps per SM, 49 % of the slots, 31 % of the FMA pipe), so
-// half the instructions shorten them. 16 frames of 192 atoms: reverse pass
-// 1774 -> 1584 us, backward 494 -> 466, tangent 440 -> 402; forward unchanged.
+// them (8 warps per SM, half of the slots, 31 % of the FMA pipe), so half the
+// instructions shorten them. 16 frames of 192 atoms: reverse pass 1774 -> 1584 us
+// (the standard net has its own, 1011), backward 494 -> 466, tangent 440 -> 402;
+// forward unchanged.
 template <typename T, int R>
 __device__ __forceinline__ void tr_axpy(T (&acc)[R], const T (&a)[R], T w) {
   if constexpr (sizeof(T) == 4 && R % 2 == 0) {

@@ -96,25 +96,28 @@ __device__ __forceinline__ int em_c2(int j, int u, int v) {
 }
 
 // layer 2 and its adjoint in fragment order, W1 and b1 padded to 28
-__device__ inline void em_stage_f2(double* F2, const double* W2) {
+template <typename T>
+__device__ inline void em_stage_f2(T* F2, const T* W2) {
   for (int e = threadIdx.x; e < EM_F2; e += blockDim.x) {
     const int lane = e & 31, j = (e >> 5) % 7, s = (e >> 5) / 7, g = lane >> 2;
     const int k = 4 * s + (lane & 3), c = em_c2(j, g >> 1, g & 1);
-    F2[e] = k < 25 && c >= 0 ? W2[k * 50 + c] : 0.;
+    F2[e] = k < 25 && c >= 0 ? W2[k * 50 + c] : (T)0;
   }
 }
-__device__ inline void em_stage_b2(double* B2, const double* W2) {
+template <typename T>
+__device__ inline void em_stage_b2(T* B2, const T* W2) {
   for (int e = threadIdx.x; e < EM_B2; e += blockDim.x) {
     const int lane = e & 31, q = (e >> 5) & 3, step = (e >> 5) >> 2, g = lane >> 2;
     const int c = em_c2(step >> 1, lane & 3, step & 1);
     const int k = 4 * (2 * q + (g & 1)) + (g >> 1);
-    B2[e] = c >= 0 && k < 25 ? W2[k * 50 + c] : 0.;
+    B2[e] = c >= 0 && k < 25 ? W2[k * 50 + c] : (T)0;
   }
 }
-__device__ inline void em_stage_v(double* V, const TrNet<double>& net, int t) {
+template <typename T>
+__device__ inline void em_stage_v(T* V, const TrNet<T>& net, int t) {
   for (int e = threadIdx.x; e < 28; e += blockDim.x) {
-    V[e] = e < 25 ? net.W[t][0][e] : 0.;
-    V[28 + e] = e < 25 ? net.b[t][0][e] : 0.;
+    V[e] = e < 25 ? net.W[t][0][e] : (T)0;
+    V[28 + e] = e < 25 ? net.b[t][0][e] : (T)0;
   }
   for (int e = threadIdx.x; e < 50; e += blockDim.x) V[56 + e] = net.b[t][1][e];
 }
@@ -516,10 +519,10 @@ k_emb_bwd_dmma(double* __restrict__ gem, const double* __restrict__ em,
 }
 
 // ------------------------------------------------- reverse over tangent --
-// The weight gradients of J = sum Ebar E + <u, g> (k_tr_rev's) on the FP64
-// matrix instructions. The FMA form adds every row group's share of the 6,250
-// weight gradients to shared memory: the atomics and the operand reads around
-// them held it at a seventh of the FP64 rate. Here the eight warps of a CTA
+// The weight gradients of J = sum Ebar E + <u, g> (k_tr_rev's) on the matrix
+// instructions, FP64 and FP32. The FMA form adds every row group's share of the
+// 6,250 weight gradients to shared memory: the atomics and the operand reads
+// around them held it at a seventh of the FMA rate. Here the eight warps of a CTA
 // take one 16-row tile each, of any atoms, and go through the net in step: layer
 // 3 one 16-channel tile at a time, whose adjoints of all 128 rows meet in
 // shared memory, and warp w adds their product with the rows' layer-2 outputs
@@ -534,24 +537,131 @@ k_emb_bwd_dmma(double* __restrict__ gem, const double* __restrict__ em,
 // Tiles are numbered tile-in-atom first, so the empty ones (beyond an atom's
 // neighbors) are the last and the rest come out even over the warps.
 //
-// Measured, 4 frames of 192 atoms: 1666 -> 461 us (FP64 matrix pipe 44 % busy, the
-// FMA pipe 10 %; the eight warps' waits for each other and for operands are the rest).
+// Measured: FP64, 4 frames of 192 atoms 1666 -> 461 us (FP64 matrix pipe 44 % busy,
+// the FMA pipe 10 %); FP32, 16 frames 1584 -> 1011 us (matrix pipe 35 %, issue
+// slots 43 %: splitting the operands takes three instructions per element). The rest
+// is the latency of two warps per scheduler; the accumulators leave room for no more.
 constexpr int EM_REV_NW = 8;
-constexpr int EM_REV_W3 = 54 * 100 + 4;
-constexpr int EM_REV_V = 28 + 28 + 52;
-constexpr int EM_P2S = 52;                     // row stride of staged layer-2 vectors
-constexpr int EM_P1S = 28;                     // of layer-1 vectors
-constexpr int EM_REV_H = 2 * 16 * EM_P2S;      // per warp: outputs, tangents
-constexpr int EM_REV_Z = 2 * 16 * EM_TS;       // layer-3 adjoints of a channel tile
-constexpr int EM_REV_R = 16 * 8;               // env rows and their tangents
-constexpr int EM_REV_N = EM_REV_W3 + EM_F2 + EM_B2 + EM_REV_V +
-                         EM_REV_NW * (EM_REV_H + EM_REV_Z + EM_REV_R + 56) + 4;
+// Row strides that keep the operand reads free of (most) bank conflicts for
+// 8-byte and 4-byte elements, in elements; W3's rows, staged layer-2 and
+// layer-1 vectors. NJ: unit tiles per warp in the W3 gradient. Four-byte
+// accumulators leave room for two, each warp then over half of the rows: an
+// operand read serves twice as many products.
+template <typename T>
+struct EmRev {
+  static constexpr bool F64 = sizeof(T) == 8;
+  static constexpr int S3 = 100, P2S = F64 ? 52 : 56, P1S = F64 ? 28 : 40;
+  static constexpr int NJ = F64 ? 1 : 2;
+  static constexpr int W3 = 54 * S3 + 4;    // operand elements
+  static constexpr int V = 28 + 28 + 52;
+  static constexpr int H = 2 * 16 * P2S;    // per warp: layer-2 outputs, tangents
+  static constexpr int Z = 2 * 16 * EM_TS;  // layer-3 adjoints of a channel tile
+  static constexpr int R = 16 * 8;          // env rows and their tangents
+  static constexpr int N = W3 * 8 / (int)sizeof(T) + EM_F2 + EM_B2 + V + EM_REV_NW * (H + Z + R + 56) +
+                           EM_REV_NW * 4 / (int)sizeof(T);
+};
 
+// An operand element: FP64 as it is, FP32 as two TF32 terms (8 bytes either way).
+struct EmTf {
+  uint32_t hi, lo;
+};
+template <typename T>
+struct EmOp {
+  using type = T;
+};
+template <>
+struct EmOp<float> {
+  using type = EmTf;
+};
+__device__ __forceinline__ double em_op(double x) { return x; }
+__device__ __forceinline__ EmTf em_op(float x) {
+  EmTf r;
+  r.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+  r.lo = __float_as_uint(x - __uint_as_float(r.hi));
+  return r;
+}
+
+// d = A B + c over eight k
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
+                                         uint32_t b1, float c0, float c1, float c2, float c3) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%10, %11, %12, %13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2),
+        "f"(c3));
+}
+
+// c += A B over eight k: a0, a1 rows g, g + 8 at k = t, a2, a3 at k = 4 + t, b0, b1
+// column g at k = t, 4 + t; the same with rows 0 .. 7 only, and over four k.
+__device__ __forceinline__ void em_mma(double (&c)[4], double a0, double a1, double a2, double a3,
+                                       double b0, double b1) {
+  dmma16(c, a0, a1, b0);
+  dmma16(c, a2, a3, b1);
+}
+__device__ __forceinline__ void em_mma8(double (&c)[4], double a0, double a2, double b0,
+                                        double b1) {
+  dmma8(c[0], c[1], a0, b0);
+  dmma8(c[0], c[1], a2, b1);
+}
+__device__ __forceinline__ void em_mma_k4(double (&c)[4], double a0, double a1, double b) {
+  dmma16(c, a0, a1, b);
+}
+__device__ __forceinline__ void em_mma8_k4(double (&c)[4], double a, double b) {
+  dmma8(c[0], c[1], a, b);
+}
+// FP32: three products (the fourth is below 2^-23 of the result). The matrix
+// instruction truncates what it adds to its accumulator, which shows in sums
+// that run on (five times the error of FP32 sums in the first layer's
+// gradient): every eight k start from zero, the small products on their own, and
+// the rounded FP32 add carries the sum.
+__device__ __forceinline__ void em_mma(float (&c)[4], EmTf a0, EmTf a1, EmTf a2, EmTf a3, EmTf b0,
+                                       EmTf b1) {
+  const uint32_t ah[4] = {a0.hi, a1.hi, a2.hi, a3.hi}, al[4] = {a0.lo, a1.lo, a2.lo, a3.lo};
+  float d[4], e[4];
+  mma_tf32(d, al, b0.hi, b1.hi, 0.f, 0.f, 0.f, 0.f);
+  mma_tf32(e, ah, b0.hi, b1.hi, 0.f, 0.f, 0.f, 0.f);
+  mma_tf32(d, ah, b0.lo, b1.lo, d[0], d[1], d[2], d[3]);
+#pragma unroll
+  for (int k = 0; k < 4; k += 2) {
+    const float2 v = __fadd2_rn(make_float2(c[k], c[k + 1]),
+                                __fadd2_rn(make_float2(d[k], d[k + 1]),
+                                           make_float2(e[k], e[k + 1])));
+    c[k] = v.x;
+    c[k + 1] = v.y;
+  }
+}
+__device__ __forceinline__ void em_mma8(float (&c)[4], EmTf a0, EmTf a2, EmTf b0, EmTf b1) {
+  em_mma(c, a0, EmTf{0, 0}, a2, EmTf{0, 0}, b0, b1);
+}
+__device__ __forceinline__ void em_mma_k4(float (&c)[4], EmTf a0, EmTf a1, EmTf b) {
+  em_mma(c, a0, a1, EmTf{0, 0}, EmTf{0, 0}, b, EmTf{0, 0});
+}
+__device__ __forceinline__ void em_mma8_k4(float (&c)[4], EmTf a, EmTf b) {
+  em_mma(c, a, EmTf{0, 0}, EmTf{0, 0}, EmTf{0, 0}, b, EmTf{0, 0});
+}
+__device__ __forceinline__ double em_tanh(double x) { return tanh_f64(x); }
+__device__ __forceinline__ float em_tanh(float x) { return tr_tanh(x); }
+
+template <typename T>
+struct EmPair;
+template <>
+struct EmPair<double> {
+  using type = double2;
+};
+template <>
+struct EmPair<float> {
+  using type = float2;
+};
+
+template <typename T>
 __global__ void __launch_bounds__(32 * EM_REV_NW, 1)
-k_emb_rev_dmma(TrGrad<double> grad, const double* __restrict__ xbar,
-               const double* __restrict__ xbard, const double* __restrict__ avg,
-               const double* __restrict__ std_, const double* __restrict__ fbar,
-               const double* __restrict__ vbar, TrNet<double> net, TrGeom g, EmSplit split) {
+k_emb_rev_mma(TrGrad<T> grad, const T* __restrict__ xbar,
+               const T* __restrict__ xbard, const T* __restrict__ avg,
+               const T* __restrict__ std_, const double* __restrict__ fbar,
+               const double* __restrict__ vbar, TrNet<T> net, TrGeom g, EmSplit split) {
+  using Ly = EmRev<T>;
+  using T2 = typename EmPair<T>::type;
+  constexpr int S3 = Ly::S3, P2S = Ly::P2S, P1S = Ly::P1S, NJ = Ly::NJ;
   extern __shared__ __align__(16) double esm[];
   pdl_wait();
   pdl_trigger();
@@ -559,39 +669,43 @@ k_emb_rev_dmma(TrGrad<double> grad, const double* __restrict__ xbar,
   const int gr = lane >> 2, t4 = lane & 3;
   int t = 0;
   while (t + 1 < g.ntypes && (int)blockIdx.x >= split.first[t + 1]) ++t;
-  double* W3 = esm;
-  double* F2 = W3 + EM_REV_W3;
-  double* B2 = F2 + EM_F2;
-  double* V = B2 + EM_B2;
-  double* H = V + EM_REV_V;
-  double* Z = H + EM_REV_NW * EM_REV_H;
-  double* R = Z + EM_REV_NW * EM_REV_Z;
-  double* G1 = R + EM_REV_NW * EM_REV_R;
+  using Op = typename EmOp<T>::type;
+  Op* W3 = reinterpret_cast<Op*>(esm);
+  T* F2 = reinterpret_cast<T*>(W3 + Ly::W3);
+  T* B2 = F2 + EM_F2;
+  T* V = B2 + EM_B2;
+  T* H = V + Ly::V;
+  T* Z = H + EM_REV_NW * Ly::H;
+  T* R = Z + EM_REV_NW * Ly::Z;
+  T* G1 = R + EM_REV_NW * Ly::R;
   int* act = reinterpret_cast<int*>(G1 + EM_REV_NW * 56);
-  for (int e = threadIdx.x; e < EM_REV_W3; e += blockDim.x) {
-    const int r = e / 100, c = e - r * 100;
-    W3[e] = r < 25 ? net.W[t][2][e]
-            : r == 25 ? net.b[t][2][c]
-            : r < 51 ? net.W[t][2][(r - 1) * 100 + c] : 0.;
+  for (int e = threadIdx.x; e < Ly::W3; e += blockDim.x) {
+    const int r = e / S3, c = e - r * S3;
+    W3[e] = em_op(r < 25    ? net.W[t][2][e]
+                  : r == 25 ? net.b[t][2][c]
+                  : r < 51  ? net.W[t][2][e - S3]
+                            : (T)0);
   }
   em_stage_f2(F2, net.W[t][1]);
   em_stage_b2(B2, net.W[t][1]);
   em_stage_v(V, net, t);
-  for (int e = threadIdx.x; e < EM_REV_NW * 56; e += blockDim.x) G1[e] = 0.;
-  double* hs = H + w * EM_REV_H;
-  double* hd = hs + 16 * EM_P2S;
-  double* zs = Z + w * EM_REV_Z;
-  double* zd = zs + 16 * EM_TS;
-  double* rr = R + w * EM_REV_R;
-  double* g1 = G1 + w * 56;
+  for (int e = threadIdx.x; e < EM_REV_NW * 56; e += blockDim.x) G1[e] = (T)0;
+  T* hs = H + w * Ly::H;
+  T* hd = hs + 16 * P2S;
+  T* zs = Z + w * Ly::Z;
+  T* zd = zs + 16 * EM_TS;
+  T* rr = R + w * Ly::R;
+  T* g1 = G1 + w * 56;
   int* ent = reinterpret_cast<int*>(zs);  // read before the first adjoints are written
   int* secn = ent + g.nnei;
-  double gw3[7][4], gw2[2][4];
+  T gw3[7][NJ][4], gw2[2][4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    gw2[0][k] = gw2[1][k] = 0.;
+    gw2[0][k] = gw2[1][k] = (T)0;
 #pragma unroll
-    for (int m = 0; m < 7; ++m) gw3[m][k] = 0.;
+    for (int m = 0; m < 7; ++m)
+#pragma unroll
+      for (int n = 0; n < NJ; ++n) gw3[m][n][k] = (T)0;
   }
   const int nb = split.first[t + 1] - split.first[t];
   const long long ntile = (long long)g.nrows * ((g.sec[t + 1] - g.sec[t] + 15) / 16);
@@ -612,28 +726,28 @@ k_emb_rev_dmma(TrGrad<double> grad, const double* __restrict__ xbar,
     if (lane == 0) act[w] = ne > 0;
     if (!__syncthreads_or(ne > 0)) break;
     any = true;
-    const double* xb = xbar + (size_t)row * 400;
-    const double* xd = xbard + (size_t)row * 400;
-    double x0 = 0., x1 = 0., d0 = 0., d1 = 0.;  // input and tangent of rows g, g + 8
-    double hb2[7][4], hbd2[7][4];               // adjoints of layer 2's output and tangent
-    auto layer1 = [&](double (&ha)[EM_S1], double (&hb)[EM_S1]) {
+    const T* xb = xbar + (size_t)row * 400;
+    const T* xd = xbard + (size_t)row * 400;
+    T x0 = (T)0, x1 = (T)0, d0 = (T)0, d1 = (T)0;  // input and tangent of rows g, g + 8
+    T hb2[7][4], hbd2[7][4];               // adjoints of layer 2's output and tangent
+    auto layer1 = [&](T (&ha)[EM_S1], T (&hb)[EM_S1]) {
 #pragma unroll
       for (int s = 0; s < EM_S1; ++s) {
-        const double w1 = V[4 * s + t4], b1 = V[28 + 4 * s + t4];
-        ha[s] = tanh_f64(fma(x0, w1, b1));
-        hb[s] = tanh_f64(fma(x1, w1, b1));
+        const T w1 = V[4 * s + t4], b1 = V[28 + 4 * s + t4];
+        ha[s] = em_tanh(fma(x0, w1, b1));
+        hb[s] = em_tanh(fma(x1, w1, b1));
       }
     };
     if (ne > 0) {
-      double x = 0., d = 0.;
+      T x = (T)0, d = (T)0;
       if (lane < 16) {
-        double Rv[4] = {0., 0., 0., 0.}, Rd[4] = {0., 0., 0., 0.}, mu = 0.;
+        T Rv[4] = {(T)0, (T)0, (T)0, (T)0}, Rd[4] = {(T)0, (T)0, (T)0, (T)0}, mu = (T)0;
         if (lane < ne) {
           const TrAtom A = tr_atom(g, row);
           const int en = ent[e0 + lane];
-          tr_env_tangent<double>(Rv, Rd, g, A, en & 0xFFFF, avg + (size_t)A.ti * g.nnei * 4,
+          tr_env_tangent<T>(Rv, Rd, g, A, en & 0xFFFF, avg + (size_t)A.ti * g.nnei * 4,
                                  std_ + (size_t)A.ti * g.nnei * 4, fbar, vbar);
-          mu = (double)(en >> 16);
+          mu = (T)(en >> 16);
         }
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
@@ -649,65 +763,77 @@ k_emb_rev_dmma(TrGrad<double> grad, const double* __restrict__ xbar,
       d1 = __shfl_sync(0xffffffffu, d, 8 + gr);
       __syncwarp();
       // layers 1 and 2, outputs and tangents staged at their positions
-      double h1a[EM_S1], h1b[EM_S1], h2[7][4], ht[7][4];
+      T h1a[EM_S1], h1b[EM_S1], h2[7][4], ht[7][4];
       layer1(h1a, h1b);
 #pragma unroll
       for (int j = 0; j < 7; ++j) {
         const bool ok = 4 * j + t4 < 25;
-        h2[j][0] = h2[j][2] = ok ? V[56 + 4 * j + t4] : 0.;
-        h2[j][1] = h2[j][3] = ok ? V[56 + 4 * j + t4 + 25] : 0.;
+        h2[j][0] = h2[j][2] = ok ? V[56 + 4 * j + t4] : (T)0;
+        h2[j][1] = h2[j][3] = ok ? V[56 + 4 * j + t4 + 25] : (T)0;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) ht[j][k] = 0.;
+        for (int k = 0; k < 4; ++k) ht[j][k] = (T)0;
       }
 #pragma unroll
-      for (int s = 0; s < EM_S1; ++s) {
-        const double w1 = V[4 * s + t4];
-        const double ta = (1. - h1a[s] * h1a[s]) * (d0 * w1);
-        const double tb = (1. - h1b[s] * h1b[s]) * (d1 * w1);
+      for (int s = 0; s < EM_S1; s += 2) {
+        Op ha[2], hb[2], ta[2], tb[2];
+#pragma unroll
+        for (int e = 0; e < 2 && s + e < EM_S1; ++e) {
+          const T w1 = V[4 * (s + e) + t4];
+          ta[e] = em_op(((T)1 - h1a[s + e] * h1a[s + e]) * (d0 * w1));
+          tb[e] = em_op(((T)1 - h1b[s + e] * h1b[s + e]) * (d1 * w1));
+          ha[e] = em_op(h1a[s + e]);
+          hb[e] = em_op(h1b[s + e]);
+        }
 #pragma unroll
         for (int j = 0; j < 7; ++j) {
-          const double b = F2[(s * 7 + j) * 32 + lane];
-          dmma16(h2[j], h1a[s], h1b[s], b);
-          dmma16(ht[j], ta, tb, b);
+          const Op b = em_op(F2[(s * 7 + j) * 32 + lane]);
+          if (s + 1 < EM_S1) {
+            const Op c = em_op(F2[((s + 1) * 7 + j) * 32 + lane]);
+            em_mma(h2[j], ha[0], hb[0], ha[1], hb[1], b, c);
+            em_mma(ht[j], ta[0], tb[0], ta[1], tb[1], b, c);
+          } else {
+            em_mma_k4(h2[j], ha[0], hb[0], b);
+            em_mma_k4(ht[j], ta[0], tb[0], b);
+          }
         }
       }
 #pragma unroll
       for (int j = 0; j < 7; ++j) {
-        const double w1 = V[4 * j + t4];
-        const double ta = (1. - h1a[j] * h1a[j]) * (d0 * w1);
-        const double tb = (1. - h1b[j] * h1b[j]) * (d1 * w1);
+        const T w1 = V[4 * j + t4];
+        const T ta = ((T)1 - h1a[j] * h1a[j]) * (d0 * w1);
+        const T tb = ((T)1 - h1b[j] * h1b[j]) * (d1 * w1);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const double y = tanh_f64(h2[j][k]);
+          const T y = em_tanh(h2[j][k]);
           h2[j][k] = y + (k < 2 ? h1a[j] : h1b[j]);
-          ht[j][k] = (1. - y * y) * ht[j][k] + (k < 2 ? ta : tb);
+          ht[j][k] = ((T)1 - y * y) * ht[j][k] + (k < 2 ? ta : tb);
         }
         if (j == 6 && t4 == 1) {  // positions 50 (the constant), 51
-          h2[j][0] = h2[j][2] = 1.;
-          h2[j][1] = h2[j][3] = 0.;
+          h2[j][0] = h2[j][2] = (T)1;
+          h2[j][1] = h2[j][3] = (T)0;
 #pragma unroll
-          for (int k = 0; k < 4; ++k) ht[j][k] = 0.;
+          for (int k = 0; k < 4; ++k) ht[j][k] = (T)0;
         }
         if (j < 6 || t4 < 2) {
-          const int o = gr * EM_P2S + 8 * j + 2 * t4;
-          *reinterpret_cast<double2*>(hs + o) = make_double2(h2[j][0], h2[j][1]);
-          *reinterpret_cast<double2*>(hs + o + 8 * EM_P2S) = make_double2(h2[j][2], h2[j][3]);
-          *reinterpret_cast<double2*>(hd + o) = make_double2(ht[j][0], ht[j][1]);
-          *reinterpret_cast<double2*>(hd + o + 8 * EM_P2S) = make_double2(ht[j][2], ht[j][3]);
+          const int o = gr * P2S + 8 * j + 2 * t4;
+          *reinterpret_cast<T2*>(hs + o) = T2{h2[j][0], h2[j][1]};
+          *reinterpret_cast<T2*>(hs + o + 8 * P2S) = T2{h2[j][2], h2[j][3]};
+          *reinterpret_cast<T2*>(hd + o) = T2{ht[j][0], ht[j][1]};
+          *reinterpret_cast<T2*>(hd + o + 8 * P2S) = T2{ht[j][2], ht[j][3]};
         }
       }
       // the layer-3 residual's share of the layer-2 adjoints
-      const double ra = rr[gr * 8 + t4], rb = rr[(gr + 8) * 8 + t4];
-      const double qa = rr[gr * 8 + 4 + t4], qb = rr[(gr + 8) * 8 + 4 + t4];
+      const Op ra = em_op(rr[gr * 8 + t4]), rb = em_op(rr[(gr + 8) * 8 + t4]);
+      const Op qa = em_op(rr[gr * 8 + 4 + t4]), qb = em_op(rr[(gr + 8) * 8 + 4 + t4]);
 #pragma unroll
       for (int j = 0; j < 7; ++j) {
         const int c = em_c2(j, gr >> 1, gr & 1), o = t4 * 100 + (c < 0 ? 0 : c);
-        const double u = c < 0 ? 0. : xb[o] + xb[o + 50], v = c < 0 ? 0. : xd[o] + xd[o + 50];
+        const Op u = em_op(c < 0 ? (T)0 : xb[o] + xb[o + 50]);
+        const Op v = em_op(c < 0 ? (T)0 : xd[o] + xd[o + 50]);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) hb2[j][k] = hbd2[j][k] = 0.;
-        dmma16(hb2[j], ra, rb, u);
-        dmma16(hb2[j], qa, qb, v);
-        dmma16(hbd2[j], ra, rb, v);
+        for (int k = 0; k < 4; ++k) hb2[j][k] = hbd2[j][k] = (T)0;
+        em_mma(hb2[j], ra, rb, qa, qb, u, v);
+        em_mma_k4(hbd2[j], ra, rb, v);
       }
       __syncwarp();
     }
@@ -717,98 +843,116 @@ k_emb_rev_dmma(TrGrad<double> grad, const double* __restrict__ xbar,
         const int c = 16 * m + gr;
         const bool in = !LAST || gr < 4;
         const int o = t4 * 100 + c;
-        const double xb0 = in ? xb[o] : 0., xb1 = LAST ? 0. : xb[o + 8];
-        const double xd0 = in ? xd[o] : 0., xd1 = LAST ? 0. : xd[o + 8];
+        const Op xb0 = em_op(in ? xb[o] : (T)0), xb1 = em_op(LAST ? (T)0 : xb[o + 8]);
+        const Op xd0 = em_op(in ? xd[o] : (T)0), xd1 = em_op(LAST ? (T)0 : xd[o + 8]);
 #pragma unroll 1
         for (int n = 0; n < 2; ++n) {
-          double z[4] = {0., 0., 0., 0.}, zt[4] = {0., 0., 0., 0.};
-          const double* hr = hs + (8 * n + gr) * EM_P2S + 2 * t4;
+          T z[4] = {(T)0, (T)0, (T)0, (T)0}, zt[4] = {(T)0, (T)0, (T)0, (T)0};
+          const T* hr = hs + (8 * n + gr) * P2S + 2 * t4;
 #pragma unroll
           for (int j = 0; j < 7; ++j) {
-            double2 h = *reinterpret_cast<const double2*>(hr + 8 * j);
-            double2 q = *reinterpret_cast<const double2*>(hr + 16 * EM_P2S + 8 * j);
+            T2 h = *reinterpret_cast<const T2*>(hr + 8 * j);
+            T2 q = *reinterpret_cast<const T2*>(hr + 16 * P2S + 8 * j);
             if (j == 6) {  // positions past 50: the next row's
-              h.x = t4 < 2 ? h.x : 0.;
-              q.x = t4 < 2 ? q.x : 0.;
-              h.y = t4 < 1 ? h.y : 0.;
-              q.y = t4 < 1 ? q.y : 0.;
+              h.x = t4 < 2 ? h.x : (T)0;
+              q.x = t4 < 2 ? q.x : (T)0;
+              h.y = t4 < 1 ? h.y : (T)0;
+              q.y = t4 < 1 ? q.y : (T)0;
             }
-            const double* a = W3 + (4 * j + t4) * 100 + c;
-            const double* b = a + 2600;
+            const Op* a = W3 + (4 * j + t4) * S3 + c;
+            const Op* b = a + 26 * S3;
             if (LAST) {
-              dmma8(z[0], z[1], a[0], h.x);
-              dmma8(zt[0], zt[1], a[0], q.x);
-              dmma8(z[0], z[1], b[0], h.y);
-              dmma8(zt[0], zt[1], b[0], q.y);
+              em_mma8(z, a[0], b[0], em_op(h.x), em_op(h.y));
+              em_mma8(zt, a[0], b[0], em_op(q.x), em_op(q.y));
             } else {
-              const double a0 = a[0], a1 = a[8], b0 = b[0], b1 = b[8];
-              dmma16(z, a0, a1, h.x);
-              dmma16(zt, a0, a1, q.x);
-              dmma16(z, b0, b1, h.y);
-              dmma16(zt, b0, b1, q.y);
+              const Op a0 = a[0], a1 = a[8], b0 = b[0], b1 = b[8];
+              em_mma(z, a0, a1, b0, b1, em_op(h.x), em_op(h.y));
+              em_mma(zt, a0, a1, b0, b1, em_op(q.x), em_op(q.y));
             }
           }
-          double gb[4] = {0., 0., 0., 0.}, gd[4] = {0., 0., 0., 0.};
-          const double rv = rr[(8 * n + gr) * 8 + t4], rd = rr[(8 * n + gr) * 8 + 4 + t4];
+          T gb[4] = {(T)0, (T)0, (T)0, (T)0}, gd[4] = {(T)0, (T)0, (T)0, (T)0};
+          const Op rv = em_op(rr[(8 * n + gr) * 8 + t4]);
+          const Op rd = em_op(rr[(8 * n + gr) * 8 + 4 + t4]);
           if (LAST) {
-            dmma8(gb[0], gb[1], xb0, rv);
-            dmma8(gb[0], gb[1], xd0, rd);
-            dmma8(gd[0], gd[1], xd0, rv);
+            em_mma8(gb, xb0, xd0, rv, rd);
+            em_mma8_k4(gd, xd0, rv);
           } else {
-            dmma16(gb, xb0, xb1, rv);
-            dmma16(gb, xd0, xd1, rd);
-            dmma16(gd, xd0, xd1, rv);
+            em_mma(gb, xb0, xb1, xd0, xd1, rv, rd);
+            em_mma_k4(gd, xd0, xd1, rv);
           }
 #pragma unroll
           for (int k = 0; k < (LAST ? 2 : 4); ++k)
             if (in) {
-              const double y = tanh_f64(z[k]), q = 1. - y * y;
+              const T y = em_tanh(z[k]), q = (T)1 - y * y;
               const int p = (8 * n + 2 * t4 + (k & 1)) * EM_TS + gr + 8 * (k >> 1);
-              zs[p] = (gb[k] - 2. * y * zt[k] * gd[k]) * q;
+              zs[p] = (gb[k] - (T)2 * y * zt[k] * gd[k]) * q;
               zd[p] = gd[k] * q;
             }
         }
         __syncwarp();
 #pragma unroll 1
-        for (int s = 0; s < (LAST ? 1 : 4); ++s) {
-          const int k = 4 * s + t4;
-          const double a0 = zs[gr * EM_TS + k], a1 = zs[(gr + 8) * EM_TS + k];
-          const double e0_ = zd[gr * EM_TS + k], e1_ = zd[(gr + 8) * EM_TS + k];
-          const double* bp = W3 + ((gr >> 1) + 26 * (gr & 1)) * 100 + 16 * m + k;
+        for (int s = 0; s < (LAST ? 1 : 2); ++s) {
+          const int k = 8 * s + t4;
+          const T *zp = zs + gr * EM_TS + k, *dp = zd + gr * EM_TS + k;
+          const Op* bp = W3 + ((gr >> 1) + 26 * (gr & 1)) * S3 + 16 * m + k;
+          const Op a0 = em_op(zp[0]), a1 = em_op(zp[8 * EM_TS]);
+          const Op b0 = em_op(dp[0]), b1 = em_op(dp[8 * EM_TS]);
+          if (LAST) {  // four channels
 #pragma unroll
-          for (int j = 0; j < 7; ++j) {
-            const double b = bp[400 * j];
-            dmma16(hb2[j], a0, a1, b);
-            dmma16(hbd2[j], e0_, e1_, b);
+            for (int j = 0; j < 7; ++j) {
+              em_mma_k4(hb2[j], a0, a1, bp[4 * S3 * j]);
+              em_mma_k4(hbd2[j], b0, b1, bp[4 * S3 * j]);
+            }
+          } else {
+            const Op a2 = em_op(zp[4]), a3 = em_op(zp[8 * EM_TS + 4]);
+            const Op b2 = em_op(dp[4]), b3 = em_op(dp[8 * EM_TS + 4]);
+#pragma unroll
+            for (int j = 0; j < 7; ++j) {
+              const Op c0 = bp[4 * S3 * j], c1 = bp[4 * S3 * j + 4];
+              em_mma(hb2[j], a0, a1, a2, a3, c0, c1);
+              em_mma(hbd2[j], b0, b1, b2, b3, c0, c1);
+            }
           }
         }
       }
       __syncthreads();
-      // W3 gradient of this tile's channels, units at positions 8 w ..
-      if (w < 7) {
-        double c[2][4];
+      // W3 gradient of this tile's channels, units at positions 8 jt .. (+ 8)
+      if (NJ == 2 || w < 7) {
+        const int jt = NJ == 2 ? 2 * (w & 3) : w, v0 = NJ == 2 ? 4 * (w >> 2) : 0;
+        T c[2][NJ][4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) c[0][k] = c[1][k] = 0.;
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+          for (int n = 0; n < NJ; ++n) c[0][n][k] = c[1][n][k] = (T)0;
 #pragma unroll 1
-        for (int v = 0; v < EM_REV_NW; ++v) {
+        for (int v = v0; v < (NJ == 2 ? v0 + 4 : EM_REV_NW); ++v) {
           if (!act[v]) continue;
-          const double* zp = Z + v * EM_REV_Z + t4 * EM_TS + gr;
-          const double* hp = H + v * EM_REV_H + t4 * EM_P2S + 8 * w + gr;
+          const T* zp = Z + v * Ly::Z + t4 * EM_TS + gr;
+          const T* hp = H + v * Ly::H + t4 * P2S + 8 * jt + gr;
 #pragma unroll
-          for (int s = 0; s < 8; ++s) {  // four steps of outputs, four of tangents
-            const double* zq = zp + 4 * s * EM_TS;
-            const double b = hp[4 * s * EM_P2S];
-            if (LAST)
-              dmma8(c[s & 1][0], c[s & 1][1], zq[0], b);
-            else
-              dmma16(c[s & 1], zq[0], zq[8], b);
+          for (int s = 0; s < 4; ++s) {  // two steps of outputs, two of tangents
+            const T *zq = zp + 8 * s * EM_TS, *zr = zq + 4 * EM_TS;
+            const T *hq = hp + 8 * s * P2S, *hr = hq + 4 * P2S;
+            if (LAST) {
+              const Op a0 = em_op(zq[0]), a2 = em_op(zr[0]);
+#pragma unroll
+              for (int n = 0; n < NJ; ++n)
+                em_mma8(c[s & 1][n], a0, a2, em_op(hq[8 * n]), em_op(hr[8 * n]));
+            } else {
+              const Op a0 = em_op(zq[0]), a1 = em_op(zq[8]), a2 = em_op(zr[0]), a3 = em_op(zr[8]);
+#pragma unroll
+              for (int n = 0; n < NJ; ++n)
+                em_mma(c[s & 1][n], a0, a1, a2, a3, em_op(hq[8 * n]), em_op(hr[8 * n]));
+            }
           }
         }
 #pragma unroll
         for (int q = 0; q < 7; ++q)
           if (q == m)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) gw3[q][k] += c[0][k] + c[1][k];
+            for (int n = 0; n < NJ; ++n)
+#pragma unroll
+              for (int k = 0; k < 4; ++k) gw3[q][n][k] += c[0][n][k] + c[1][n][k];
       }
       __syncthreads();
     };
@@ -816,10 +960,10 @@ k_emb_rev_dmma(TrGrad<double> grad, const double* __restrict__ xbar,
     for (int m = 0; m < 6; ++m) tile(std::integral_constant<int, 0>{}, m);
     tile(std::integral_constant<int, 1>{}, 6);
     // layer 2's pre-activation adjoints take the place of its outputs and tangents
-    double h1a[EM_S1], h1b[EM_S1];
+    T h1a[EM_S1], h1b[EM_S1];
     if (ne > 0) {
       layer1(h1a, h1b);
-      double u[4][4], v[4][4];  // layer 1's: channel 4 s + t of row g at [s / 2][s % 2]
+      T u[4][4], v[4][4];  // layer 1's: channel 4 s + t of row g at [s / 2][s % 2]
 #pragma unroll
       for (int j = 0; j < 7; ++j) {
         u[j >> 1][j & 1] = hb2[j][0] + hb2[j][1];
@@ -827,44 +971,46 @@ k_emb_rev_dmma(TrGrad<double> grad, const double* __restrict__ xbar,
         v[j >> 1][j & 1] = hbd2[j][0] + hbd2[j][1];
         v[j >> 1][2 + (j & 1)] = hbd2[j][2] + hbd2[j][3];
         if (j == 6 && t4 > 0) continue;
-        const double w1 = V[4 * j + t4];
-        double* ho = hs + gr * EM_P2S + 8 * j + 2 * t4;
-        double* po = hd + gr * EM_P2S + 8 * j + 2 * t4;
+        const T w1 = V[4 * j + t4];
+        T* ho = hs + gr * P2S + 8 * j + 2 * t4;
+        T* po = hd + gr * P2S + 8 * j + 2 * t4;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const int o = (k >> 1) * 8 * EM_P2S + (k & 1);
-          const double h = k < 2 ? h1a[j] : h1b[j];
-          const double y = ho[o] - h, q = 1. - y * y;
-          const double yt = po[o] - (1. - h * h) * ((k < 2 ? d0 : d1) * w1);  // q times zdot
-          ho[o] = hb2[j][k] * q - 2. * y * yt * hbd2[j][k];
+          const int o = (k >> 1) * 8 * P2S + (k & 1);
+          const T h = k < 2 ? h1a[j] : h1b[j];
+          const T y = ho[o] - h, q = (T)1 - y * y;
+          const T yt = po[o] - ((T)1 - h * h) * ((k < 2 ? d0 : d1) * w1);  // q times zdot
+          ho[o] = hb2[j][k] * q - (T)2 * y * yt * hbd2[j][k];
           po[o] = hbd2[j][k] * q;
         }
       }
-      u[3][1] = u[3][3] = v[3][1] = v[3][3] = 0.;
+      u[3][1] = u[3][3] = v[3][1] = v[3][3] = (T)0;
       __syncwarp();
 #pragma unroll
-      for (int j = 0; j < 7; ++j)
+      for (int j = 0; j < 7; ++j) {
+        const int o = gr * P2S + 8 * j + 2 * t4;
+        const bool ok = j < 6 || t4 == 0;
+        const T2 zero = T2{(T)0, (T)0};
+        const T2 a0 = ok ? *reinterpret_cast<const T2*>(hs + o) : zero;
+        const T2 a1 = ok ? *reinterpret_cast<const T2*>(hs + o + 8 * P2S) : zero;
+        const T2 b0 = ok ? *reinterpret_cast<const T2*>(hd + o) : zero;
+        const T2 b1 = ok ? *reinterpret_cast<const T2*>(hd + o + 8 * P2S) : zero;
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int o = gr * EM_P2S + 8 * j + 2 * t4 + e;
-          const bool ok = j < 6 || t4 == 0;
-          const double a0 = ok ? hs[o] : 0., a1 = ok ? hs[o + 8 * EM_P2S] : 0.;
-          const double b0 = ok ? hd[o] : 0., b1 = ok ? hd[o + 8 * EM_P2S] : 0.;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const double b = B2[((2 * j + e) * 4 + q) * 32 + lane];
-            dmma16(u[q], a0, a1, b);
-            dmma16(v[q], b0, b1, b);
-          }
+        for (int q = 0; q < 4; ++q) {
+          const Op c0 = em_op(B2[((2 * j) * 4 + q) * 32 + lane]);
+          const Op c1 = em_op(B2[((2 * j + 1) * 4 + q) * 32 + lane]);
+          em_mma(u[q], em_op(a0.x), em_op(a1.x), em_op(a0.y), em_op(a1.y), c0, c1);
+          em_mma(v[q], em_op(b0.x), em_op(b1.x), em_op(b0.y), em_op(b1.y), c0, c1);
         }
+      }
 #pragma unroll
       for (int s = 0; s < EM_S1; ++s) {
-        const double w1 = V[4 * s + t4];
-        const double qa = 1. - h1a[s] * h1a[s], qb = 1. - h1b[s] * h1b[s];
-        const double ta = v[s >> 1][s & 1], tb = v[s >> 1][2 + (s & 1)];
-        const double za = (u[s >> 1][s & 1] - 2. * h1a[s] * (d0 * w1) * ta) * qa;
-        const double zb = (u[s >> 1][2 + (s & 1)] - 2. * h1b[s] * (d1 * w1) * tb) * qb;
-        double gws = fma(x0, za, fma(d0, ta * qa, fma(x1, zb, d1 * (tb * qb)))), gbs = za + zb;
+        const T w1 = V[4 * s + t4];
+        const T qa = (T)1 - h1a[s] * h1a[s], qb = (T)1 - h1b[s] * h1b[s];
+        const T ta = v[s >> 1][s & 1], tb = v[s >> 1][2 + (s & 1)];
+        const T za = (u[s >> 1][s & 1] - (T)2 * h1a[s] * (d0 * w1) * ta) * qa;
+        const T zb = (u[s >> 1][2 + (s & 1)] - (T)2 * h1b[s] * (d1 * w1) * tb) * qb;
+        T gws = fma(x0, za, fma(d0, ta * qa, fma(x1, zb, d1 * (tb * qb)))), gbs = za + zb;
 #pragma unroll
         for (int o = 4; o < 32; o <<= 1) {
           gws += __shfl_xor_sync(0xffffffffu, gws, o);
@@ -883,41 +1029,47 @@ k_emb_rev_dmma(TrGrad<double> grad, const double* __restrict__ xbar,
     for (int half = 0; half < 2; ++half) {
       if (half) __syncthreads();
       if (ne > 0) {
-        double* p = Z + (w * 16 + gr) * EM_P1S + t4;
+        T* p = Z + (w * 16 + gr) * P1S + t4;
 #pragma unroll
         for (int s = 0; s < EM_S1; ++s) {
           const bool one = s == 6 && t4 == 1;
-          const double w1 = V[4 * s + t4];
-          p[4 * s] = half ? (1. - h1a[s] * h1a[s]) * (d0 * w1) : one ? 1. : h1a[s];
-          p[8 * EM_P1S + 4 * s] = half ? (1. - h1b[s] * h1b[s]) * (d1 * w1) : one ? 1. : h1b[s];
+          const T w1 = V[4 * s + t4];
+          p[4 * s] = half ? ((T)1 - h1a[s] * h1a[s]) * (d0 * w1) : one ? (T)1 : h1a[s];
+          p[8 * P1S + 4 * s] = half ? ((T)1 - h1b[s] * h1b[s]) * (d1 * w1) : one ? (T)1 : h1b[s];
         }
       }
       __syncthreads();
 #pragma unroll 1
       for (int v = 0; v < EM_REV_NW; ++v) {
         if (!act[v]) continue;
-        const double* ap = H + v * EM_REV_H + half * 16 * EM_P2S + t4 * EM_P2S + 16 * (w >> 1) + gr;
-        const double* bp = Z + (v * 16 + t4) * EM_P1S + 16 * (w & 1) + gr;
+        const T* ap = H + v * Ly::H + half * 16 * P2S + t4 * P2S + 16 * (w >> 1) + gr;
+        const T* bp = Z + (v * 16 + t4) * P1S + 16 * (w & 1) + gr;
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-          const double a0 = ap[4 * s * EM_P2S], a1 = ap[4 * s * EM_P2S + 8];
-          dmma16(gw2[0], a0, a1, bp[4 * s * EM_P1S]);
-          dmma16(gw2[1], a0, a1, bp[4 * s * EM_P1S + 8]);
+        for (int s = 0; s < 2; ++s) {
+          const T *aq = ap + 8 * s * P2S, *ar = aq + 4 * P2S;
+          const T *bq = bp + 8 * s * P1S, *br = bq + 4 * P1S;
+          const Op a0 = em_op(aq[0]), a1 = em_op(aq[8]), a2 = em_op(ar[0]), a3 = em_op(ar[8]);
+          em_mma(gw2[0], a0, a1, a2, a3, em_op(bq[0]), em_op(br[0]));
+          em_mma(gw2[1], a0, a1, a2, a3, em_op(bq[8]), em_op(br[8]));
         }
       }
     }
   }
   if (!any) return;
-  if (w < 7)
+  if (NJ == 2 || w < 7)
 #pragma unroll
     for (int m = 0; m < 7; ++m)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int c = 16 * m + gr + 8 * (k >> 1), p = 8 * w + 2 * t4 + (k & 1);
-        if (c >= 100 || p > 50) continue;
-        atomicAdd(p == 50 ? grad.b[t][2] + c : grad.W[t][2] + ((p >> 1) + 25 * (p & 1)) * 100 + c,
-                  gw3[m][k]);
-      }
+      for (int n = 0; n < NJ; ++n)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int c = 16 * m + gr + 8 * (k >> 1);
+          const int p = 8 * (NJ == 2 ? 2 * (w & 3) + n : w) + 2 * t4 + (k & 1);
+          if (c >= 100 || p > 50) continue;
+          atomicAdd(p == 50 ? grad.b[t][2] + c
+                            : grad.W[t][2] + ((p >> 1) + 25 * (p & 1)) * 100 + c,
+                    gw3[m][n][k]);
+        }
 #pragma unroll
   for (int n = 0; n < 2; ++n)
 #pragma unroll
@@ -931,7 +1083,7 @@ k_emb_rev_dmma(TrGrad<double> grad, const double* __restrict__ xbar,
   for (int e = threadIdx.x; e < 56; e += blockDim.x) {
     const int i = e % 28;
     if (i >= 25) continue;
-    double s = 0.;
+    T s = (T)0;
     for (int v = 0; v < EM_REV_NW; ++v) s += G1[v * 56 + e];
     atomicAdd((e < 28 ? grad.W[t][0] : grad.b[t][0]) + i, s);
   }
@@ -1009,17 +1161,18 @@ static int em_bwd(double* gem, const double* em, const double* xbar, const TrNet
   return DPB_OK;
 }
 
-static int em_rev(const TrGrad<double>& gr, const double* xb, const double* xbd, const double* avg,
-                  const double* std_, const double* fbar, const double* vbar,
-                  const TrNet<double>& net, const TrGeom& g, cudaStream_t st) {
+template <typename T>
+static int em_rev(const TrGrad<T>& gr, const T* xb, const T* xbd, const T* avg, const T* std_,
+                  const double* fbar, const double* vbar, const TrNet<T>& net, const TrGeom& g,
+                  cudaStream_t st) {
   int sms, used;
   const EmSplit sp = em_split(g, sms, used);
-  const size_t smem = (size_t)EM_REV_N * 8;
-  DPB_CUDA(cudaFuncSetAttribute(k_emb_rev_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem),
+  const size_t smem = (size_t)EmRev<T>::N * sizeof(T);
+  auto kern = k_emb_rev_mma<T>;
+  DPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
            "se_a_train_rev");
-  DPB_CUDA(launch_pdl(k_emb_rev_dmma, dim3(used), dim3(32 * EM_REV_NW), smem, st, gr, xb, xbd, avg,
-                      std_, fbar, vbar, net, g, sp),
+  DPB_CUDA(launch_pdl(kern, dim3(used), dim3(32 * EM_REV_NW), smem, st, gr, xb, xbd, avg, std_,
+                      fbar, vbar, net, g, sp),
            "se_a_train_rev");
   return DPB_OK;
 }
@@ -1046,10 +1199,9 @@ template <typename T>
 static int em_try_rev(const TrGrad<T>& gr, const T* xb, const T* xbd, const T* avg, const T* std_,
                       const double* fbar, const double* vbar, const TrNet<T>& net, const TrGeom& g,
                       cudaStream_t st) {
-  if constexpr (std::is_same_v<T, double>)
-    if (net.n1 == 25 && net.n2 == 50 && net.n3 == 100 &&
-        g.nnei + TR_MAXT + 1 <= EM_REV_Z * 2)
-      return em_rev(gr, xb, xbd, avg, std_, fbar, vbar, net, g, st);
+  if (net.n1 == 25 && net.n2 == 50 && net.n3 == 100 &&
+      (size_t)(g.nnei + TR_MAXT + 1) * 4 <= EmRev<T>::Z * sizeof(T))
+    return em_rev<T>(gr, xb, xbd, avg, std_, fbar, vbar, net, g, st);
   return -1;
 }
 
