@@ -252,9 +252,9 @@ __device__ __forceinline__ void tr_load_col(T (&a)[R], const T* base, int c) {
 // acc[r] += a[r] w for the R rows of a group. FP32 rows go two at a time (packed
 // FMA): the warp-per-atom kernels are bound by issue slots and the latency between
 // them (8 warps per SM, half of the slots, 31 % of the FMA pipe), so half the
-// instructions shorten them. 16 frames of 192 atoms: reverse pass 1774 -> 1584 us
-// (the standard net has its own, 1011), backward 494 -> 466, tangent 440 -> 402;
-// forward unchanged.
+// instructions shorten them. 16 frames of 192 atoms: backward 494 -> 466 us,
+// reverse pass 1774 -> 1584, tangent 440 -> 402 (the latter two have kernels of
+// their own for the standard net); forward unchanged.
 template <typename T, int R>
 __device__ __forceinline__ void tr_axpy(T (&acc)[R], const T (&a)[R], T w) {
   if constexpr (sizeof(T) == 4 && R % 2 == 0) {
@@ -1891,6 +1891,9 @@ using namespace dpb;
       set_error("se_a_train_tan: null buffer");                                                 \
       return DPB_ERR_INVALID;                                                                   \
     }                                                                                           \
+    rc = em_try_tan<T>(xyz_t, descrpt_t, xyz, avg, std_, force_bar, virial_bar, net, g,          \
+                       as_stream(stream));                                                      \
+    if (rc >= 0) return rc;                                                                     \
     auto kern = !tr_std_net(net) ? k_tr_tan<T, TrTraits<T>::R, 0, 0, 0>                         \
                 : (R == 4 ? k_tr_tan<T, 4, 25, 50, 100> : k_tr_tan<T, 8, 25, 50, 100>);\
     int grid;                                                                                   \
