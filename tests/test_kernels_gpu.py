@@ -379,6 +379,32 @@ def test_prod_force_virial_random(ops, port, wl, dtype):
     _close(av.cpu().numpy(), av0, dtype, "atom_virial")
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("nloc,nnei,shift", [(1, 1, 0), (5, 31, 1), (3, 33, 0), (2, 70, 3)])
+def test_prod_force_virial_rows(ops, port, dtype, nloc, nnei, shift):
+    """Lists around the 32 slots of a warp, neighbors repeated and missing, bases
+    on and off the 16-byte boundary."""
+    rng = np.random.default_rng(nnei)
+    nall = nloc + 7
+    nd = rng.normal(size=(nloc, nnei * 4)).astype(dtype)
+    ed = rng.normal(size=(nloc, nnei * 12)).astype(dtype)
+    rij = rng.normal(size=(nloc, nnei * 3)).astype(dtype)
+    nl = rng.integers(-1, nall, (nloc, nnei)).astype(np.int32)
+    tdt = torch.float64 if dtype == np.float64 else torch.float32
+
+    def dev(a):
+        buf = torch.zeros(a.size + shift, dtype=tdt, device="cuda")
+        buf[shift:] = _t(a, tdt).reshape(-1)
+        return buf[shift:].view(a.shape)
+
+    f = ops.prod_force_a(dev(nd), dev(ed), _t(nl), nloc, nall)
+    _close(f.cpu().numpy(), port.prod_force_a(nd, ed, nl, nloc, nall), dtype, "force")
+    v, av = ops.prod_virial_a(dev(nd), dev(ed), dev(rij), _t(nl), nloc, nall)
+    v0, av0 = port.prod_virial_a(nd, ed, rij, nl, nloc, nall)
+    _close(v.cpu().numpy(), v0, dtype, "virial")
+    _close(av.cpu().numpy(), av0, dtype, "atom_virial")
+
+
 def test_prod_force_virial_golden(ops, port, ref_fixtures):
     kf = "test_prod_force_a.cc:TestProdForceA:"
     kv = "test_prod_virial_a.cc:TestProdVirialA:"
