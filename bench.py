@@ -804,8 +804,10 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
     # of this workload (profiles/ncu_dram_water12288.json)
     # (matched on the name before its template arguments, which follow the
     # tile shape the autotuner picked)
-    kernel_of = {"env_mat": "dpb::k_env", "descriptor_fwd": "dpb::k_desc_fwd",
-                 "descriptor_bwd": "dpb::k_desc_bwd", "force_virial": "dpb::k_force_virial_rc"}
+    cheb = ev.ptab.nets is not None
+    desc = "dpb::k_desc_%s_cheb" if cheb else "dpb::k_desc_%s"
+    kernel_of = {"env_mat": "dpb::k_env", "descriptor_fwd": desc % "fwd",
+                 "descriptor_bwd": desc % "bwd", "force_virial": "dpb::k_force_virial_rc"}
     traffic = None
     dram_path = os.path.join(ROOT, "profiles", "ncu_dram_water12288.json")
     if nloc == 12288 and os.path.exists(dram_path):
@@ -820,13 +822,14 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
                 "algorithmic_bytes_per_launch": per_atom_bytes[dom] * nloc,
                 "algorithmic_bytes_per_atom": per_atom_bytes[dom],
                 "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"}
-    # The descriptor kernels are bound by L1/TEX serving the gathers of table
-    # rows (ncu: L1/TEX 76-85% busy, DRAM 6-7%), not by HBM: a second roof for
+    # On tables the descriptor kernels are bound by L1/TEX serving the gathers
+    # of table rows (ncu: L1/TEX 76-85% busy, DRAM 6-7%), not by HBM (the
+    # Chebyshev form gathers nothing: issue slots bound it): a second roof for
     # the dominant descriptor stage counts the algorithmic gather bytes (one
     # (degree + 1) x M FP32 coefficient row per evaluated slot: the real
     # neighbors plus one folded padding slot per type section) against the
     # nominal L1 data rate (128 B/clk/SM at the sampled SM clock).
-    if dom.startswith("descriptor"):
+    if dom.startswith("descriptor") and not cheb:
         nl = ev.nlist.view(nloc, cfg.nnei).cpu().numpy()
         sec = cfg.sec
         slots = 0
@@ -851,13 +854,13 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
                     "peak and issue 62% in k_desc_bwd, L1/TEX 85% busy in k_desc_fwd, DRAM "
                     "6-7%); the HBM fraction above is low by construction"}
     # every stage against its own roof: HBM bytes for the memory stages, the
-    # tensor pipe for the fitting GEMMs (split TF32: three or four TF32
-    # products per FP32 multiply-add, the fit_terms knob; TF32 dense peak
-    # taken as half the measured BF16 GEMM rate)
+    # tensor pipe for the fitting GEMMs (split operands: three or four
+    # products per FP32 multiply-add, the fit_terms knob; FP16 products at the
+    # measured BF16 GEMM rate, TF32 ones, fit_split_b = 1, at half of it)
     fit = cfg.fitting
     din = cfg.neuron[-1] * cfg.axis_neuron
     mac_fit = 2 * (din * fit[0] + sum(fit[k] * fit[k + 1] for k in range(len(fit) - 1)))
-    tf32_peak = float(peaks.get("bf16_tflops", 1590.0)) / 2
+    bf16_peak = float(peaks.get("bf16_tflops", 1590.0))
     stage_roofs = {}
     for k, v in stage_ms.items():
         if k in per_atom_bytes:
@@ -867,8 +870,11 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
             capi = importlib.import_module("deepmd_kit_lr_pt_b200._capi")
             terms = int(capi.lib().dpb_tune_get(b"fit_terms"))
             tf = terms * 2 * mac_fit * nloc / (v * 1e-3) / 1e12
-            stage_roofs[k] = {"bound": "tensor", "achieved_tflops_tf32": tf, "tf32_terms": terms,
-                              "peak_tflops_tf32": tf32_peak, "frac": tf / tf32_peak}
+            tf32 = int(capi.lib().dpb_tune_get(b"fit_split_b")) == 1
+            fit_peak = bf16_peak / 2 if tf32 else bf16_peak
+            stage_roofs[k] = {"bound": "tensor", "operands": "tf32" if tf32 else "fp16",
+                              "achieved_tflops": tf, "terms": terms,
+                              "peak_tflops": fit_peak, "frac": tf / fit_peak}
 
     # ---- CPU baseline: the reference CPU path on a bounded sample (rank 0, N=1)
     cpu = None

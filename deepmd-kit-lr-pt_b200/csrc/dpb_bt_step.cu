@@ -1,18 +1,19 @@
-// One batched-frames step as ONE persistent cooperative launch (one CTA per
-// SM, 18 warps), its passes separated by grid-wide barriers:
+// One batched-frames step as ONE persistent cooperative launch (one CTA of 16
+// warps per SM), its passes separated by grid-wide barriers:
 //
 //   P0  force / virial / atomic-energy accumulators zeroed; every frame's
 //       positions wrapped and binned into its cells (one CTA per frame)
 //   P1  one warp per center row: the env row and neighbor list over the 27
 //       lattice cells (bt_env_row), then at once the row's compressed
-//       embedding, contraction and descriptor (desc_fwd_atom), reading the env
+//       embedding, contraction and descriptor (desc_fwd_atom, or with
+//       Chebyshev nets cheb_fwd_group by groups of 8 warps), reading the env
 //       row just written from L2
 //   P2-P7 the six fitting GEMMs on the tensor cores (gemm_run: TMA ring,
-//       TF32 hi / lo split into TMEM, tcgen05.mma, fused epilogues), the
+//       FP16 hi / lo split into TMEM, tcgen05.mma, fused epilogues), the
 //       80-column tiles with chunked accumulation; tensor memory is allocated
 //       once for the whole launch
 //   P8  one CTA per frame: the frame's energy in FP64; then one warp per row:
-//       the descriptor backward (desc_bwd_atom) and at once the row's forces
+//       the descriptor backward (desc_bwd_atom / cheb_bwd_group) and at once the row's forces
 //       and virial (bt_force_row), reading net_deriv just written from L2
 //
 // The same device bodies as the per-stage kernels (dpb_batch.cu, dpb_se_a.cu,

@@ -4,8 +4,13 @@
 //
 //   C[m, n] = sum_k A[m, k] B[n, k]      A: [M, K] FP32 row-major (activations)
 //                                        B: [N, K] FP32 row-major (weights),
-//                                           given pre-split into TF32 hi / lo,
-//                                           or in FP32 and split in the kernel
+//                                           given pre-split into FP16 or TF32
+//                                           hi / lo, or in FP32 and split in
+//                                           the kernel
+// Two operand forms. The evaluators use the FP16 one (dpb_f16split.cuh: terms
+// scaled by powers of two, dpb_gemm_f16x3_f32; twice the TF32 rate), training
+// and fit_split_b = 1 the TF32 one described here; tiles, ring and epilogues are
+// shared (GemmCfg::F16).
 // Split TF32: A = Ah + Al and B = Bh + Bl with Ah, Bh the TF32 roundings and
 // Al, Bl the TF32 roundings of the remainders (so A and B are represented to
 // 2^-24 relative, FP32 resolution); the product is Ah Bh + Al Bh + Ah Bl

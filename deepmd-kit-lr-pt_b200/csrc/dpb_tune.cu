@@ -19,19 +19,19 @@ static Knob g_knobs[] = {
     // warps (one center atom each) per CTA of the fused descriptor kernels
     {"desc_atoms_per_cta", 4, 3, {2, 4, 8}},
     // L1 policy of the table-coefficient loads in the fused descriptor
-    // kernels: 0 default, 1 no_allocate, 2 evict_first, 3 evict_last (measured
+    // kernels on tables (not the Chebyshev form): 0 default, 1 no_allocate, 2 evict_first, 3 evict_last (measured
     // fastest on 12,288-atom water: rows near the switch cutoff are shared),
     // 4 evict_last in L1 and L2
     {"desc_coef_l1", 3, 5, {0, 1, 2, 3, 4}},
     // widest tensor-core tile of the fitting GEMMs (a width is used where it
     // divides N; 240 only for K <= 512)
     {"fit_n_tile", 160, 3, {80, 160, 240}},
-    // fitting GEMM weights: 0 pre-split TF32 hi / lo read from L2, 1 FP32
-    // read and split in shared memory by four dedicated warps (half the
-    // weight bytes; 14% slower on the 12,288-atom water step: the GEMMs are
-    // not limited by the weight bytes)
+    // fitting GEMM weights: 0 pre-split hi / lo read from L2 (FP16 in the
+    // evaluators, TF32 in training), 1 FP32 read and split into TF32 in shared
+    // memory by four dedicated warps (half the TF32 weight bytes; 14% slower
+    // than pre-split TF32 on the 12,288-atom water step)
     {"fit_split_b", 0, 2, {0, 1}},
-    // TF32 products per k step of the fitting GEMM: 3 (Ah Bh + Al Bh + Ah Bl)
+    // products per k step of the fitting GEMM: 3 (Ah Bh + Al Bh + Ah Bl)
     // or 4 (with Al Bl, 2^-22 of a product: measured to change no output
     // beyond FP32 accumulation noise, at 4% more fitting time)
     {"fit_terms", 3, 2, {3, 4}},
@@ -39,8 +39,8 @@ static Knob g_knobs[] = {
     // accumulator per output tile: the tensor cores' FP32 accumulation loses
     // up to an ulp of the running sum per instruction, always in the same
     // direction, so long sums over rows that are alike drift
-    // (measured, 12,288-atom water fitting stage / worst Cu-frame energy
-    // error: 0 298 us / 1.4e-6 eV/atom; 8 k-block order 302 us / 2.3e-7;
+    // (measured on the TF32 form, 12,288-atom water fitting stage / worst
+    // Cu-frame energy error: 0 298 us / 1.4e-6 eV/atom; 8 k-block order 302 us / 2.3e-7;
     // 4 k-block order 320 us / 1.1e-7; 4 cross first 345 us / 3.1e-8)
     {"fit_kchunk", 8, 5, {0, 1, 2, 4, 8}},
     // order inside a chunk: 1 the cross products of all its k-blocks first
@@ -61,29 +61,32 @@ static Knob g_knobs[] = {
     // descriptor backward and the forces) as separate passes, 0 back to back
     // per row in one pass
     {"batch_fused_split", 0, 2, {0, 1}},
-    // neighbor rows per group in the FP32 training kernels
+    // neighbor rows per group in the FP32 training kernels on the FMA pipe
+    // (forward and backward; tangent and reverse too for other nets than
+    // 25-50-100)
     {"train_rows_per_group", 8, 2, {4, 8}},
-    // the same for the FP64 force-backward kernel (also the embedding
-    // backward of the FP64 plain evaluation path)
+    // the same for the FP64 force-backward kernel of nets that the matrix
+    // form does not take
     {"train_rows_per_group_f64", 8, 2, {4, 8}},
     // most warps per CTA of the training kernels (fewer when shared memory
     // does not allow them)
     {"train_warps_per_cta", 8, 4, {1, 2, 4, 8}},
-    // reverse training kernel: one weight-gradient copy per block, updated
-    // with shared-memory atomics, so 8 warps fit instead of 4 (measured: FP32
-    // step 4.19 -> 4.01 ms, FP64 step 15.4 -> 12.8 ms, same gradients)
+    // reverse training kernel of other nets than 25-50-100: one
+    // weight-gradient copy per block, updated with shared-memory atomics, so 8
+    // warps fit instead of 4 (measured on the standard net before it had its
+    // own kernel: FP32 step 4.19 -> 4.01 ms, FP64 step 15.4 -> 12.8 ms)
     {"train_rev_shared_acc", 1, 2, {0, 1}},
     // one frame's wrap / ghost copy / cell grid: 1 one cooperative launch,
     // 0 the separate kernels
     {"geometry_fused", 1, 2, {0, 1}},
-    // contraction of the fused descriptor forward: 0 FP32 CUDA cores (packed
+    // contraction of the fused descriptor forward on tables: 0 FP32 CUDA cores (packed
     // FMA on the table values in registers), 1 tensor cores (mma.sync
     // m16n8k8, 3xTF32; the table values are evaluated in the MMA fragment
     // layout). Measured on 12,288-atom water: 172 us (0) against 342 us (1),
     // so 1 is a tested option the autotuner does not try
     // (the kernel is bound by the table gathers, which 1 makes scalar)
     {"desc_tc", 0, 2, {0, 1}},
-    // SIMT GEMMs (FP64 plain path and training, FP32 odd widths): 1 the
+    // SIMT GEMMs (FP32, odd widths; FP64 has its matrix form): 1 the
     // 128 x 64 tile with 8 x 4 outputs per thread where M >= 128, 0 the
     // 64 x 64 tile with 4 x 4 outputs
     {"gemm_simt_big", 1, 2, {0, 1}},
