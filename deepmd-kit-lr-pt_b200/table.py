@@ -269,21 +269,24 @@ def chebyshev_net(table: np.ndarray, info: np.ndarray, tol: float = 1.5e-8,
     if (first < 1 or first > table.shape[0] or abs(first * s0 - (upper - lower)) > 1e-9 or
             ncell != round(ncell) or not 1 <= ncell <= 1 << 16):
         return None
-    T = np.asarray(table[:first], np.float64).reshape(first, M, 6)
+    # coefficient by coefficient: each [first, M] contiguous
+    T = np.ascontiguousarray(np.asarray(table[:first], np.float64).reshape(first, M, 6)
+                             .transpose(2, 0, 1))
 
-    def poly(rows, t):
-        c = T[rows]
-        t = t[:, None]
-        v, g = c[..., 5], 5.0 * c[..., 5]
+    def value(rows, t):
+        v = T[5, rows]
         for p in range(4, -1, -1):
-            v = v * t + c[..., p]
-        for p in range(4, 0, -1):
-            g = g * t + p * c[..., p]
-        return v, g
+            v = v * t
+            v += T[p, rows]
+        return v
 
-    knots = np.arange(first)
-    zero, half = np.zeros(first), np.full(first, 0.5 * s0)
-    ref = [poly(knots, zero), poly(knots, half)]
+    # value and slope at the knots and at the midpoints
+    every, mid = slice(None), 0.5 * s0
+    slope = 5.0 * T[5]
+    for p in range(4, 0, -1):
+        slope *= mid
+        slope += p * T[p]
+    ref = [(T[0], T[1]), (value(every, mid), slope)]
     big = max(np.abs(v).max() for v, _ in ref)
     steep = max(np.abs(g).max() for _, g in ref)
     if not (np.isfinite(big) and np.isfinite(steep)) or big == 0.0:
@@ -298,7 +301,7 @@ def chebyshev_net(table: np.ndarray, info: np.ndarray, tol: float = 1.5e-8,
         c, h = 0.5 * (a + b), 0.5 * (b - a)
         x = c + h * node
         r = np.clip(((x - lower) / s0).astype(np.int64), 0, first - 1)
-        C = dct @ poly(r, x - (lower + r * s0))[0]
+        C = dct @ value(r, (x - (lower + r * s0))[:, None])
         for off, (v, g) in zip((0.0, 0.5 * s0), ref):
             i0 = int(np.ceil((a - lower - off) / s0 - 1e-9))
             i1 = int(np.ceil((b - lower - off) / s0 - 1e-9))
@@ -309,8 +312,14 @@ def chebyshev_net(table: np.ndarray, info: np.ndarray, tol: float = 1.5e-8,
                 P.append(2 * t * P[-1] - P[-2])
                 U.append(2 * t * U[-1] - U[-2])
             dP = np.stack([np.zeros_like(t)] + [q * U[q - 1] for q in range(1, CHEB_K)], 1)
-            if i1 > i0 and (np.abs(np.stack(P, 1) @ C - v[i0:i1]).max() > tol * big or
-                            np.abs(dP @ C / h - g[i0:i1]).max() > tol_slope * steep):
+
+            def off_by(Q, want):
+                e = Q @ C
+                e -= want[i0:i1]
+                return max(e.max(), -e.min())
+
+            if i1 > i0 and (off_by(np.stack(P, 1), v) > tol * big or
+                            off_by(dP / h, g) > tol_slope * steep):
                 return None
         return C
 
