@@ -262,11 +262,18 @@ class PipelineTables:
         self.bwd = "dpb_se_a_descriptor_bwd" + sfx
         # the intervals each group of eight rows uses, from forward to backward
         self.touched = None
+        self.rows = int(rows)
         if self.nets is not None:
             self.touched = torch.zeros((max(rows, 1) + 7) // 8 * len(self.tabs),
                                        dtype=torch.int32, device=dev)
         # operand scales of the descriptor rows, written by the forward
         self.row_scale = torch.ones(max(rows, 1), device=dev)
+
+    def _check_rows(self, n: int) -> None:
+        # the kernels write touched and row_scale by row and know no capacity
+        if n > self.rows:
+            raise _capi.DPBInvalidArgument(
+                f"PipelineTables: a pass over {n} rows, made for at most {self.rows}")
 
     def _cheb_nets(self, params: SeAParams, dev):
         """Host array of dpb_cheb_net, or None when a net does not expand."""
@@ -295,6 +302,7 @@ class PipelineTables:
 
     def forward(self, xyz, D, drow, em, sec: np.ndarray, n: int, M: int, ax: int, s):
         """xyz and the descriptor rows of n centers from their env rows."""
+        self._check_rows(n)
         if self.nets is None:
             call(self.fwd, ptr(xyz), ptr(D), ptr(drow), ptr(em), self.ptrs,
                  self.info.ctypes.data, sec.ctypes.data, sec.size, n, M, ax, s)
@@ -306,6 +314,7 @@ class PipelineTables:
 
     def backward(self, net_deriv, dD, drow, xyz, em, sec: np.ndarray, n: int, M: int, ax: int, s):
         """net_deriv = dE/d(em) of the rows of the last forward."""
+        self._check_rows(n)
         if self.nets is None:
             call(self.bwd, ptr(net_deriv), ptr(dD), ptr(drow), ptr(xyz), ptr(em), self.ptrs,
                  self.info.ctypes.data, sec.ctypes.data, sec.size, n, M, ax, s)
