@@ -109,6 +109,8 @@ _FUNCS = {
     "dpb_se_a_descriptor_bwd_cubic_f32": "ppppp" "pp" "pi" "iiip",
     "dpb_se_a_descriptor_fwd_cheb_f32": "pppp" "ppppp" "pi" "iiip",
     "dpb_gemm_f16x3_f32": "piipppp" "ipii" "pppp" "pppp" "pp",
+    "dpb_gemm_f16x3_rows_f32": "piippppp" "ipii" "pppp" "pppp" "pp",
+    "dpb_bt_step_set_b_inv": "pp",
     "dpb_se_a_descriptor_bwd_cheb_f32": "ppppp" "pppp" "pi" "iiip",
     "dpb_bt_step_set_nets": "ppppppp",
     "dpb_se_a_row_scale_f32": "pppiip",

@@ -220,9 +220,10 @@ class BatchEvaluator:
         handle = ctypes.c_void_p()
         call("dpb_bt_step_create", ctypes.byref(handle), ctypes.byref(d))
         if pt.nets is not None:
-            b, a_scale, b_scale = fit.f16_layers()
+            b, a_scale, b_scale, b_inv = fit.f16_layers()
             call("dpb_bt_step_set_nets", handle, pt.nets, ptr(pt.touched), ptr(pt.row_scale), b,
                  a_scale.ctypes.data, b_scale.ctypes.data)
+            call("dpb_bt_step_set_b_inv", handle, b_inv)
         self._split = _capi.lib().dpb_tune_get(b"batch_fused_split") != 0
         self.plan = handle
 

@@ -583,6 +583,23 @@ int dpb_bt_step_set_nets(void* plan, const dpb_cheb_net* nets, unsigned* touched
   return DPB_OK;
 }
 
+int dpb_bt_step_set_b_inv(void* plan, const float* const* b_inv) {
+  BtStepPlan* p = static_cast<BtStepPlan*>(plan);
+  if (p == nullptr || !p->cheb || b_inv == nullptr) {
+    set_error("bt_step_set_b_inv: needs a plan with nets, and the reciprocals");
+    return DPB_ERR_INVALID;
+  }
+  for (int l = 0, o = 0; l < BS_PASSES; ++l)
+    for (int t = 0; t < p->a.shp[l].ntypes; ++t, ++o) {
+      if (b_inv[o] == nullptr || ((uintptr_t)b_inv[o] & 15) != 0) {
+        set_error("bt_step_set_b_inv: the reciprocals must be 16-byte aligned");
+        return DPB_ERR_INVALID;
+      }
+      p->a.epi[l].b_inv[t] = b_inv[o];
+    }
+  return DPB_OK;
+}
+
 int dpb_bt_step_launch(const void* plan, dpb_stream_t stream) {
   if (plan == nullptr) {
     set_error("bt_step: no plan");

@@ -22,8 +22,8 @@
 //
 // FP32 operands are split into two FP16 terms, hi + lo, after scaling by a
 // power of two (per atom and type from a bound of the row; per net for C), so
-// that hi + lo holds 22-23 significant bits for every value within 2^-28 of
-// the largest; the product is lo hi + hi lo + hi hi accumulated in FP32 from
+// that hi + lo holds 23 bits of every value down to 2^-16 of the largest and
+// 2^-39 of the largest below that (dpb_f16split.cuh); the product is lo hi + hi lo + hi hi accumulated in FP32 from
 // zero for each interval (16 k), and the intervals are added in FP32 outside
 // the tensor cores, whose own accumulation truncates.
 //

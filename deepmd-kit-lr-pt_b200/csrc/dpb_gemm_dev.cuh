@@ -103,10 +103,12 @@ struct GemmEpi {
   const float* w[GT_MAXT];
   float* e;
   // FP16 form: power-of-two scale of A's rows per type (times row_scale[row]
-  // where given) and its product's reciprocal with the weights' scale
+  // where given) and its product's reciprocal with the weights' scale; b_inv:
+  // where given, a further reciprocal per weight row (output column)
   const float* row_scale;
   float a_scale[GT_MAXT];
   float inv_scale[GT_MAXT];
+  const float* b_inv[GT_MAXT];
 };
 
 struct GemmShape {
@@ -706,8 +708,10 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
       const float* idt = epi.idt[tc.ty];
       const float* wv = epi.w[tc.ty];
       float inv = 1.f;
+      const float* b_inv = nullptr;
       if constexpr (F16) {
         inv = epi.inv_scale[tc.ty];
+        b_inv = epi.b_inv[tc.ty];
         if (epi.row_scale != nullptr && ok) inv /= __ldg(epi.row_scale + row);  // powers of two
       }
       constexpr bool NEED0 = MODE >= EPI_RES_DT, NEED1 = MODE == EPI_BWD_RES;
@@ -732,6 +736,15 @@ __device__ __forceinline__ void gemm_run(const GemmMaps& maps, const GemmShape& 
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int cj = n0 + c0 + 4 * j;
+          if constexpr (F16) {
+            if (b_inv != nullptr) {
+              const float4 s = __ldg(reinterpret_cast<const float4*>(b_inv + cj));
+              v[4 * j] *= s.x;
+              v[4 * j + 1] *= s.y;
+              v[4 * j + 2] *= s.z;
+              v[4 * j + 3] *= s.w;
+            }
+          }
           float4 bb = make_float4(0.f, 0.f, 0.f, 0.f), dd = bb, ww = bb;
           if (MODE == EPI_TANH || MODE == EPI_RES_DT || MODE == EPI_LAST)
             bb = __ldg(reinterpret_cast<const float4*>(bias + cj));

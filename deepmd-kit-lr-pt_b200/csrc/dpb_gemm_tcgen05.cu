@@ -351,7 +351,22 @@ int dpb_gemm_f16x3_f32(const float* A, int M, int K, const float* row_scale,
                        const float* aux0, const float* aux1, const float* const* bias,
                        const float* const* idt, const float* const* w, float* e, int* status,
                        dpb_stream_t stream) {
-  if (status == nullptr || a_scale == nullptr || b_scale == nullptr) {
+  if (b_scale == nullptr) {
+    set_error("gemm_f16x3: the operand scales are required");
+    return DPB_ERR_INVALID;
+  }
+  return dpb_gemm_f16x3_rows_f32(A, M, K, row_scale, a_scale, b, b_scale, nullptr, N, type_rows,
+                                 ntypes, mode, out0, out1, aux0, aux1, bias, idt, w, e, status,
+                                 stream);
+}
+
+int dpb_gemm_f16x3_rows_f32(const float* A, int M, int K, const float* row_scale,
+                            const float* a_scale, const void* const* b, const float* b_scale,
+                            const float* const* b_inv, int N, const int* type_rows, int ntypes,
+                            int mode, float* out0, float* out1, const float* aux0,
+                            const float* aux1, const float* const* bias, const float* const* idt,
+                            const float* const* w, float* e, int* status, dpb_stream_t stream) {
+  if (status == nullptr || a_scale == nullptr || (b_scale == nullptr && b_inv == nullptr)) {
     set_error("gemm_f16x3: a status word and the operand scales are required");
     return DPB_ERR_INVALID;
   }
@@ -367,7 +382,12 @@ int dpb_gemm_f16x3_f32(const float* A, int M, int K, const float* row_scale,
   ep.row_scale = row_scale;
   for (int t = 0; t < ntypes; ++t) {
     ep.a_scale[t] = a_scale[t];
-    ep.inv_scale[t] = 1.f / (a_scale[t] * b_scale[t]);
+    ep.inv_scale[t] = 1.f / (a_scale[t] * (b_scale ? b_scale[t] : 1.f));
+    ep.b_inv[t] = b_inv ? b_inv[t] : nullptr;
+    if (((uintptr_t)ep.b_inv[t] & 15) != 0) {
+      set_error("gemm_f16x3: b_inv must be 16-byte aligned");
+      return DPB_ERR_INVALID;
+    }
   }
   cudaStream_t st = as_stream(stream);
   if (BN == CfgH240::BN) return launch<CfgH240>(maps, shp, ep, status, st);

@@ -479,33 +479,44 @@ class _FittingTC:
         return self._tf32[name]
 
     def f16(self, name):
-        """(pointer array, scales) of the weights ``name`` as FP16 pairs."""
+        """(pairs, reciprocals of the row scales) of the weights ``name``,
+        pointer arrays by type. Every row has its own power of two, which
+        brings its largest entry to 2^13 .. 2^14: with one per matrix an output
+        whose weights are small beside another's lost bits (2^-39 of the largest
+        is what a pair resolves)."""
         if name not in self._f16:
-            ts, scales = [], []
+            ts, inv = [], []
             for m in self._mats[name]:
-                w = torch.tensor(np.ascontiguousarray(m, np.float32), device=self.dev)
-                scale = 2.0 ** (14 - int(np.ceil(np.log2(max(float(np.abs(m).max()), 1e-30)))))
-                w = torch.nn.functional.pad(w * scale, (0, -w.shape[1] % 32))
+                m = np.ascontiguousarray(m, np.float32)
+                big = np.abs(m).max(1)
+                if not np.isfinite(big).all():
+                    big = np.where(np.isfinite(m), np.abs(m), np.float32(0)).max(1)
+                e = np.clip(np.frexp(big)[1], -112, 128)  # big < 2^e
+                one = np.ones(e.size, np.float32)
+                scale = torch.tensor(np.ldexp(one, 14 - e), device=self.dev)
+                w = torch.nn.functional.pad(torch.tensor(m, device=self.dev) * scale[:, None],
+                                            (0, -m.shape[1] % 32))
                 hi = w.half()
                 pair = torch.stack([x.view(w.shape[0], -1, 32) for x in
                                     (hi, (w - hi.float()).half())], 2)
                 ts.append(pair.contiguous())
-                scales.append(scale)
-            self._keep.extend(ts)
-            self._f16[name] = ((ctypes.c_void_p * len(ts))(*[t.data_ptr() for t in ts]),
-                               np.array(scales, np.float32))
+                inv.append(torch.tensor(np.ldexp(one, e - 14), device=self.dev))
+            self._keep.extend(ts + inv)
+            self._f16[name] = tuple((ctypes.c_void_p * len(x))(*[t.data_ptr() for t in x])
+                                    for x in (ts, inv))
         return self._f16[name]
 
     def f16_layers(self):
-        """(weights, A scales, weight scales) of the six GEMMs in order, flat:
-        the arguments of dpb_bt_step_set_nets."""
+        """(weights, A scales, weight scales, reciprocals of their row scales) of
+        the six GEMMs in order, flat: the arguments of dpb_bt_step_set_nets and
+        dpb_bt_step_set_b_inv."""
         names = (("1f", None), ("2f", "H1"), ("3f", "H2"), ("3b", "G3"), ("2b", "G2"),
                  ("1b", "G1"))
-        b = [p for n, _ in names for p in self.f16(n)[0]]
+        b, inv = ([p for n, _ in names for p in self.f16(n)[k]] for k in range(2))
         one = np.ones(self.ntypes, np.float32)
         a = np.concatenate([one if k is None else self._scales[k] for _, k in names])
         return ((ctypes.c_void_p * len(b))(*b), np.ascontiguousarray(a),
-                np.concatenate([self.f16(n)[1] for n, _ in names]))
+                np.ones(6 * self.ntypes, np.float32), (ctypes.c_void_p * len(inv))(*inv))
 
     @staticmethod
     def _operand_scales(params):
@@ -529,9 +540,9 @@ class _FittingTC:
     def _gemm(self, A, K, name, N, mode, out0, out1=None, aux0=None, aux1=None, bias=None,
               idt=None, w=None, s=None, scale=None, row_scale=None):
         if scale is not None:
-            b, bs = self.f16(name)
-            call("dpb_gemm_f16x3_f32", ptr(A), self.n, K, ptr(row_scale), scale.ctypes.data, b,
-                 bs.ctypes.data, N, self.type_rows.ctypes.data, self.ntypes, mode, ptr(out0),
+            b, inv = self.f16(name)
+            call("dpb_gemm_f16x3_rows_f32", ptr(A), self.n, K, ptr(row_scale), scale.ctypes.data,
+                 b, None, inv, N, self.type_rows.ctypes.data, self.ntypes, mode, ptr(out0),
                  ptr(out1), ptr(aux0), ptr(aux1), bias, idt, w, ptr(self.e), ptr(self.status), s)
             return
         B = self.tf32(name)

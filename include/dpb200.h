@@ -513,6 +513,10 @@ DPB_API int dpb_bt_step_create(void** plan, const dpb_bt_step_desc* desc);
 DPB_API int dpb_bt_step_set_nets(void* plan, const dpb_cheb_net* nets, unsigned* touched,
                                  float* row_scale, const void* const* b, const float* a_scale,
                                  const float* b_scale);
+/* Reciprocals of the FP16 weights' scales per row, as b_inv of
+ * dpb_gemm_f16x3_rows_f32: ntypes device arrays for each of the six GEMMs, after
+ * dpb_bt_step_set_nets. */
+DPB_API int dpb_bt_step_set_b_inv(void* plan, const float* const* b_inv);
 /* One step: env, descriptor, fitting, descriptor backward, forces, virials
  * and energies of every frame in ONE cooperative launch (one CTA per SM),
  * preceded by a 32-byte memset of the barrier and work counters. */
@@ -675,8 +679,8 @@ DPB_API int dpb_gemm_tf32x3_f32(const float* A, int M, int K,
                                 const float* const* idt, const float* const* w,
                                 float* e, int* status, dpb_stream_t stream);
 /* The same GEMM and epilogues with the operands as two FP16 terms (three
- * products, twice the tensor-core rate of TF32 at the same 22-23 significant
- * bits). Row r of A, of type t, is multiplied by a_scale[t] (host, a power of
+ * products, twice the tensor-core rate of TF32): a scaled value v is held to
+ * max(2^-23 |v|, 2^-25). Row r of A, of type t, is multiplied by a_scale[t] (host, a power of
  * two) and, where row_scale (device [M], powers of two) is not NULL, by
  * row_scale[r]; the scaled values must stay below 2^15. b (host array of
  * device pointers): B[n, k] * b_scale[t] as halves, per row n and block of 32 k
@@ -688,6 +692,18 @@ DPB_API int dpb_gemm_f16x3_f32(const float* A, int M, int K, const float* row_sc
                                const float* const* bias, const float* const* idt,
                                const float* const* w, float* e, int* status,
                                dpb_stream_t stream);
+/* The same with weights whose rows have scales of their own: b holds
+ * B[n, k] * b_scale[t] / b_inv[t][n] (b_scale may be NULL: 1; b_inv: device
+ * [N] per type, powers of two, may be NULL: 1). Rows of very different size then
+ * keep their bits. */
+DPB_API int dpb_gemm_f16x3_rows_f32(const float* A, int M, int K, const float* row_scale,
+                                    const float* a_scale, const void* const* b,
+                                    const float* b_scale, const float* const* b_inv, int N,
+                                    const int* type_rows, int ntypes, int mode, float* out0,
+                                    float* out1, const float* aux0, const float* aux1,
+                                    const float* const* bias, const float* const* idt,
+                                    const float* const* w, float* e, int* status,
+                                    dpb_stream_t stream);
 /* energy[0] = e_const + sum of e[0, n) in FP64 (fixed summation order), then
  * e[0, n) = 0: the per-row energies the mode-3 epilogue accumulates, reduced
  * and cleared for the next step's accumulation. work: device buffer of
