@@ -534,7 +534,8 @@ class _FittingTC:
             g1 = g2 + np.abs(W2) @ z2
             for key, b in (("H1", 1.0), ("H2", 1.0 + np.abs(d2).max()), ("G3", g3.max()),
                            ("G2", z2.max()), ("G1", g1.max())):
-                out[key].append(2.0 ** (13 - int(np.ceil(np.log2(max(float(b), 1e-30))))))
+                e = int(np.frexp(float(b))[1]) if np.isfinite(b) else 0  # b < 2^e
+                out[key].append(2.0 ** (13 - min(max(e, -112), 128)))
         return {k: np.array(v, np.float32) for k, v in out.items()}
 
     def _gemm(self, A, K, name, N, mode, out0, out1=None, aux0=None, aux1=None, bias=None,
