@@ -463,9 +463,17 @@ class _FittingTC:
         self.esum_work = torch.zeros(int(_capi.lib().dpb_fit_energy_sum_work_bytes()),
                                      dtype=torch.uint8, device=dev)
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
+        # the weights in the form that the steps take, complete before the first
+        # of them: it may come on another stream, or under capture, where nothing
+        # can be uploaded
+        pack = self.tf32 if _capi.lib().dpb_tune_get(b"fit_split_b") == 1 else self.f16
+        for name in self._mats:
+            pack(name)
+        torch.cuda.current_stream(dev).synchronize()
 
-    # Weights in the GEMMs' layouts, made on first use: TF32 hi / lo (or FP32 for
-    # the fit_split_b knob) and the FP16 pairs of dpb_gemm_f16x3_f32.
+    # Weights in the GEMMs' layouts: TF32 hi / lo (or FP32 for the fit_split_b
+    # knob) and the FP16 pairs of dpb_gemm_f16x3_rows_f32; the form that the
+    # constructor did not make is made on first use.
     def tf32(self, name):
         """(hi, lo, fp32) pointer arrays of the weights ``name``."""
         if name not in self._tf32:
