@@ -94,6 +94,30 @@ __device__ __forceinline__ int fold_start(const T* em_x, const T* em, int nnei, 
   return nnei;
 }
 
+template <typename T>
+struct Coef {
+  T a0, a1, a2, a3, a4, a5;
+};
+
+__device__ __forceinline__ Coef<float> load_coef(const float* p) {
+  const float2* q = reinterpret_cast<const float2*>(p);
+  float2 x = __ldg(q), y = __ldg(q + 1), z = __ldg(q + 2);
+  return {x.x, x.y, y.x, y.y, z.x, z.y};
+}
+__device__ __forceinline__ Coef<double> load_coef(const double* p) {
+  const double2* q = reinterpret_cast<const double2*>(p);
+  double2 x = __ldg(q), y = __ldg(q + 1), z = __ldg(q + 2);
+  return {x.x, x.y, y.x, y.y, z.x, z.y};
+}
+
+// value (with extrapolation) and derivative of the quintic (tabulate.cc:116-144)
+template <typename T>
+__device__ __forceinline__ void poly(const Coef<T>& a, T xx, T delta, T& v, T& g) {
+  g = a.a1 + ((T)2. * a.a2 + ((T)3. * a.a3 + ((T)4. * a.a4 + (T)5. * a.a5 * xx) * xx) * xx) * xx;
+  v = a.a0 + (a.a1 + (a.a2 + (a.a3 + (a.a4 + a.a5 * xx) * xx) * xx) * xx) * xx;
+  v = v + g * delta;
+}
+
 constexpr int TW = 4;     // warps per block
 constexpr int TB = 64;    // channels per warp
 constexpr int TP = 6;     // coefficient pairs per lane (3 TB / 32)
@@ -172,23 +196,89 @@ __device__ __forceinline__ void load_row(typename Pair<T>::type (&a)[TP], const 
   }
 }
 
+// An extrapolation so long (or x so odd: infinite, NaN) that the weighted
+// coefficients could overflow one by one, with signs of their own, where
+// v + g delta does not
+template <typename T>
+__device__ __forceinline__ bool far_x(T x) {
+  return !(fabs(x) <= (sizeof(T) == 4 ? (T)1e18 : (T)1e150));
+}
+
 // one slot per lane: its row and the weights w_k of the value (with the linear
-// extrapolation, tabulate.cc:116-144: v + g delta) and dw_k of the slope
+// extrapolation, tabulate.cc:116-144: v + g delta) and dw_k of the slope; of a far
+// slot, some finite ones
 template <typename T>
 __device__ __forceinline__ int stage_weights(T* sw, const TabInfo<T>& ti, T x, int lane) {
   int idx;
   T t, delta;
-  locate(ti, x, idx, t, delta);
+  locate(ti, far_x(x) ? ti.lower : x, idx, t, delta);
   T p = (T)1, d = (T)0;  // t^k, k t^(k - 1)
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
-    sw[lane * TS + k] = d != (T)0 ? p + delta * d : p;  // an infinite delta stays out of
-                                                        // the powers that have no slope
+    sw[lane * TS + k] = p + delta * d;
     sw[lane * TS + 6 + k] = d;
     d = (T)(k + 1) * p;
     p *= t;
   }
   return idx;
+}
+
+// The far slots of an atom, added to its finished results (all pointers at the
+// atom's rows; o and tab at the block of nc channels). Apart from the loop over
+// the slots, where a test cost 3 to 5 %; this way it costs up to 1 %.
+template <typename T, bool GG>
+__device__ __forceinline__ void fwd_far(T* o, const T* tab, TabInfo<T> ti, const T* ex, const T* ee,
+                                     int nnei, int M, int nc, int brk, int last, const T* dzx,
+                                     const T* dze, int lane) {
+  for (int j = 0; j <= last; ++j) {
+    int idx;
+    T t, delta;
+    if (!far_x(ex[j])) continue;
+    locate(ti, ex[j], idx, t, delta);
+    const T rep = j == brk ? (T)(nnei - j) : (T)1;
+#pragma unroll 1
+    for (int c = lane; c < nc; c += 32) {
+      T v, g;
+      poly(load_coef(tab + ((size_t)idx * M + c) * 6), t, delta, v, g);
+      for (int k = 0; k < 4; ++k)
+        o[k * M + c] += GG ? rep * (v * dze[j * 4 + k] + dzx[j] * g * ee[j * 4 + k])
+                           : rep * v * ee[j * 4 + k];
+    }
+  }
+}
+
+template <typename T>
+__device__ __noinline__ void grad_far(T* ox, T* oe, const T* table, TabInfo<T> ti, const T* ex,
+                                      const T* ee, const T* dy, int nnei, int M, int brk, int last,
+                                      int lane) {
+  for (int j = 0; j <= last; ++j) {
+    int idx;
+    T t, delta;
+    if (!far_x(ex[j])) continue;
+    locate(ti, ex[j], idx, t, delta);
+    T V[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
+    for (int c = lane; c < M; c += 32) {
+      T v, g;
+      poly(load_coef(table + ((size_t)idx * M + c) * 6), t, delta, v, g);
+      T s = (T)0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const T y = dy[k * M + c];
+        s += ee[j * 4 + k] * y;
+        V[k + 1] += v * y;
+      }
+      V[0] += g * s;
+    }
+    const T rep = j == brk ? (T)(nnei - j) : (T)1;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) V[k] = rep * warp_sum(V[k]);
+    __syncwarp();  // after what the kernel's loop stored here
+    if (lane == 0) {
+      ox[j] = V[0];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) oe[j * 4 + k] = V[k + 1];
+    }
+  }
 }
 
 // out[i,k,m] = sum_jj w_jj * (G_m(x_jj) * em[jj,k])              (forward)
@@ -220,10 +310,12 @@ k_tab_fwd(T* __restrict__ out, const T* __restrict__ table, TabInfo<T> ti,
   const T* ee = em + (size_t)i * nnei * 4;
   const int brk = fold_start(ex, ee, nnei, lane);
   const int last = brk < nnei ? brk : nnei - 1;
+  bool far = false;  // this lane has had a far slot
   for (int base = 0; base <= last; base += 32) {
     const int cnt = min(32, last + 1 - base), jj = base + lane;
     if (lane < cnt) {
       const T rep = jj == brk ? (T)(nnei - jj) : (T)1;
+      far |= far_x(ex[jj]);
       s_row[w][lane] = stage_weights(s_w[w], ti, ex[jj], lane);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -235,6 +327,8 @@ k_tab_fwd(T* __restrict__ out, const T* __restrict__ table, TabInfo<T> ti,
           s_e[w][lane * 4 + k] = rep * ee[jj * 4 + k];
         }
       }
+      if (far_x(ex[jj]))
+        for (int k = 0; k < (GG ? 8 : 4); ++k) s_e[w][lane * (GG ? 8 : 4) + k] = (T)0;
     }
     __syncwarp();
     const T* tab = table + (size_t)m0 * 6;
@@ -286,6 +380,9 @@ k_tab_fwd(T* __restrict__ out, const T* __restrict__ table, TabInfo<T> ti,
       o[k * M + c] = red[3 * c] + red[3 * c + 1] + red[3 * c + 2];
     __syncwarp();
   }
+  if (__any_sync(0xffffffffu, far))
+    fwd_far<T, GG>(o, table + (size_t)m0 * 6, ti, ex, ee, nnei, M, npair / 3, brk, last,
+                   dz_dem_x + (size_t)i * nnei, dz_dem + (size_t)i * nnei * 4, lane);
 }
 
 // dy_dem_x[i,jj] = sum_m G'_m * sum_k em[jj,k] dy[k,m]
@@ -325,6 +422,7 @@ k_tab_grad(T* __restrict__ dy_dem_x, T* __restrict__ dy_dem, const T* __restrict
   const int brk = fold_start(ex, ee, nnei, lane);
   const int last = brk < nnei ? brk : nnei - 1;
   const int b4 = (lane >> 4) & 1, b3 = (lane >> 3) & 1;
+  bool anyfar = false;
   for (int base = 0; base < nnei; base += 32) {
     const int cnt = act ? max(0, min(32, last + 1 - base)) : 0, jj = base + lane;
     if (lane < cnt) {
@@ -332,6 +430,7 @@ k_tab_grad(T* __restrict__ dy_dem_x, T* __restrict__ dy_dem, const T* __restrict
 #pragma unroll
       for (int k = 0; k < 4; ++k) s_e[lane * 4 + k] = ee[jj * 4 + k];
     }
+    anyfar |= __any_sync(0xffffffffu, lane < cnt && far_x(ex[jj])) != 0;
     __syncwarp();
     // two rows in turn, the next slot's in flight (FP64: one, the registers of a
     // second would not fit a 16-warp CTA)
@@ -411,35 +510,14 @@ k_tab_grad(T* __restrict__ dy_dem_x, T* __restrict__ dy_dem, const T* __restrict
     }
     __syncthreads();
   }
+  if (act && mb == 0 && anyfar)
+    grad_far(dy_dem_x + (size_t)i * nnei, dy_dem + (size_t)i * nnei * 4, table, ti, ex, ee,
+             dy + (size_t)i * 4 * M, nnei, M, brk, last, lane);
 }
 
 // The gradient by channels, for many atoms: one warp per atom, lane l owns the
 // channels mb + 32 c + l and reads a channel's six coefficients itself. With the
 // chip full of atoms the smaller instruction count wins over the wide loads.
-template <typename T>
-struct Coef {
-  T a0, a1, a2, a3, a4, a5;
-};
-
-__device__ __forceinline__ Coef<float> load_coef(const float* p) {
-  const float2* q = reinterpret_cast<const float2*>(p);
-  float2 x = __ldg(q), y = __ldg(q + 1), z = __ldg(q + 2);
-  return {x.x, x.y, y.x, y.y, z.x, z.y};
-}
-__device__ __forceinline__ Coef<double> load_coef(const double* p) {
-  const double2* q = reinterpret_cast<const double2*>(p);
-  double2 x = __ldg(q), y = __ldg(q + 1), z = __ldg(q + 2);
-  return {x.x, x.y, y.x, y.y, z.x, z.y};
-}
-
-// value (with extrapolation) and derivative of the quintic (tabulate.cc:116-144)
-template <typename T>
-__device__ __forceinline__ void poly(const Coef<T>& a, T xx, T delta, T& v, T& g) {
-  g = a.a1 + ((T)2. * a.a2 + ((T)3. * a.a3 + ((T)4. * a.a4 + (T)5. * a.a5 * xx) * xx) * xx) * xx;
-  v = a.a0 + (a.a1 + (a.a2 + (a.a3 + (a.a4 + a.a5 * xx) * xx) * xx) * xx) * xx;
-  v = v + g * delta;
-}
-
 template <typename T, int MC>
 __global__ void __launch_bounds__(TW * 32)
 k_tab_grad_channels(T* __restrict__ dy_dem_x, T* __restrict__ dy_dem,
