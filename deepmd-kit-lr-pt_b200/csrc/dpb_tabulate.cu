@@ -1,8 +1,8 @@
 // Compressed se_a embedding: the quintic table G_m(x) fused with the
 // contraction over neighbors (tabulate_fusion_se_a and its two gradients).
 //
-// Layout: one warp per (center atom, block of 64 embedding channels). The
-// reference's table row holds a channel's six coefficients side by side; read
+// Layout: one warp per (center atom, block of 64 embedding channels; 32 of narrow
+// nets, whose half-empty block would cost as much as a full one). The reference's table row holds a channel's six coefficients side by side; read
 // per channel (24 or 48 bytes per lane) every line of the row went through L1
 // three times, and one warp per atom left small systems waiting on each row.
 // Here a row is read as it lies, 16 bytes per lane, and a lane works on
@@ -14,7 +14,8 @@
 // Measured, 92 slots, M = 100, FP32: forward 192 atoms 68 -> 19 us, 12,288 atoms
 // 234 -> 191 us (now FP32 issue and the L2 reads of the rows), grad_grad 70 -> 21
 // and 260 -> 258 us, gradient 78 -> 31 us at 192 atoms (k_tab_grad below; many
-// atoms stay on k_tab_grad_channels).
+// atoms stay on k_tab_grad_channels, and some widths' grad_grad on
+// k_tab_gg_channels).
 //
 // Semantics follow the CPU reference (source/lib/src/tabulate.cc): locate_xx
 // (:45-73) with the nextafter upper bound (:21-30), linear extrapolation
@@ -119,8 +120,6 @@ __device__ __forceinline__ void poly(const Coef<T>& a, T xx, T delta, T& v, T& g
 }
 
 constexpr int TW = 4;     // warps per block
-constexpr int TB = 64;    // channels per warp
-constexpr int TP = 6;     // coefficient pairs per lane (3 TB / 32)
 constexpr int TS = 12;    // staged values per slot: six weights of the value, six of
                           // the slope
 
@@ -174,7 +173,7 @@ __host__ __device__ constexpr int pair_power(int p) {
   return VW == 4 ? (64 * (p >> 1) + (p & 1)) % 3 : (32 * p) % 3;
 }
 
-template <typename T, int VW>
+template <typename T, int VW, int TP>
 __device__ __forceinline__ void load_row(typename Pair<T>::type (&a)[TP], const T* row, int npair,
                                          int lane) {
   using T2 = typename Pair<T>::type;
@@ -284,12 +283,13 @@ __device__ __noinline__ void grad_far(T* ox, T* oe, const T* table, TabInfo<T> t
 // out[i,k,m] = sum_jj w_jj * (G_m(x_jj) * em[jj,k])              (forward)
 // out[i,k,m] = sum_jj w_jj * (G_m * dz_dem[jj,k] + dz_dem_x[jj] * G'_m * em[jj,k])
 //                                                   (GG: grad_grad)
-template <typename T, int VW, bool GG>
+template <typename T, int VW, int TB, bool GG>
 __global__ void __launch_bounds__(TW * 32)
 k_tab_fwd(T* __restrict__ out, const T* __restrict__ table, TabInfo<T> ti,
           const T* __restrict__ em_x, const T* __restrict__ em, int nloc, int nnei, int M,
           const T* __restrict__ dz_dem_x, const T* __restrict__ dz_dem) {
   using T2 = typename Pair<T>::type;
+  constexpr int TP = 3 * TB / 32;  // coefficient pairs per lane
   // per warp: weights [32][TS], env rows [32][4] (GG: and the two multipliers of
   // value and slope); the pair sums of one env column at the end
   __shared__ __align__(16) T s_w[TW][32 * TS];
@@ -335,7 +335,7 @@ k_tab_fwd(T* __restrict__ out, const T* __restrict__ table, TabInfo<T> ti,
     const int rs = M * 6;
     T2 a[2][TP];  // two rows in turn: the next slot's is in flight
     auto fetch = [&](T2 (&v)[TP], int q) {
-      load_row<T, VW>(v, tab + (size_t)s_row[w][q] * rs, npair, lane);
+      load_row<T, VW, TP>(v, tab + (size_t)s_row[w][q] * rs, npair, lane);
     };
     auto slot = [&](const T2 (&v)[TP], int q) {
       T2 pw[3], dw[3];
@@ -390,12 +390,13 @@ k_tab_fwd(T* __restrict__ out, const T* __restrict__ table, TabInfo<T> ti,
 // A CTA holds the nmb channel blocks of blockDim / (32 nmb) atoms; a warp's
 // five sums per slot are reduced over its lanes in groups of four slots and
 // over the blocks in shared memory.
-template <typename T, int VW>
+template <typename T, int VW, int TB>
 __global__ void __launch_bounds__(512)
 k_tab_grad(T* __restrict__ dy_dem_x, T* __restrict__ dy_dem, const T* __restrict__ table,
            TabInfo<T> ti, const T* __restrict__ em_x, const T* __restrict__ em,
            const T* __restrict__ dy, int nloc, int nnei, int M, int nmb) {
   using T2 = typename Pair<T>::type;
+  constexpr int TP = 3 * TB / 32;
   extern __shared__ __align__(16) unsigned char tab_smem[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   T* s_w = reinterpret_cast<T*>(tab_smem) + (size_t)w * 32 * (TS + 4 + 5);
@@ -439,7 +440,7 @@ k_tab_grad(T* __restrict__ dy_dem_x, T* __restrict__ dy_dem, const T* __restrict
     const int rs = M * 6;
     T2 a[NB][TP];
     auto fetch = [&](T2 (&v)[TP], int q) {
-      load_row<T, VW>(v, tab + (size_t)s_row[q] * rs, npair, lane);
+      load_row<T, VW, TP>(v, tab + (size_t)s_row[q] * rs, npair, lane);
     };
     if (NB == 2 && cnt > 0) fetch(a[0], 0);
     for (int q0 = 0; q0 < cnt; q0 += 4) {
@@ -603,6 +604,53 @@ k_tab_grad_channels(T* __restrict__ dy_dem_x, T* __restrict__ dy_dem,
   }
 }
 
+// grad_grad by channels in the same way
+template <typename T, int MC>
+__global__ void __launch_bounds__(TW * 32)
+k_tab_gg_channels(T* __restrict__ out, const T* __restrict__ table, TabInfo<T> ti,
+                  const T* __restrict__ em_x, const T* __restrict__ em, int nloc, int nnei, int M,
+                  const T* __restrict__ dz_dem_x, const T* __restrict__ dz_dem) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * TW + w;
+  if (i >= nloc) return;
+  T acc[MC][4];
+#pragma unroll
+  for (int c = 0; c < MC; ++c)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[c][k] = (T)0;
+  const size_t row0 = (size_t)i * nnei;
+  const int brk = fold_start(em_x + row0, em + row0 * 4, nnei, lane);
+  const int last = brk < nnei ? brk : nnei - 1;
+  for (int jj = 0; jj <= last; ++jj) {
+    const size_t at = row0 + jj;
+    const T rep = jj == brk ? (T)(nnei - jj) : (T)1, dzx = dz_dem_x[at];
+    T e[4], h[4], t, delta;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) e[k] = em[at * 4 + k], h[k] = dz_dem[at * 4 + k];
+    int idx;
+    locate(ti, em_x[at], idx, t, delta);
+    const T* row = table + (size_t)idx * M * 6;
+#pragma unroll
+    for (int c = 0; c < MC; ++c) {
+      const int m = c * 32 + lane;
+      if (m >= M) continue;
+      T v, g;
+      poly(load_coef(row + (size_t)m * 6), t, delta, v, g);
+      const T dg = dzx * g;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[c][k] += rep * (v * h[k] + dg * e[k]);
+    }
+  }
+  T* o = out + (size_t)i * 4 * M;
+#pragma unroll
+  for (int c = 0; c < MC; ++c) {
+    const int m = c * 32 + lane;
+    if (m < M)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[k * M + m] = acc[c][k];
+  }
+}
+
 // 16-byte row loads need an even M (rows of 24 M bytes) and an aligned table;
 // FP64 pairs are 16 bytes (as the reference's double2 loads, an aligned table is
 // required)
@@ -611,13 +659,21 @@ static bool wide_rows(const T* table, int M) {
   return sizeof(T) == 4 && (M & 1) == 0 && (reinterpret_cast<uintptr_t>(table) & 15) == 0;
 }
 
-template <typename T, int VW>
+template <typename T, int VW, int TB>
 static void launch_fwd(T* out, const T* table, const TabInfo<T>& ti, const T* em_x,
                        const T* em, int nloc, int nnei, int M, const T* dzx,
                        const T* dze, cudaStream_t st) {
   const dim3 grid(ceil_div(nloc, TW), ceil_div(M, TB));
-  auto kern = dze != nullptr ? k_tab_fwd<T, VW, true> : k_tab_fwd<T, VW, false>;
+  auto kern = dze != nullptr ? k_tab_fwd<T, VW, TB, true> : k_tab_fwd<T, VW, TB, false>;
   kern<<<grid, TW * 32, 0, st>>>(out, table, ti, em_x, em, nloc, nnei, M, dzx, dze);
+}
+
+template <typename T, int MC>
+static void launch_gg_channels(T* out, const T* table, const TabInfo<T>& ti, const T* em_x,
+                               const T* em, int nloc, int nnei, int M, const T* dzx,
+                               const T* dze, cudaStream_t st) {
+  k_tab_gg_channels<T, MC><<<ceil_div(nloc, TW), TW * 32, 0, st>>>(out, table, ti, em_x, em, nloc,
+                                                                  nnei, M, dzx, dze);
 }
 
 template <typename T>
@@ -637,14 +693,24 @@ static int tab_fwd(T* out, const T* table, const T* info, const T* em_x,
     DPB_CUDA(cudaMemsetAsync(out, 0, sizeof(T) * (size_t)nloc * 4 * M, st), name);
     return DPB_OK;
   }
-  if constexpr (sizeof(T) == 4) {
-    if (wide_rows(table, M)) {
-      launch_fwd<T, 4>(out, table, ti, em_x, em, nloc, nnei, M, dzx, dze, st);
-      DPB_CHECK_LAUNCH(name);
-      return DPB_OK;
-    }
-  }
-  launch_fwd<T, 2>(out, table, ti, em_x, em, nloc, nnei, M, dzx, dze, st);
+  auto run = [&](auto launch) { launch(out, table, ti, em_x, em, nloc, nnei, M, dzx, dze, st); };
+  // grad_grad of many atoms by channels where those fill their lanes better than
+  // pairs fill their blocks: a third 32-channel share that would take a second block
+  // of 64 (us at 12,288 atoms of 92 slots, M = 96, pairs against channels: FP32 307,
+  // 259, FP64 598, 494; at 3,000 atoms about even in FP32, 160 and 190 in FP64), and
+  // FP64 up to 32 channels (M = 32: 12,288 atoms 251, 189, 3,000 84, 60, 192 25, 45;
+  // FP32 112, 137)
+  const long long per_sm = nloc / sm_count();
+  if (dze != nullptr && M > 64 && M <= 96 && per_sm >= 48)
+    run(launch_gg_channels<T, 3>);
+  else if (dze != nullptr && sizeof(T) == 8 && M <= 32 && per_sm >= 16)
+    run(launch_gg_channels<T, 1>);
+  else if (M <= 32)
+    run(launch_fwd<T, 2, 32>);
+  else if (wide_rows(table, M))
+    run(launch_fwd<T, sizeof(T) == 4 ? 4 : 2, 64>);
+  else
+    run(launch_fwd<T, 2, 64>);
   DPB_CHECK_LAUNCH(name);
   return DPB_OK;
 }
@@ -676,7 +742,7 @@ static int tab_grad(T* dy_dem_x, T* dy_dem, const T* table, const T* info,
     DPB_CHECK_LAUNCH("tabulate_fusion_se_a_grad");
     return DPB_OK;
   }
-  const int nmb = ceil_div(M, TB);  // at most 16 warps per atom
+  const int nmb = ceil_div(M, M <= 32 ? 32 : 64);  // at most 16 warps per atom
   const int atoms = nmb < TW ? TW / nmb : 1, nw = atoms * nmb;
   const size_t smem = (size_t)nw * 32 * ((TS + 4 + 5) * sizeof(T) + sizeof(int));
   auto run = [&](auto kern) -> int {
@@ -687,10 +753,12 @@ static int tab_grad(T* dy_dem_x, T* dy_dem, const T* table, const T* info,
                                                        nloc, nnei, M, nmb);
     return DPB_OK;
   };
-  if constexpr (sizeof(T) == 4)
-    rc = wide_rows(table, M) ? run(k_tab_grad<T, 4>) : run(k_tab_grad<T, 2>);
+  if (M <= 32)
+    rc = run(k_tab_grad<T, 2, 32>);
+  else if (wide_rows(table, M))
+    rc = run(k_tab_grad<T, sizeof(T) == 4 ? 4 : 2, 64>);
   else
-    rc = run(k_tab_grad<T, 2>);
+    rc = run(k_tab_grad<T, 2, 64>);
   if (rc) return rc;
   DPB_CHECK_LAUNCH("tabulate_fusion_se_a_grad");
   return DPB_OK;
