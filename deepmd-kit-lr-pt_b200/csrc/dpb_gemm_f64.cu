@@ -68,7 +68,8 @@ k_gemm_dmma(double* __restrict__ C, const double* __restrict__ A, const double* 
   extern __shared__ __align__(16) double gsm[];
   pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-  const int m0 = blockIdx.y * GD_M, n0 = blockIdx.x * GD_N;
+  const int ntn = (N + GD_N - 1) / GD_N;  // tiles in one grid dimension: the others end at 65,535
+  const int m0 = (int)(blockIdx.x / ntn) * GD_M, n0 = (int)(blockIdx.x % ntn) * GD_N;
   const int z = blockIdx.z, Z = gridDim.z;
   const int k0 = z * kchunk, k1 = min(K, k0 + kchunk);
   const int nk = k1 > k0 ? (k1 - k0 + GD_K - 1) / GD_K : 0;
@@ -423,19 +424,23 @@ extern "C" int dpb_gemm_f64(double* C, const double* A, const double* B, const d
                             int trans_b, int accumulate, dpb_stream_t stream) {
   const int rc = gemm_args("gemm_f64", C, A, B, M, N, K, lda, ldb, ldc, trans_a, trans_b);
   if (rc || M == 0 || N == 0) return rc;
-  const int gy = grid_rows("gemm_f64", M, GD_M), gx = (N + GD_N - 1) / GD_N;
-  if (gy < 0) return DPB_ERR_INVALID;
+  if (grid_rows("gemm_f64", M, GL_M) < 0) return DPB_ERR_INVALID;
+  const long long tiles = (long long)((M + GD_M - 1) / GD_M) * ((N + GD_N - 1) / GD_N);
+  if (tiles > 0x7fffffff) {
+    set_error("gemm_f64: M=%d N=%d need more than 2^31 - 1 tiles", M, N);
+    return DPB_ERR_INVALID;
+  }
   // K split over a cluster while the tiles leave SMs idle and each share keeps
   // four k blocks
   int Z = 1;
-  while (Z < 8 && (long long)gx * gy * Z * 2 <= 2 * sm_count() && K >= 2 * Z * 4 * GD_K) Z *= 2;
+  while (Z < 8 && tiles * Z * 2 <= 2 * sm_count() && K >= 2 * Z * 4 * GD_K) Z *= 2;
   int kchunk = ((K + Z - 1) / Z + GD_K - 1) / GD_K * GD_K;
   if (kchunk == 0) kchunk = GD_K;
   auto run = [&](auto kern) -> int {
     DPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GD_SMEM),
              "gemm_f64");
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(gx, gy, Z);
+    cfg.gridDim = dim3((unsigned)tiles, 1, Z);
     cfg.blockDim = dim3(GD_T);
     cfg.dynamicSmemBytes = GD_SMEM;
     cfg.stream = as_stream(stream);
