@@ -1136,8 +1136,9 @@ k_emb_rev_mma(TrGrad<T> grad, const T* __restrict__ xbar,
 // --------------------------------------------------------------- tangent --
 // xyz' and D' along u (k_tr_tan's) with the same products: a warp takes the
 // neighbors of one type of an atom, 16 rows at a time, and adds its share of
-// sum R' G + R G' to xyz' (cleared before; with two types the sum does not
-// depend on the order). Nothing waits, so as many warps as fit: 12.
+// sum R' G + R G' to xyz' (cleared before; a launch takes two types, or one that
+// adds to earlier ones, so the sum does not depend on the order). Nothing waits, so
+// as many warps as fit: 12.
 // Measured: FP64, 4 frames of 192 atoms 417 -> 176 us; FP32, 16 frames 404 -> 316.
 constexpr int EM_TAN_NW = 12;
 template <typename T>
@@ -1298,16 +1299,18 @@ static int em_fwd(double* xyz, double* D, const double* em, const TrNet<double>&
   return DPB_OK;
 }
 
-// CTAs per type in proportion to its slots
-static EmSplit em_split(const TrGeom& g, int& sms, int& used) {
+// CTAs per type of t0 .. t1 - 1 in proportion to its slots
+static EmSplit em_split(const TrGeom& g, int& sms, int& used, int t0, int t1) {
   EmSplit sp{};
-  sms = std::max(sm_count(), g.ntypes);
+  sms = std::max(sm_count(), t1 - t0);
   used = 0;
+  const int slots = std::max(1, g.sec[t1] - g.sec[t0]);
   for (int t = 0; t < g.ntypes; ++t) {
     sp.first[t] = used;
-    const int left = g.ntypes - 1 - t;
-    int n = (int)((long long)sms * (g.sec[t + 1] - g.sec[t]) / g.nnei);
-    n = t + 1 == g.ntypes ? sms - used : std::max(1, std::min(n, sms - used - left));
+    if (t < t0 || t >= t1) continue;
+    const int left = t1 - 1 - t;
+    int n = (int)((long long)sms * (g.sec[t + 1] - g.sec[t]) / slots);
+    n = t + 1 == t1 ? sms - used : std::max(1, std::min(n, sms - used - left));
     used += n;
   }
   sp.first[g.ntypes] = used;
@@ -1317,7 +1320,7 @@ static EmSplit em_split(const TrGeom& g, int& sms, int& used) {
 static int em_bwd(double* gem, const double* em, const double* xbar, const TrNet<double>& net,
                   const TrGeom& g, cudaStream_t st) {
   int sms, used;
-  const EmSplit sp = em_split(g, sms, used);
+  const EmSplit sp = em_split(g, sms, used, 0, g.ntypes);
   const size_t base = (size_t)EM_BWD_T * 8;
   const size_t per = EM_BWD_W * 8 + (size_t)(g.nnei + TR_MAXT + 1) * 4;
   const int nw = em_warps(g.nrows, std::max(1, sms / g.ntypes), EM_BWD_MAXW, base, per);
@@ -1337,7 +1340,7 @@ static int em_rev(const TrGrad<T>& gr, const T* xb, const T* xbd, const T* avg, 
                   const double* fbar, const double* vbar, const TrNet<T>& net, const TrGeom& g,
                   cudaStream_t st) {
   int sms, used;
-  const EmSplit sp = em_split(g, sms, used);
+  const EmSplit sp = em_split(g, sms, used, 0, g.ntypes);
   const size_t smem = (size_t)EmRev<T>::N * sizeof(T);
   auto kern = k_emb_rev_mma<T>;
   DPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
@@ -1374,16 +1377,22 @@ static int em_try_tan(T* xyz_t, T* D_t, const T* xyz, const T* avg, const T* std
   if (net.n1 != 25 || net.n2 != 50 || net.n3 != 100 ||
       (size_t)(g.nnei + TR_MAXT + 1) * 4 > EmRev<T>::H * sizeof(T))
     return -1;
-  int sms, used;
-  const EmSplit sp = em_split(g, sms, used);
   const size_t smem = (size_t)EM_TAN_N<T> * sizeof(T);
   auto kern = k_emb_tan_mma<T>;
   DPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
            "se_a_train_tan");
   DPB_CUDA(cudaMemsetAsync(xyz_t, 0, (size_t)g.nrows * 400 * sizeof(T), st), "se_a_train_tan");
-  DPB_CUDA(launch_pdl(kern, dim3(used), dim3(32 * EM_TAN_NW), smem, st, xyz_t, avg, std_, fbar,
-                      vbar, net, g, sp),
-           "se_a_train_tan");
+  // two types at a time, whose shares add up to the same in either order; every
+  // further type by itself, after them
+  for (int t0 = 0, t1; t0 < g.ntypes; t0 = t1) {
+    t1 = std::min(g.ntypes, t0 == 0 ? 2 : t0 + 1);
+    if (g.sec[t1] == g.sec[t0]) continue;
+    int sms, used;
+    const EmSplit sp = em_split(g, sms, used, t0, t1);
+    DPB_CUDA(launch_pdl(kern, dim3(used), dim3(32 * EM_TAN_NW), smem, st, xyz_t, avg, std_, fbar,
+                        vbar, net, g, sp),
+             "se_a_train_tan");
+  }
   DPB_CUDA(launch_pdl(k_emb_tan_out<T>, dim3(ceil_div(g.nrows, 4)), dim3(128), 0, st, xyz_t, D_t,
                       xyz, g),
            "se_a_train_tan");
