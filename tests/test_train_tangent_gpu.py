@@ -1,10 +1,10 @@
 """The tangent pass of the embedding nets: repeatable bits with any number of
-neighbor types."""
+neighbor types, and its FP32 results at the edges of the 16-row groups."""
 
 import pytest
 import torch
 
-from test_train_dmma_gpu import _tangent_and_gradients
+from test_train_dmma_gpu import EDGES, _errors, _tangent_and_gradients
 
 pytestmark = pytest.mark.gpu
 
@@ -17,3 +17,10 @@ def test_tangent_repeats_bit_for_bit(dpb, dtype, n, sel):
     for other in runs[1:]:
         assert all(torch.equal(a, b) for a, b in zip(runs[0], other))
 
+
+@pytest.mark.parametrize("n,sel,ax", EDGES)
+def test_embedding_tangent_fp32(dpb, n, sel, ax):
+    """FP32: 2e-5 of the largest, as for the weight gradients (factors of a few
+    6e-8 each, at most ten in a row, and a factor ten for cancellation)."""
+    tangents, _ = _tangent_and_gradients(dpb, n, sel, ax, torch.float32)
+    assert max(_errors(tangents)) <= 2e-5
