@@ -404,19 +404,42 @@ __device__ bool env_one(const EnvIO<CT, OT>& io, const SecInfo& sec, int row,
   return true;
 }
 
+constexpr int ENV_SMALL_CAP = 256;
+constexpr int ENV_LIST_CAP = 1024;  // what a list of up to 1,024 neighbors always has
+constexpr int ENV_LARGE_CAP = 4096;
+
 template <typename CT, typename OT, int CAP, int WARPS, bool FROM_CELLS>
-__global__ void __launch_bounds__(WARPS * 32, (CAP <= 256 && sizeof(OT) == 4) ? 32 / WARPS : 1)
+__global__ void __launch_bounds__(WARPS * 32, sizeof(OT) != 4 || CAP > 512 ? 1
+                                               : CAP <= 256          ? 32 / WARPS
+                                                                     : 28 / WARPS)
 k_env(EnvIO<CT, OT> io, SecInfo sec, int nrows, int* redo) {
   __shared__ EnvSmem<CAP> sm[WARPS];
   pdl_wait();
   pdl_trigger();
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * WARPS + w;
-  if (row >= nrows) return;
-  const bool ok = env_one<CT, OT, CAP, FROM_CELLS>(io, sec, row, sm[w], redo != nullptr);
-  if (!ok && lane == 0) {
-    int p = atomicAdd(&redo[0], 1);
-    redo[1 + p] = row;
+  if constexpr (FROM_CELLS) {
+    if (row >= nrows) return;
+    const bool ok = env_one<CT, OT, CAP, FROM_CELLS>(io, sec, row, sm[w], redo != nullptr);
+    if (!ok && lane == 0) {
+      int p = atomicAdd(&redo[0], 1);
+      redo[1 + p] = row;
+    }
+  } else if constexpr (CAP >= ENV_LIST_CAP) {
+    if (row < nrows) env_one<CT, OT, CAP, FROM_CELLS>(io, sec, row, sm[w], false);
+  } else {
+    // a row with more candidates in range than the buffer holds (more than the
+    // caller said a list has) goes again with the buffers of all warps as one
+    static_assert(sizeof(sm) >= sizeof(EnvSmem<ENV_LIST_CAP>), "the block's buffers");
+    const bool over =
+        row < nrows && !env_one<CT, OT, CAP, FROM_CELLS>(io, sec, row, sm[w], true);
+    if (!__syncthreads_or(over)) return;
+    for (int v = 0; v < WARPS; ++v) {
+      if (over && w == v)
+        env_one<CT, OT, ENV_LIST_CAP, FROM_CELLS>(
+            io, sec, row, *reinterpret_cast<EnvSmem<ENV_LIST_CAP>*>(sm), false);
+      __syncthreads();
+    }
   }
 }
 
@@ -435,8 +458,6 @@ __global__ void __launch_bounds__(32) k_env_redo(EnvIO<CT, OT> io, SecInfo sec,
   }
 }
 
-constexpr int ENV_SMALL_CAP = 256;
-constexpr int ENV_LARGE_CAP = 4096;
 
 template <typename CT, typename OT>
 static int env_cells(OT* em, OT* em_deriv, OT* rij, int* nlist, const CT* coord,
@@ -502,15 +523,16 @@ static int env_inlist(OT* em, OT* em_deriv, OT* rij, int* nlist, const CT* coord
                    avg, std_, nloc, nall, rcut, rcut_smth, status};
   // A row's candidates within rcut go to a key buffer in shared memory, at most
   // max_nbor_size of them; the smallest buffer that holds them lets the most
-  // warps run (20 per SM with 1,024 keys, 32 with 256)
+  // warps run (20 per SM with 1,024 keys, 32 with 256). Up to 1,024 candidates are
+  // taken from every list of that size class, as GPU_MAX_NBOR_SIZE's classes do.
   constexpr int W = 4;
   if (max_nbor_size <= ENV_SMALL_CAP)
     k_env<CT, OT, ENV_SMALL_CAP, W, false><<<ceil_div(inum, W), W * 32, 0, st>>>(io, s, inum,
                                                                                 nullptr);
   else if (max_nbor_size <= 512)
     k_env<CT, OT, 512, W, false><<<ceil_div(inum, W), W * 32, 0, st>>>(io, s, inum, nullptr);
-  else if (max_nbor_size <= 1024)
-    k_env<CT, OT, 1024, W, false><<<ceil_div(inum, W), W * 32, 0, st>>>(io, s, inum, nullptr);
+  else if (max_nbor_size <= ENV_LIST_CAP)
+    k_env<CT, OT, ENV_LIST_CAP, W, false><<<ceil_div(inum, W), W * 32, 0, st>>>(io, s, inum, nullptr);
   else
     k_env<CT, OT, ENV_LARGE_CAP, 1, false><<<inum, 32, 0, st>>>(io, s, inum, nullptr);
   DPB_CHECK_LAUNCH("prod_env_mat_a");
