@@ -613,7 +613,13 @@ __device__ __forceinline__ void em_mma8_k4(double (&c)[4], double a, double b) {
 // instruction truncates what it adds to its accumulator, which shows in sums
 // that run on (five times the error of FP32 sums in the first layer's
 // gradient): every eight k start from zero, the small products on their own, and
-// the rounded FP32 add carries the sum.
+// the rounded FP32 add carries the sum. What each truncation takes off the large
+// products, 2.3 to 3.3e-8 of their sum on average (measured over normal and
+// one-signed operands; mean 2.7e-8), is given back: left out, every sum came out
+// 3e-8 small, xyz' -3.3e-8 and the weight gradients -2.9 to -6.1e-8, and the
+// gradients of a training step were 1 to 3 % further from 64 bits than with FP32
+// sums. Rounding the lower terms, or the fourth product, changed neither. The
+// reverse pass takes 3 % longer.
 __device__ __forceinline__ void em_mma(float (&c)[4], EmTf a0, EmTf a1, EmTf a2, EmTf a3, EmTf b0,
                                        EmTf b1) {
   const uint32_t ah[4] = {a0.hi, a1.hi, a2.hi, a3.hi}, al[4] = {a0.lo, a1.lo, a2.lo, a3.lo};
@@ -623,9 +629,10 @@ __device__ __forceinline__ void em_mma(float (&c)[4], EmTf a0, EmTf a1, EmTf a2,
   mma_tf32(d, ah, b0.lo, b1.lo, d[0], d[1], d[2], d[3]);
 #pragma unroll
   for (int k = 0; k < 4; k += 2) {
+    const float2 ek = make_float2(e[k], e[k + 1]);
+    const float2 lost = make_float2(2.7e-8f, 2.7e-8f);
     const float2 v = __fadd2_rn(make_float2(c[k], c[k + 1]),
-                                __fadd2_rn(make_float2(d[k], d[k + 1]),
-                                           make_float2(e[k], e[k + 1])));
+                                __fadd2_rn(__ffma2_rn(ek, lost, make_float2(d[k], d[k + 1])), ek));
     c[k] = v.x;
     c[k + 1] = v.y;
   }
