@@ -102,6 +102,13 @@ __device__ __forceinline__ int em_c2(int j, int u, int v) {
   return 4 * j + u < 25 ? 4 * j + u + 25 * v : -1;
 }
 
+// zero in the padding of the layer-1 channels (an infinite input times its zero
+// weight is none)
+template <typename T>
+__device__ __forceinline__ T em_pad(int s, int t4, T v) {
+  return 4 * s + t4 < 25 ? v : (T)0;
+}
+
 // layer 2 and its adjoint in fragment order, W1 and b1 padded to 28
 template <typename T>
 __device__ inline void em_stage_f2(T* F2, const T* W2) {
@@ -171,8 +178,8 @@ __device__ __forceinline__ void em_layers12(double (&h1a)[EM_S1], double (&h1b)[
 #pragma unroll
   for (int s = 0; s < EM_S1; ++s) {
     const double w = V[4 * s + t], b = V[28 + 4 * s + t];
-    h1a[s] = tanh_f64(fma(xa, w, b));  // padding: tanh(0)
-    h1b[s] = tanh_f64(fma(xb, w, b));
+    h1a[s] = em_pad(s, t, tanh_f64(fma(xa, w, b)));
+    h1b[s] = em_pad(s, t, tanh_f64(fma(xb, w, b)));
   }
 #pragma unroll
   for (int j = 0; j < 7; ++j) {
@@ -720,8 +727,8 @@ __device__ __forceinline__ void em_layer1(T (&ha)[EM_S1], T (&hb)[EM_S1], T x0, 
 #pragma unroll
   for (int s = 0; s < EM_S1; ++s) {
     const T w1 = V[4 * s + t4], b1 = V[28 + 4 * s + t4];
-    ha[s] = em_tanh(fma(x0, w1, b1));
-    hb[s] = em_tanh(fma(x1, w1, b1));
+    ha[s] = em_pad(s, t4, em_tanh(fma(x0, w1, b1)));
+    hb[s] = em_pad(s, t4, em_tanh(fma(x1, w1, b1)));
   }
 }
 
@@ -749,8 +756,8 @@ __device__ __forceinline__ void em_layers12_tan(T x0, T x1, T d0, T d1, const T*
 #pragma unroll
     for (int e = 0; e < 2 && s + e < EM_S1; ++e) {
       const T w1 = V[4 * (s + e) + t4];
-      ta[e] = em_op(((T)1 - h1a[s + e] * h1a[s + e]) * (d0 * w1));
-      tb[e] = em_op(((T)1 - h1b[s + e] * h1b[s + e]) * (d1 * w1));
+      ta[e] = em_op(em_pad(s + e, t4, ((T)1 - h1a[s + e] * h1a[s + e]) * (d0 * w1)));
+      tb[e] = em_op(em_pad(s + e, t4, ((T)1 - h1b[s + e] * h1b[s + e]) * (d1 * w1)));
       ha[e] = em_op(h1a[s + e]);
       hb[e] = em_op(h1b[s + e]);
     }

@@ -60,3 +60,12 @@ def test_error_bound(dpb):
     print("CUDA's", float(np.abs((cuda - want) / want).max()) * 2.0 ** 53)
     assert (np.abs(got - cuda) <= (6 * 2.0 ** -53 + 2.0 ** -52) * np.abs(cuda)).all()
 
+
+def test_special_values(dpb):
+    w = np.where(np.arange(25) % 2, -1.0, 1.0)
+    x = np.array([0.0, 5e-324, 1e-310, 2.3e-308, 19.0, 20.0, 20.5, 400.0, 1e300, np.inf, np.nan])
+    got = _through_the_net(dpb, x, w)
+    want = np.tanh(x)[:, None] * w
+    assert (np.abs(got - want)[:-1] <= 2.0 ** -50 * np.abs(want)[:-1]).all()
+    assert (np.abs(got[5:10]) == 1.0).all() and np.isnan(got[10]).all()
+    assert (got[:4] == want[:4]).all()  # tiny arguments are returned as they are
