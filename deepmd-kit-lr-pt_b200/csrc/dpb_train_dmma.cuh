@@ -1104,6 +1104,9 @@ k_emb_rev_mma(TrGrad<T> grad, const T* __restrict__ xbar,
         }
       }
       __syncthreads();
+      T c2[2][4];  // this half's sum: short chains
+#pragma unroll
+      for (int k = 0; k < 4; ++k) c2[0][k] = c2[1][k] = (T)0;
 #pragma unroll 1
       for (int v = 0; v < EM_REV_NW; ++v) {
         if (!act[v]) continue;
@@ -1114,9 +1117,14 @@ k_emb_rev_mma(TrGrad<T> grad, const T* __restrict__ xbar,
           const T *aq = ap + 8 * s * P2S, *ar = aq + 4 * P2S;
           const T *bq = bp + 8 * s * P1S, *br = bq + 4 * P1S;
           const Op a0 = em_op(aq[0]), a1 = em_op(aq[8]), a2 = em_op(ar[0]), a3 = em_op(ar[8]);
-          em_mma(gw2[0], a0, a1, a2, a3, em_op(bq[0]), em_op(br[0]));
-          em_mma(gw2[1], a0, a1, a2, a3, em_op(bq[8]), em_op(br[8]));
+          em_mma(c2[0], a0, a1, a2, a3, em_op(bq[0]), em_op(br[0]));
+          em_mma(c2[1], a0, a1, a2, a3, em_op(bq[8]), em_op(br[8]));
         }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        gw2[0][k] += c2[0][k];
+        gw2[1][k] += c2[1][k];
       }
     }
   }
