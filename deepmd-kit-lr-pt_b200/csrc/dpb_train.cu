@@ -1734,15 +1734,14 @@ static int tr_pick_warps(TrKind kind, const TrDims& d, int maxw, int R, bool sac
   return 0;
 }
 
-// rows per group: the train_rows_per_group knob for the FP32 standard net;
-// train_rows_per_group_f64 for the FP64 force-backward kernel of the
-// standard net (measured on the 12,288-atom FP64 plain step: backward 7.30
-// ms with 4 rows, 5.88 ms with 8; the forward is faster with 4, 3.18 against
-// 3.46 ms, and the tangent and reverse kernels spill at 8); else the
+// rows per group: the train_rows_per_group knob for the FP32 forward and force
+// backward of the standard net; train_rows_per_group_f64 for its FP64 force
+// backward where the matrix form does not run (more than three types; measured
+// on the 12,288-atom FP64 plain step: 7.30 ms with 4 rows, 5.88 with 8); else the
 // precision's default
 template <typename T>
 static int tr_rows(const TrNet<T>& net, TrKind kind) {
-  if (!tr_std_net(net)) return TrTraits<T>::R;
+  if (!tr_std_net(net) || kind == TR_TAN || kind == TR_REV) return TrTraits<T>::R;
   if (sizeof(T) == 4) return tune_value("train_rows_per_group", TrTraits<T>::R) == 4 ? 4 : 8;
   if (kind != TR_BWD) return TrTraits<T>::R;
   return tune_value("train_rows_per_group_f64", 8) == 4 ? 4 : 8;
@@ -1895,8 +1894,7 @@ using namespace dpb;
     rc = em_try_tan<T>(xyz_t, descrpt_t, xyz, avg, std_, force_bar, virial_bar, net, g,          \
                        as_stream(stream));                                                      \
     if (rc >= 0) return rc;                                                                     \
-    auto kern = !tr_std_net(net) ? k_tr_tan<T, TrTraits<T>::R, 0, 0, 0>                         \
-                : (R == 4 ? k_tr_tan<T, 4, 25, 50, 100> : k_tr_tan<T, 8, 25, 50, 100>);\
+    auto kern = k_tr_tan<T, TrTraits<T>::R, 0, 0, 0>;                                           \
     int grid;                                                                                   \
     size_t smem;                                                                                \
     rc = tr_launch_cfg(kern, L, sizeof(T), nrows, grid, smem);                                  \
@@ -1947,8 +1945,7 @@ using namespace dpb;
     if (rc) return rc;                                                                          \
     rc = em_try_rev<T>(gr, xb, xbd, avg, std_, force_bar, virial_bar, net, g, st);              \
     if (rc >= 0) return rc;                                                                     \
-    auto kern = !tr_std_net(net) ? k_tr_rev<T, TrTraits<T>::R, 0, 0, 0>                         \
-                : (R == 4 ? k_tr_rev<T, 4, 25, 50, 100> : k_tr_rev<T, 8, 25, 50, 100>);\
+    auto kern = k_tr_rev<T, TrTraits<T>::R, 0, 0, 0>;                                           \
     int grid;                                                                                   \
     size_t smem;                                                                                \
     rc = tr_launch_cfg(kern, L, sizeof(T), nrows, grid, smem);                                  \

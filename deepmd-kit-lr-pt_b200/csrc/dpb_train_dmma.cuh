@@ -1397,15 +1397,13 @@ static int em_try_bwd(T* gem, const T* em, const T* xbar, const TrNet<T>& net, c
 }
 
 // The tangent and the reverse pass keep one net per CTA, so any number of types;
-// the entry list of an atom has to fit where a tile's layer outputs (adjoints) go
-// later.
+// the entry list of an atom lies where a tile's layer outputs (adjoints) go later.
 template <typename T>
 static int em_try_tan(T* xyz_t, T* D_t, const T* xyz, const T* avg, const T* std_,
                       const double* fbar, const double* vbar, const TrNet<T>& net, const TrGeom& g,
                       cudaStream_t st) {
-  if (net.n1 != 25 || net.n2 != 50 || net.n3 != 100 ||
-      (size_t)(g.nnei + TR_MAXT + 1) * 4 > EmRev<T>::H * sizeof(T))
-    return -1;
+  static_assert((BT_NMAX + TR_MAXT + 1) * 4 <= EmRev<T>::H * (int)sizeof(T), "entry list");
+  if (net.n1 != 25 || net.n2 != 50 || net.n3 != 100) return -1;
   const size_t smem = (size_t)EM_TAN_N<T> * sizeof(T);
   auto kern = k_emb_tan_mma<T>;
   DPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
@@ -1432,8 +1430,8 @@ template <typename T>
 static int em_try_rev(const TrGrad<T>& gr, const T* xb, const T* xbd, const T* avg, const T* std_,
                       const double* fbar, const double* vbar, const TrNet<T>& net, const TrGeom& g,
                       cudaStream_t st) {
-  if (net.n1 == 25 && net.n2 == 50 && net.n3 == 100 &&
-      (size_t)(g.nnei + TR_MAXT + 1) * 4 <= EmRev<T>::Z * sizeof(T))
+  static_assert((BT_NMAX + TR_MAXT + 1) * 4 <= EmRev<T>::Z * (int)sizeof(T), "entry list");
+  if (net.n1 == 25 && net.n2 == 50 && net.n3 == 100)
     return em_rev<T>(gr, xb, xbd, avg, std_, fbar, vbar, net, g, st);
   return -1;
 }
