@@ -74,7 +74,7 @@ struct BtStepArgs {
   BtFrames fr;
   BtSec sec;
   TypeTables tt;
-  ChebTables ct;      // piecewise Chebyshev nets (rows then go in groups of four)
+  ChebTables ct;      // piecewise Chebyshev nets (rows then go in groups of CHEB_A)
   unsigned* touched;
   float* row_scale;
   double* cw;

@@ -61,12 +61,12 @@ static Knob g_knobs[] = {
     // descriptor backward and the forces) as separate passes, 0 back to back
     // per row in one pass
     {"batch_fused_split", 0, 2, {0, 1}},
-    // neighbor rows per group in the FP32 training kernels on the FMA pipe
-    // (forward and backward; tangent and reverse too for other nets than
-    // 25-50-100)
+    // neighbor rows per group in the FP32 training forward and force backward
+    // of the 25-50-100 net (other nets, and the general tangent and reverse
+    // kernels, have 4 in FP64 and 8 in FP32)
     {"train_rows_per_group", 8, 2, {4, 8}},
-    // the same for the FP64 force-backward kernel of nets that the matrix
-    // form does not take
+    // the same for the FP64 force backward of that net with more than three
+    // neighbor types, which the matrix form does not take
     {"train_rows_per_group_f64", 8, 2, {4, 8}},
     // most warps per CTA of the training kernels (fewer when shared memory
     // does not allow them)
