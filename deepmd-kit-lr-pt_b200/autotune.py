@@ -61,8 +61,13 @@ def _cache_path() -> str:
         os.path.expanduser("~"), ".cache", "deepmd_kit_lr_pt_b200", "tune.json"))
 
 
+# Counts the changes of the kernels that the knobs shape: a cache file of other
+# kernels has no say.
+KERNELS = 2
+
+
 def _key(signature: str, device) -> str:
-    return f"{torch.cuda.get_device_name(device)}|{signature}"
+    return f"{torch.cuda.get_device_name(device)}|kernels{KERNELS}|{signature}"
 
 
 def load_cached(signature: str, device=None) -> dict | None:

@@ -329,10 +329,10 @@ class BatchEvaluator:
             self.capture()
             return {}
         cfg = self.cfg
-        sig = (f"batch:{self.nframes}f:{self.N}a:deg{self.ptab.degree}:"
+        sig = (f"batch:{self.nframes}f:{self.N}a:{self.ptab.tune_tag()}:"
                f"sel{'-'.join(map(str, cfg.sel))}:"
                f"M{cfg.neuron[-1]}:fit{'-'.join(map(str, cfg.fitting))}")
         return autotune.tune(self.replay, lambda: self.capture(),
-                             ["batch_atoms_per_cta", "desc_atoms_per_cta", "desc_coef_l1",
-                              "fit_n_tile", "fit_split_b", "pdl"],
+                             ["batch_atoms_per_cta", *self.ptab.tune_knobs(), "fit_n_tile",
+                              "fit_split_b", "pdl"],
                              signature=sig, reps=reps, device=self.dev, use_cache=use_cache)

@@ -269,6 +269,15 @@ class PipelineTables:
         # operand scales of the descriptor rows, written by the forward
         self.row_scale = torch.ones(max(rows, 1), device=dev)
 
+    def tune_tag(self) -> str:
+        """The passes' form, for the autotuner's cache: a shape timed on one form
+        says nothing of another."""
+        return f"deg{self.degree}-{'cheb' if self.nets is not None else 'table'}"
+
+    def tune_knobs(self) -> list:
+        """The knobs that these passes read: the Chebyshev kernels have none."""
+        return [] if self.nets is not None else ["desc_atoms_per_cta", "desc_coef_l1"]
+
     def _check_rows(self, n: int) -> None:
         # the kernels write touched and row_scale by row and know no capacity
         if n > self.rows:
@@ -976,19 +985,18 @@ class SeAEvaluator:
         return hr[0:1], hr[1:1 + 3 * n].view(n, 3), hr[1 + 3 * n:]
 
     def tune(self, reps: int = 10, use_cache: bool = True) -> dict:
-        """Autotune the launch shapes of this step (atoms per CTA of the fused
-        descriptor kernels, table-load cache policy, fitting GEMM N tile and
-        weight split, programmatic dependent launch on or off); leaves it
-        captured with the fastest."""
+        """Autotune the launch shapes of this step (on tables, atoms per CTA of
+        the fused descriptor kernels and table-load cache policy; fitting GEMM N
+        tile and weight split, programmatic dependent launch on or off); leaves
+        it captured with the fastest."""
         from . import autotune
 
         cfg = self.cfg
-        sig = (f"frame:{self.nloc}a:{self.mode}:skin{self.skin:g}:deg{self.ptab.degree}:"
+        sig = (f"frame:{self.nloc}a:{self.mode}:skin{self.skin:g}:{self.ptab.tune_tag()}:"
                f"sel{'-'.join(map(str, cfg.sel))}:"
                f"M{cfg.neuron[-1]}:fit{'-'.join(map(str, cfg.fitting))}")
         return autotune.tune(self.replay, lambda: self.capture(),
-                             ["desc_atoms_per_cta", "desc_coef_l1", "fit_n_tile", "fit_split_b",
-                              "pdl"],
+                             [*self.ptab.tune_knobs(), "fit_n_tile", "fit_split_b", "pdl"],
                              signature=sig, reps=reps,
                              device=self.dev, use_cache=use_cache)
 
