@@ -253,10 +253,12 @@ def chebyshev_net(table: np.ndarray, info: np.ndarray, tol: float = 1.5e-8,
     the tensor-core descriptor kernels (dpb_se_a_descriptor_*_cheb_f32).
 
     Intervals start at width 8 and are halved until the expansion agrees with
-    the table at every knot and midpoint: the value to tol of the largest
-    |G|, the slope to tol_slope of the largest |G'| (the cubic
-    re-interpolation's own remainder is of that size, and FP32 resolves
-    6e-8). A smooth net needs 6-10 intervals; one that needs more than
+    the table at every knot, their ends included, and every midpoint: the
+    value to tol of the largest |G|, the slope to tol_slope of the largest
+    |G'| (the cubic re-interpolation's own remainder is of that size, and FP32
+    resolves 6e-8). Where two intervals meet, value and slope may therefore
+    jump by twice these (seen: 1.4e-9 and 4.3e-7 of the largest); the tables are
+    smooth to the first derivative there. A smooth net needs 6-10 intervals; one that needs more than
     CHEB_MAX_INTERVALS, or whose bounds are no multiples of the cell width,
     returns None and stays on the table.
 
@@ -286,7 +288,10 @@ def chebyshev_net(table: np.ndarray, info: np.ndarray, tol: float = 1.5e-8,
     for p in range(4, 0, -1):
         slope *= mid
         slope += p * T[p]
-    ref = [(T[0], T[1]), (value(every, mid), slope)]
+    last = T[:, -1:]
+    ref = [(np.concatenate([T[0], sum(last[p] * s0**p for p in range(6))]),
+            np.concatenate([T[1], sum(p * last[p] * s0 ** (p - 1) for p in range(1, 6))])),
+           (value(every, mid), slope)]
     big = max(np.abs(v).max() for v, _ in ref)
     steep = max(np.abs(g).max() for _, g in ref)
     if not (np.isfinite(big) and np.isfinite(steep)) or big == 0.0:
@@ -304,7 +309,7 @@ def chebyshev_net(table: np.ndarray, info: np.ndarray, tol: float = 1.5e-8,
         C = dct @ value(r, (x - (lower + r * s0))[:, None])
         for off, (v, g) in zip((0.0, 0.5 * s0), ref):
             i0 = int(np.ceil((a - lower - off) / s0 - 1e-9))
-            i1 = int(np.ceil((b - lower - off) / s0 - 1e-9))
+            i1 = int(np.ceil((b - lower - off) / s0 - 1e-9)) + (off == 0.0)  # knots: b as well
             t = (lower + off + np.arange(i0, i1) * s0 - c) / h
             P = [np.ones_like(t), t]
             U = [np.ones_like(t), 2 * t]
