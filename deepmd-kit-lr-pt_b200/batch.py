@@ -194,6 +194,11 @@ class BatchEvaluator:
         d.type_rows, d.ntypes = fit.type_rows.ctypes.data, fit.ntypes
         E = fit
 
+        def weights(name):
+            # with nets, dpb_bt_step_set_nets puts the FP16 pairs (as many bytes a
+            # row, or more) in the place of TF32 weights, which are then not made
+            return (fit.f16(name)[0],) * 2 if pt.nets is not None else fit.tf32(name)
+
         def layer(A, K, B, N, mode, out0, out1=None, aux0=None, aux1=None, bias=None,
                   idt=None, wv=None):
             g = GemmLayer()
@@ -206,14 +211,14 @@ class BatchEvaluator:
             return g
 
         layers = [
-            layer(self.D, din, E.tf32("1f"), w, E.EPI_TANH, E.H1, bias=E.b1),
-            layer(E.H1, w, E.tf32("2f"), w, E.EPI_RES_DT, E.Y2, E.H2, aux0=E.H1, bias=E.b2,
+            layer(self.D, din, weights("1f"), w, E.EPI_TANH, E.H1, bias=E.b1),
+            layer(E.H1, w, weights("2f"), w, E.EPI_RES_DT, E.Y2, E.H2, aux0=E.H1, bias=E.b2,
                   idt=E.d2),
-            layer(E.H2, w, E.tf32("3f"), w, E.EPI_LAST, E.G3, aux0=E.H2, bias=E.b3, idt=E.d3,
+            layer(E.H2, w, weights("3f"), w, E.EPI_LAST, E.G3, aux0=E.H2, bias=E.b3, idt=E.d3,
                   wv=E.w4),
-            layer(E.G3, w, E.tf32("3b"), w, E.EPI_BWD_DT, E.G2, E.g2, aux0=E.Y2, idt=E.d2, wv=E.w4),
-            layer(E.G2, w, E.tf32("2b"), w, E.EPI_BWD_RES, E.G1, aux0=E.H1, aux1=E.g2),
-            layer(E.G1, w, E.tf32("1b"), din, E.EPI_STORE, self.dD)]
+            layer(E.G3, w, weights("3b"), w, E.EPI_BWD_DT, E.G2, E.g2, aux0=E.Y2, idt=E.d2, wv=E.w4),
+            layer(E.G2, w, weights("2b"), w, E.EPI_BWD_RES, E.G1, aux0=E.H1, aux1=E.g2),
+            layer(E.G1, w, weights("1b"), din, E.EPI_STORE, self.dD)]
         for k, g in enumerate(layers):
             d.fit[k] = g
         self._desc = d

@@ -35,3 +35,18 @@ def test_first_step_under_capture(dpb, split_b):
     finally:
         at.set_knob("fit_split_b", 0)
     assert torch.equal(got, want) and bool(got.any())
+
+
+@pytest.mark.parametrize("fused", [True, False])
+def test_batch_keeps_one_form(dpb, fused):
+    """The batched step on Chebyshev nets holds no TF32 weights beside the FP16
+    pairs it runs on."""
+    wl = importlib.import_module("deepmd_kit_lr_pt_b200.workload")
+    model = importlib.import_module("deepmd_kit_lr_pt_b200.model")
+    batch = importlib.import_module("deepmd_kit_lr_pt_b200.batch")
+    coord, atype, box = wl.water_frame(3, seed=2)
+    p = model.prepare(model.init_params(model.SeAConfig(), seed=2), coord, atype, box)
+    ev = batch.BatchEvaluator(p, [(coord, atype, box)], fused=fused)
+    e, f, _ = ev.compute()
+    assert ev.ptab.nets is not None and not ev.fit._tf32 and len(ev.fit._f16) == 6
+    assert np.isfinite(e).all() and np.abs(f).max() > 0
