@@ -591,7 +591,7 @@ int dpb_bt_step_set_b_inv(void* plan, const float* const* b_inv) {
   }
   for (int l = 0, o = 0; l < BS_PASSES; ++l)
     for (int t = 0; t < p->a.shp[l].ntypes; ++t, ++o) {
-      if (b_inv[o] == nullptr || ((uintptr_t)b_inv[o] & 15) != 0) {
+      if (((uintptr_t)b_inv[o] & 15) != 0) {
         set_error("bt_step_set_b_inv: the reciprocals must be 16-byte aligned");
         return DPB_ERR_INVALID;
       }

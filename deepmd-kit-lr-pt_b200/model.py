@@ -496,31 +496,40 @@ class _FittingTC:
         return self._tf32[name]
 
     def f16(self, name):
-        """(pairs, reciprocals of the row scales) of the weights ``name``,
-        pointer arrays by type. Every row has its own power of two, which
-        brings its largest entry to 2^13 .. 2^14: with one per matrix an output
-        whose weights are small beside another's lost bits (2^-39 of the largest
-        is what a pair resolves)."""
+        """(pairs, reciprocals of the row scales, scales) of the weights ``name``
+        by type. A matrix whose rows' largest entries lie within 2^8 of one
+        another has one scale, a power of two that brings its largest to 2^13 ..
+        2^14 (no reciprocals: NULL). A pair resolves 2^-39 of that, 2^-31 of such a
+        row's largest. Wider apart, every row has its own and the epilogue undoes
+        it, at 1 % of a step (12,288 atoms 566 -> 571 us)."""
         if name not in self._f16:
-            ts, inv = [], []
+            ts, inv, scales = [], [], []
             for m in self._mats[name]:
                 m = np.ascontiguousarray(m, np.float32)
                 big = np.abs(m).max(1)
                 if not np.isfinite(big).all():
                     big = np.where(np.isfinite(m), np.abs(m), np.float32(0)).max(1)
                 e = np.clip(np.frexp(big)[1], -112, 128)  # big < 2^e
-                one = np.ones(e.size, np.float32)
-                scale = torch.tensor(np.ldexp(one, 14 - e), device=self.dev)
-                w = torch.nn.functional.pad(torch.tensor(m, device=self.dev) * scale[:, None],
-                                            (0, -m.shape[1] % 32))
+                e = np.where(big > 0, e, e[big > 0].max(initial=-112))
+                rows = int(e.max()) - int(e.min()) > 8
+                scales.append(1.0 if rows else 2.0 ** (14 - int(e.max())))
+                w = torch.tensor(m, device=self.dev)
+                if rows:
+                    one = np.ones(e.size, np.float32)
+                    inv.append(torch.tensor(np.ldexp(one, e - 14), device=self.dev))
+                    w = w * torch.tensor(np.ldexp(one, 14 - e), device=self.dev)[:, None]
+                else:
+                    inv.append(None)
+                    w = w * scales[-1]
+                w = torch.nn.functional.pad(w, (0, -w.shape[1] % 32))
                 hi = w.half()
                 pair = torch.stack([x.view(w.shape[0], -1, 32) for x in
                                     (hi, (w - hi.float()).half())], 2)
                 ts.append(pair.contiguous())
-                inv.append(torch.tensor(np.ldexp(one, e - 14), device=self.dev))
-            self._keep.extend(ts + inv)
-            self._f16[name] = tuple((ctypes.c_void_p * len(x))(*[t.data_ptr() for t in x])
-                                    for x in (ts, inv))
+            self._keep.extend(ts + [t for t in inv if t is not None])
+            at = [(ctypes.c_void_p * len(x))(*[None if t is None else t.data_ptr() for t in x])
+                  for x in (ts, inv)]
+            self._f16[name] = (*at, np.array(scales, np.float32))
         return self._f16[name]
 
     def f16_layers(self):
@@ -533,7 +542,8 @@ class _FittingTC:
         one = np.ones(self.ntypes, np.float32)
         a = np.concatenate([one if k is None else self._scales[k] for _, k in names])
         return ((ctypes.c_void_p * len(b))(*b), np.ascontiguousarray(a),
-                np.ones(6 * self.ntypes, np.float32), (ctypes.c_void_p * len(inv))(*inv))
+                np.concatenate([self.f16(n)[2] for n, _ in names]),
+                (ctypes.c_void_p * len(inv))(*inv))
 
     @staticmethod
     def _operand_scales(params):
@@ -558,9 +568,9 @@ class _FittingTC:
     def _gemm(self, A, K, name, N, mode, out0, out1=None, aux0=None, aux1=None, bias=None,
               idt=None, w=None, s=None, scale=None, row_scale=None):
         if scale is not None:
-            b, inv = self.f16(name)
+            b, inv, bs = self.f16(name)
             call("dpb_gemm_f16x3_rows_f32", ptr(A), self.n, K, ptr(row_scale), scale.ctypes.data,
-                 b, None, inv, N, self.type_rows.ctypes.data, self.ntypes, mode, ptr(out0),
+                 b, bs.ctypes.data, inv, N, self.type_rows.ctypes.data, self.ntypes, mode, ptr(out0),
                  ptr(out1), ptr(aux0), ptr(aux1), bias, idt, w, ptr(self.e), ptr(self.status), s)
             return
         B = self.tf32(name)

@@ -514,8 +514,8 @@ DPB_API int dpb_bt_step_set_nets(void* plan, const dpb_cheb_net* nets, unsigned*
                                  float* row_scale, const void* const* b, const float* a_scale,
                                  const float* b_scale);
 /* Reciprocals of the FP16 weights' scales per row, as b_inv of
- * dpb_gemm_f16x3_rows_f32: ntypes device arrays for each of the six GEMMs, after
- * dpb_bt_step_set_nets. */
+ * dpb_gemm_f16x3_rows_f32: ntypes device arrays (NULL: 1) for each of the six
+ * GEMMs, after dpb_bt_step_set_nets. */
 DPB_API int dpb_bt_step_set_b_inv(void* plan, const float* const* b_inv);
 /* One step: env, descriptor, fitting, descriptor backward, forces, virials
  * and energies of every frame in ONE cooperative launch (one CTA per SM),
@@ -694,7 +694,7 @@ DPB_API int dpb_gemm_f16x3_f32(const float* A, int M, int K, const float* row_sc
                                dpb_stream_t stream);
 /* The same with weights whose rows have scales of their own: b holds
  * B[n, k] * b_scale[t] / b_inv[t][n] (b_scale may be NULL: 1; b_inv: device
- * [N] per type, powers of two, may be NULL: 1). Rows of very different size then
+ * [N] per type, powers of two; it, or one type's, may be NULL: 1). Rows of very different size then
  * keep their bits. */
 DPB_API int dpb_gemm_f16x3_rows_f32(const float* A, int M, int K, const float* row_scale,
                                     const float* a_scale, const void* const* b,

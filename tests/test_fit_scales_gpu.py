@@ -48,6 +48,41 @@ def test_units_with_small_weights(dpb, mdl):
         o += k
 
 
+@pytest.mark.parametrize("spread", [40, 9, 7, 0])
+def test_units_of_uneven_weights(dpb, mdl, spread):
+    """First layer with the units' weights 2^0 .. 2^-spread of the largest (a scale
+    per row from a spread of 2^8 on): the
+    pre-activation error is within (2^-22 + 2^-23 * 100) sum |a| |b| of each
+    unit's own terms (operand splits, and half an ulp of the truncating
+    tensor-core sum per instruction of 16 k), and tanh adds 2^-22 of its
+    value (2 ulp)."""
+    cfg = mdl.SeAConfig()
+    p = mdl.init_params(cfg, seed=5)
+    rows, n = [130, 67], 197
+    rng = np.random.default_rng(5)
+    size = 2.0 ** -(np.arange(240) % (spread + 1))
+    for f in p.fit:
+        (W, b, d), *rest = f["layers"]
+        f["layers"] = [((W * size).astype(np.float32), 0 * b, d), *rest]
+    D = rng.normal(size=(n, 1600)).astype(np.float32)
+    fit = mdl._FittingTC(p, rows, "cuda")
+    scale = torch.full((n,), 2.0 ** 11, device="cuda")  # |D| < 8
+    assert np.abs(D).max() < 8
+    dD = torch.zeros((n, 1600), device="cuda")
+    if spread in (0, 40):  # the rows' largest entries differ by less than 2 by themselves
+        assert all((t is not None) == (spread == 40) for t in fit.f16("1f")[1])
+    fit.layers(torch.tensor(D, device="cuda"), dD, row_scale=scale)
+    got = fit.H1.cpu().numpy().astype(np.float64)
+    o = 0
+    for k, f in zip(rows, p.fit):
+        W = f["layers"][0][0].astype(np.float64)
+        a = D[o:o + k].astype(np.float64)
+        want, mag = np.tanh(a @ W), np.abs(a) @ np.abs(W)
+        err = np.abs(got[o:o + k] - want)
+        assert (err <= (2.0 ** -22 + 2.0 ** -23 * 100) * mag + 2.0 ** -22 * np.abs(want)).all()
+        o += k
+
+
 def test_batched_step_with_uneven_units(dpb):
     """The one-launch step takes the weights in the same form: forces and
     energies as the evaluator's, frame by frame. Both run the FP16 GEMMs, so
