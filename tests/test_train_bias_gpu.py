@@ -39,13 +39,8 @@ def _run(dpb, dt, n, sel, ax, cfg, d):
     return [q.double() for q in out + g]
 
 
-@pytest.mark.parametrize("seed", [0, 1, 2])
-def test_no_systematic_shrinking(dpb, seed):
-    """<got - want, want> / <want, want> over each whole result: rounded FP32 sums
-    leave a factor of order 1 / sqrt(entries) of their 2^-24 roundings, truncated
-    ones 2^-25 and more per product of a layer. The bound is 2^-26 for xyz' and D'
-    (30,000 and 480,000 entries); the mean over the weight gradients, whose entries
-    share their roundings, stays within 2^-25."""
+def _shift(dpb, seed):
+    """<got - want, want> / <want, want> of xyz', D' and each weight gradient."""
     wl = importlib.import_module("deepmd_kit_lr_pt_b200.workload")
     n, sel, ax = 300, (46, 92), 16
     cfg = wl.SeAConfig(sel=sel, axis_neuron=ax)
@@ -70,6 +65,17 @@ def test_no_systematic_shrinking(dpb, seed):
          "xyz": r32(rng.normal(0, .3, (n, 4, 100))), "xyzt": r32(rng.normal(0, .3, (n, 4, 100))),
          "dD": r32(rng.normal(0, 1, (n, 100 * ax))), "dDt": r32(rng.normal(0, 1, (n, 100 * ax)))}
     got, want = (_run(dpb, dt, n, sel, ax, cfg, d) for dt in (torch.float32, torch.float64))
-    shift = [float(((a - b) * b).sum() / (b * b).sum()) for a, b in zip(got, want)]
-    assert max(abs(v) for v in shift[:2]) <= 2.0 ** -26, shift
-    assert abs(np.mean(shift[2:])) <= 2.0 ** -25, shift
+    return [float(((a - b) * b).sum() / (b * b).sum()) for a, b in zip(got, want)]
+
+
+def test_no_systematic_shrinking(dpb):
+    """Rounded FP32 sums leave each draw of inputs a factor of either sign (of
+    order 2^-25 for the weight gradients, whose entries share their roundings; plain
+    FMA kernels show the same), truncated ones add one of the same sign to every
+    draw, 2^-25 and more per product of a layer. So the mean over 16 draws is held: to
+    2^-26 for xyz' and D' (30,000 and 480,000 entries a draw), to 2^-25 for the mean
+    of the weight gradients."""
+    shift = np.array([_shift(dpb, seed) for seed in range(16)])
+    mean = shift.mean(axis=0)
+    assert np.abs(mean[:2]).max() <= 2.0 ** -26, shift
+    assert abs(mean[2:].mean()) <= 2.0 ** -25, shift
