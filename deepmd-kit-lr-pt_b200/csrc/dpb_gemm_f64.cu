@@ -35,8 +35,8 @@ constexpr int GB_M = 64, GB_N = 64, GB_K = 16, GB_T = 256;
 // M): a cluster of Z CTAs shares the tile's K range and adds the Z partial
 // tiles through distributed shared memory in rank order, so the result does
 // not depend on scheduling and no workspace is needed. Measured, the fitting
-// GEMMs of one step: 3,993 atoms 1.63 -> 0.81 ms, a training step of 768 atoms
-// (two streams) 4.0 -> 1.4 ms of kernel time.
+// GEMMs of one step: 3,993 atoms 1.63 -> 0.52 ms, a training step of 768 atoms
+// (two streams) 4.0 -> 1.15 ms of kernel time.
 constexpr int GD_M = 64, GD_N = 80, GD_K = 16, GD_ST = 3, GD_T = 256;
 constexpr int GD_SK = GD_K + 4;                        // row stride of [m][k] / [n][k]
 constexpr int GD_SM = GD_M + 4, GD_SN = GD_N + 4;      // of [k][m], [k][n]

@@ -11,9 +11,9 @@
 // pair and over a channel's three pairs once at the end (forward), or multiplied
 // by the channel's gradient at once (backward). Slots are located 32 at a time,
 // one per lane, and the next slot's row is in flight while one is summed.
-// Measured, 92 slots, M = 100, FP32: forward 192 atoms 68 -> 19 us, 12,288 atoms
-// 234 -> 191 us (now FP32 issue and the L2 reads of the rows), grad_grad 70 -> 21
-// and 260 -> 258 us, gradient 78 -> 31 us at 192 atoms (k_tab_grad below; many
+// Measured, 92 slots, M = 100, FP32: forward 192 atoms 94 -> 22 us, 12,288 atoms
+// 317 -> 232 us (now L1 at 80 % and FP32 issue at 65 %), grad_grad 96 -> 23 and 338
+// -> 316 us, gradient 101 -> 31 us at 192 atoms (k_tab_grad below; many
 // atoms stay on k_tab_grad_channels, and some widths' grad_grad on
 // k_tab_gg_channels).
 //

@@ -551,10 +551,11 @@ k_emb_bwd_dmma(double* __restrict__ gem, const double* __restrict__ em,
 // Tiles are numbered tile-in-atom first, so the empty ones (beyond an atom's
 // neighbors) are the last and the rest come out even over the warps.
 //
-// Measured: FP64, 4 frames of 192 atoms 1666 -> 461 us (FP64 matrix pipe 44 % busy,
-// the FMA pipe 10 %); FP32, 16 frames 1584 -> 1011 us (matrix pipe 35 %, issue
-// slots 43 %: splitting the operands takes three instructions per element). The rest
-// is the latency of two warps per scheduler; the accumulators leave room for no more.
+// Measured: FP64, 4 frames of 192 atoms 1666 -> 439 us (FP64 matrix pipe 49 % busy,
+// the FMA pipe 10 %, issue slots 18 %); FP32, 16 frames 1584 -> 1033 us (matrix pipe
+// 36 %, issue slots 45 %: splitting the operands takes three instructions per
+// element). The rest is the latency of two warps per scheduler; the accumulators
+// leave room for no more.
 constexpr int EM_REV_NW = 8;
 // Row strides that keep the operand reads free of (most) bank conflicts for
 // 8-byte and 4-byte elements, in elements; W3's rows, staged layer-2 and
@@ -1168,7 +1169,7 @@ k_emb_rev_mma(TrGrad<T> grad, const T* __restrict__ xbar,
 // sum R' G + R G' to xyz' (cleared before; a launch takes two types, or one that
 // adds to earlier ones, so the sum does not depend on the order). Nothing waits, so
 // as many warps as fit: 12.
-// Measured: FP64, 4 frames of 192 atoms 417 -> 176 us; FP32, 16 frames 404 -> 316.
+// Measured: FP64, 4 frames of 192 atoms 417 -> 182 us; FP32, 16 frames 404 -> 334.
 constexpr int EM_TAN_NW = 12;
 template <typename T>
 constexpr int EM_TAN_N = EmRev<T>::W3 * 8 / (int)sizeof(T) + EM_F2 + EmRev<T>::V +
